@@ -60,9 +60,13 @@ cudaError_t launch_radix_tree(const Launch& L, const K* codes, const uint32_t* d
       cudaError_t e = cudaMemsetAsync(q_count, 0, 4, L.stream);
       if (e != cudaSuccess) return e;
     }
-    cudaError_t e = launch_kernel(L, radix_tree_window_kernel<K, false>, max(1u, ceil_div(work, TW_T)), TW_THREADS, 0,
-                                  codes, d_u, u_host, nullptr, 0u, prefix_n, hll, hlr, left, parent, edge, d_m, queue,
-                                  q_count);
+    auto window = [&](auto shape) {
+      using SH = decltype(shape);
+      return launch_kernel(L, radix_tree_window_kernel<K, false, SH>, max(1u, ceil_div(work, SH::T)), TW_THREADS, 0,
+                           codes, d_u, u_host, nullptr, 0u, prefix_n, hll, hlr, left, parent, edge, d_m, queue,
+                           q_count);
+    };
+    cudaError_t e = work <= TW_SMALL_MAX ? window(TwSmall{}) : window(TwLarge{});
     if (e != cudaSuccess || !queue) return e;
     return launch_kernel(L, radix_tree_slow_kernel<K, false>, L.num_sms * 2, 256, 0, codes, d_u, u_host, nullptr, 0u,
                          prefix_n, hll, hlr, left, parent, edge, queue, q_count);

@@ -21,7 +21,7 @@
 //      chunk;
 //   2. the rest are found through two threshold tables: for every value v,
 //      which of a warp-block's 32 chunks has a minimum below v, and which of
-//      the window's 20 warp-blocks does - a few bit operations name the
+//      the window's warp-blocks does - a few bit operations name the
 //      first chunk holding a smaller value, and one 16-byte SIMD compare
 //      finds the position inside it;
 //   3. a split whose range reaches past the halo (0.04% of the splits of the
@@ -38,16 +38,39 @@ namespace gtc {
 
 constexpr int TW_THREADS = 512;
 constexpr int TW_C = 16;                   // splits per chunk (one lane's in-chunk pass)
-constexpr int TW_T = TW_THREADS * TW_C;    // 8192 splits per block
-constexpr int TW_H = 1024;                 // halo on each side
-constexpr int TW_W = TW_T + 2 * TW_H;      // 10240 window positions
-constexpr int TW_NCH = TW_W / TW_C;        // 640 chunks
-constexpr int TW_NWB = TW_NCH / 32;        // 20 warp-blocks of 32 chunks
 constexpr int TW_TV = 64;                  // prefix lengths are < 64
 constexpr int TW_MAXB = 512;               // cloud starts cached per window (batched)
 constexpr int TW_LQ = 128;                 // long-range splits a block resolves itself
-static_assert(TW_H % (32 * TW_C) == 0, "the tile starts on a warp-block");
-static_assert(TW_NWB <= 32, "one ballot covers the window's warp-blocks");
+
+// Window shape: T splits per block and a halo of H on each side.  Below about
+// half a million splits the kernel is one dependent chain per block (window,
+// tables, T / TW_THREADS splits per thread, then the block's long-range
+// splits), and blocks are too few to hide it, so a short tile is the faster
+// one; above, the halo a block loads and tabulates twice over costs more than
+// the chain.  Per launch on uniform 64-bit codes (us; the last column is the
+// 8192 + 2 x 1024 window that was used at every size before):
+//   splits    1024 + 2 x 512   2048 + 2 x 512   4096 + 2 x 512   8192 + 2 x 1024
+//   4,096         8.4              10.3             12.4             12.5
+//   120,000      10.3              10.5             14.5             22.7
+//   400,000      12.4              12.5             14.6             22.7
+//   1,048,576    19.5              18.6             18.6             22.7
+//   4,000,000    56.9              46.9             44.4             49.4
+//   10,000,000  131.2             106.5             96.9            100.5
+template <int T_, int H_>
+struct TwShape {
+  static constexpr int T = T_;
+  static constexpr int H = H_;
+  static constexpr int W = T + 2 * H;      // window positions
+  static constexpr int NCH = W / TW_C;     // chunks
+  static constexpr int NWB = NCH / 32;     // warp-blocks of 32 chunks
+  static_assert(H % (32 * TW_C) == 0 && T % (32 * TW_C) == 0, "the tile is whole warp-blocks");
+  static_assert(T <= TW_THREADS * TW_C, "one in-chunk pass per lane");
+  static_assert(NWB <= 32, "one ballot covers the window's warp-blocks");
+};
+using TwSmall = TwShape<1024, 512>;
+using TwLarge = TwShape<4096, 512>;
+using TwSegLarge = TwShape<8192, 1024>;     // batches, where each block also finds its clouds: a build of 83.5M points takes 4.68 ms, 4.73 with TwLarge
+constexpr uint32_t TW_SMALL_MAX = 700000;  // splits up to which TwSmall is the faster shape (table above)
 
 // First index in a[0..n) with a[i] > x.
 __device__ __forceinline__ uint32_t upper_bound_u32(const uint32_t* a, uint32_t n, uint32_t x) {
@@ -60,21 +83,38 @@ __device__ __forceinline__ uint32_t upper_bound_u32(const uint32_t* a, uint32_t 
   return lo;
 }
 
+// upper_bound_u32 by a whole warp, 32 probes a round (a thread's binary
+// search over 512 clouds is nine dependent loads, this one is two).
+__device__ __forceinline__ uint32_t warp_upper_bound_u32(const uint32_t* a, uint32_t n, uint32_t x) {
+  const uint32_t lane = threadIdx.x & 31;
+  uint32_t lo = 0, hi = n;  // the answer is in [lo, hi]
+  while (lo < hi) {         // warp-uniform
+    const uint32_t step = (hi - lo + 31) / 32;
+    const uint32_t p = lo + (lane + 1) * step - 1;
+    const uint32_t b = __ballot_sync(0xffffffffu, p < hi && a[p] <= x);  // a prefix of the lanes
+    const uint32_t c = __popc(b);
+    hi = min(hi, lo + (c + 1) * step - 1);
+    lo += c * step;
+  }
+  return lo;
+}
+
 // The cloud that owns position x of a run of offsets off[0..S] (off[S] > x):
 // the last c with off[c] <= x, which skips empty clouds.
 __device__ __forceinline__ uint32_t owner(const uint32_t* off, uint32_t S, uint32_t x) {
   return upper_bound_u32(off, S + 1, x) - 1;
 }
 
+template <class SH>
 struct TwSmem {
-  alignas(16) uint8_t d[TW_W];   // prefix length of pair w0 + i (0 = boundary)
-  alignas(16) uint8_t lr[TW_T];  // per split: (left answer in chunk << 4) | right answer in chunk
-  uint8_t cmin[TW_NCH];          // chunk minima
-  uint32_t t4[TW_NWB][TW_TV];    // t4[b][v] bit k: chunk 32b + k has a value < v
+  alignas(16) uint8_t d[SH::W];          // prefix length of pair w0 + i (0 = boundary)
+  alignas(16) uint8_t lr[SH::T];         // per split: (left answer in chunk << 4) | right answer in chunk
+  alignas(16) uint8_t cmin[SH::NCH];     // chunk minima
+  uint32_t t4[SH::NWB][TW_TV];   // t4[b][v] bit k: chunk 32b + k has a value < v
   uint32_t t9[TW_TV];            // t9[v] bit b: warp-block b has a value < v
   uint32_t cb[TW_MAXB];          // batched: cloud starts from c_first on
   uint32_t lq[TW_LQ];            // this block's splits whose range reaches past the window
-  uint32_t c_first, nb, lq_n;
+  uint32_t c_first, c_end, lq_n;
 };
 
 // Bytes of a word below t (prefix lengths < 128): bit 7 of each byte of
@@ -94,8 +134,9 @@ __device__ __forceinline__ uint32_t tw_below(uint32_t w, uint32_t tt) {
 // lengths never face each other across larger ones for distinct keys, so
 // strictly smaller and smaller-or-equal give the same answers; boundaries
 // (0) have no answers of their own and are never queried.
-__device__ __forceinline__ void tw_chunk_stack(TwSmem& s, int chunk) {
-  const uint4 dv = *reinterpret_cast<const uint4*>(s.d + TW_H + chunk * TW_C);
+template <class SH>
+__device__ __forceinline__ void tw_chunk_stack(TwSmem<SH>& s, int chunk) {
+  const uint4 dv = *reinterpret_cast<const uint4*>(s.d + SH::H + chunk * TW_C);
   const uint32_t a01 = __byte_perm(dv.x, dv.y, 0x5140), a23 = __byte_perm(dv.z, dv.w, 0x5140);
   const uint32_t c01 = __byte_perm(dv.x, dv.y, 0x7362), c23 = __byte_perm(dv.z, dv.w, 0x7362);
   const uint32_t wt[4] = {__byte_perm(a01, a23, 0x5410), __byte_perm(a01, a23, 0x7632), __byte_perm(c01, c23, 0x5410),
@@ -171,7 +212,8 @@ __device__ __forceinline__ int tw_last_below(const uint8_t* p, uint32_t t) {
 }
 
 // First window position after chunk c with a value < t, or -1.
-__device__ __forceinline__ int tw_next_tab(const TwSmem& s, int c, uint32_t t) {
+template <class SH>
+__device__ __forceinline__ int tw_next_tab(const TwSmem<SH>& s, int c, uint32_t t) {
   const int b = c >> 5, k = c & 31;
   const uint32_t m = s.t4[b][t] & ~((2u << k) - 1u);
   int cc;
@@ -187,7 +229,8 @@ __device__ __forceinline__ int tw_next_tab(const TwSmem& s, int c, uint32_t t) {
 }
 
 // Last window position before chunk c with a value < t, or -1.
-__device__ __forceinline__ int tw_prev_tab(const TwSmem& s, int c, uint32_t t) {
+template <class SH>
+__device__ __forceinline__ int tw_prev_tab(const TwSmem<SH>& s, int c, uint32_t t) {
   const int b = c >> 5, k = c & 31;
   const uint32_t m = s.t4[b][t] & ((1u << k) - 1u);
   int cc;
@@ -324,7 +367,7 @@ __device__ __forceinline__ void tw_warp_split(const K* codes, uint32_t x, uint32
 // queue (capacity: one entry per split), splits whose range reaches past
 // the halo are appended to it for radix_tree_slow_kernel; without one they
 // are searched here by their own thread.
-template <class K, bool SEG>
+template <class K, bool SEG, class SH>
 __global__ void __launch_bounds__(TW_THREADS, 4) radix_tree_window_kernel(
     const K* __restrict__ codes, const uint32_t* d_u, uint32_t u_host, const uint32_t* uoff, uint32_t S,
     uint8_t* __restrict__ prefix_n, uint8_t* __restrict__ hll, uint8_t* __restrict__ hlr,
@@ -332,16 +375,16 @@ __global__ void __launch_bounds__(TW_THREADS, 4) radix_tree_window_kernel(
     uint32_t* queue, uint32_t* q_count) {
   griddep_wait();
   constexpr int A = KeyTraits<K>::A;
-  __shared__ TwSmem s;
+  __shared__ TwSmem<SH> s;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t U = SEG ? uoff[S] : (d_u ? *d_u : u_host);
   const uint32_t P = U > 0 ? U - 1 : 0;  // pair positions [0, P)
   if (!SEG && blockIdx.x == 0 && tid == 0 && d_m) *d_m = P;
   // Positions fit in int: U < 2^30, and the window starts at most H before 0.
-  const int t0 = (int)blockIdx.x * TW_T;
-  const int x_end = min(t0 + TW_T, (int)(SEG ? U : P));
+  const int t0 = (int)blockIdx.x * SH::T;
+  const int x_end = min(t0 + SH::T, (int)(SEG ? U : P));
   if (t0 >= x_end) return;
-  const int w0 = t0 - TW_H;
+  const int w0 = t0 - SH::H;
   if (tid == 0) s.lq_n = 0;
 
   // 1. prefix lengths of the window's pairs.
@@ -349,7 +392,7 @@ __global__ void __launch_bounds__(TW_THREADS, 4) radix_tree_window_kernel(
   // and one more) give four lengths, stored as one word.
   const bool vec = (reinterpret_cast<uintptr_t>(codes) & 15) == 0;
 #pragma unroll
-  for (int g = tid; g < TW_W / 4; g += TW_THREADS) {
+  for (int g = tid; g < SH::W / 4; g += TW_THREADS) {
     const int x = w0 + 4 * g;
     uint32_t v = 0;
     if (vec && x >= 0 && x + 4 <= (int)P) {
@@ -380,25 +423,24 @@ __global__ void __launch_bounds__(TW_THREADS, 4) radix_tree_window_kernel(
     reinterpret_cast<uint32_t*>(s.d)[g] = v;
   }
   if (SEG) {
-    if (tid == 0) {
-      const uint32_t lo_pos = (uint32_t)max(w0, 0);
-      const uint32_t hi_pos = (uint32_t)min(w0 + TW_W, (int)U);
-      s.c_first = owner(uoff, S, lo_pos);
-      s.nb = upper_bound_u32(uoff, S + 1, hi_pos) - s.c_first;  // clouds starting at or before hi_pos
+    if (warp < 2) {  // the window's first cloud, and the clouds starting at or before its end
+      const uint32_t pos = warp ? (uint32_t)min(w0 + SH::W, (int)U) : (uint32_t)max(w0, 0);
+      const uint32_t k = warp_upper_bound_u32(uoff, S + 1, pos);
+      if (lane == 0) (warp ? s.c_end : s.c_first) = warp ? k : k - 1;
     }
     __syncthreads();
-    const uint32_t c_first = s.c_first, nb = s.nb;
+    const uint32_t c_first = s.c_first, nb = s.c_end - s.c_first;
     // A pair that straddles two clouds is no split: mark it as a boundary.
     for (uint32_t k = 1 + tid; k < nb; k += TW_THREADS) {
       const int p = (int)uoff[c_first + k] - 1 - w0;
-      if (p >= 0 && p < TW_W) s.d[p] = 0;
+      if (p >= 0 && p < SH::W) s.d[p] = 0;
     }
     for (uint32_t k = tid; k < min(nb, (uint32_t)TW_MAXB); k += TW_THREADS) s.cb[k] = uoff[c_first + k];
   }
   __syncthreads();
 
   // 2. chunk minima.
-  for (int c = tid; c < TW_NCH; c += TW_THREADS) {
+  for (int c = tid; c < SH::NCH; c += TW_THREADS) {
     const uint4 q = *reinterpret_cast<const uint4*>(s.d + c * TW_C);
     const uint32_t m = __vminu4(__vminu4(q.x, q.y), __vminu4(q.z, q.w));
     s.cmin[c] = (uint8_t)min(min(m & 0xffu, (m >> 8) & 0xffu), min((m >> 16) & 0xffu, m >> 24));
@@ -409,7 +451,7 @@ __global__ void __launch_bounds__(TW_THREADS, 4) radix_tree_window_kernel(
   // for threshold v is the OR of the bits of every entry whose minimum is
   // below v: each entry ORs its bit into row min + 1, then a prefix-OR over
   // the 64 rows (two per lane) completes them.
-  for (int b = warp; b < TW_NWB; b += TW_THREADS / 32) {
+  for (int b = warp; b < SH::NWB; b += TW_THREADS / 32) {
     s.t4[b][lane] = 0;
     s.t4[b][lane + 32] = 0;
     __syncwarp();
@@ -422,7 +464,7 @@ __global__ void __launch_bounds__(TW_THREADS, 4) radix_tree_window_kernel(
     s.t9[lane] = 0;
     s.t9[lane + 32] = 0;
     __syncwarp();
-    if (lane < TW_NWB) {
+    if (lane < SH::NWB) {
       const uint4 q0 = *reinterpret_cast<const uint4*>(s.cmin + lane * 32);
       const uint4 q1 = *reinterpret_cast<const uint4*>(s.cmin + lane * 32 + 16);
       const uint32_t m = __vminu4(__vminu4(__vminu4(q0.x, q0.y), __vminu4(q0.z, q0.w)),
@@ -433,7 +475,7 @@ __global__ void __launch_bounds__(TW_THREADS, 4) radix_tree_window_kernel(
     __syncwarp();
     tw_prefix_or_rows(s.t9, lane);
   }
-  tw_chunk_stack(s, tid);
+  if (SH::T == TW_THREADS * TW_C || tid < SH::T / TW_C) tw_chunk_stack(s, tid);
   __syncthreads();
 
   // 4. each split: its two answers, then its node.
@@ -447,8 +489,8 @@ __global__ void __launch_bounds__(TW_THREADS, 4) radix_tree_window_kernel(
     uint32_t U0 = 0, U1 = U;
     if (SEG) {
       uint32_t c;
-      if (s.nb <= (uint32_t)TW_MAXB) {
-        uint32_t lo = 0, hi = s.nb;  // last cached start <= x
+      if (s.c_end - s.c_first <= (uint32_t)TW_MAXB) {
+        uint32_t lo = 0, hi = s.c_end - s.c_first;  // last cached start <= x
         while (lo < hi) {
           const uint32_t mid = (lo + hi) >> 1;
           if (s.cb[mid] <= x) lo = mid + 1;
