@@ -223,7 +223,9 @@ def build_octree(pts: np.ndarray, key_bits: int, min_coord=0.0, rng=1024.0, flag
     parent = np.zeros(nn, np.int32)
     edge = np.zeros(nn, np.uint32)
     ps = np.zeros(nn, np.uint32)
-    nodes = np.zeros(nn + 1, OCTNODE_DTYPE)
+    # A radix node owns up to one octree node per level (single-child chains), which a few close points
+    # reach; large clouds average far below one.
+    nodes = np.zeros((21 if nn <= 1 << 16 else 1) * nn + 1, OCTNODE_DTYPE)
     counts = np.zeros(3, np.uint32)
     stage_ms = np.zeros(8, np.float64)
     t0 = time.perf_counter()
