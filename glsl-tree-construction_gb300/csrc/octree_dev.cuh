@@ -52,17 +52,28 @@ __device__ __forceinline__ void set_child(int4& lo, int4& hi, int w, int32_t v) 
   hi.w = (w == 7) ? v : hi.w;
 }
 
-// One 64-byte node as four 16-byte streaming stores: nothing in the build
+// One 64-byte node as two 32-byte streaming stores (whole sectors; four of 16
+// bytes where the caller's array is not 32-byte aligned): nothing in the build
 // reads the nodes back, so they are marked to leave L2 first and the radix
 // tree arrays the octree gathers from stay cached longer.
 __device__ __forceinline__ void store_node(gtc_octnode* nodes, uint32_t slot, int4 a, int4 b, float4 corner,
                                            float cell, int32_t nmask, int32_t lmask) {
   int4* p = reinterpret_cast<int4*>(nodes + slot);
-  __stcs(p + 0, a);
-  __stcs(p + 1, b);
-  __stcs(p + 2, make_int4(__float_as_int(corner.x), __float_as_int(corner.y), __float_as_int(corner.z),
-                          __float_as_int(corner.w)));
-  __stcs(p + 3, make_int4(__float_as_int(cell), nmask, lmask, 0));
+  const int4 c = make_int4(__float_as_int(corner.x), __float_as_int(corner.y), __float_as_int(corner.z),
+                           __float_as_int(corner.w));
+  if ((reinterpret_cast<uintptr_t>(nodes) & 31) == 0) {
+    asm volatile("st.global.cs.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(a.x), "r"(a.y), "r"(a.z),
+                 "r"(a.w), "r"(b.x), "r"(b.y), "r"(b.z), "r"(b.w)
+                 : "memory");
+    asm volatile("st.global.cs.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p + 2), "r"(c.x), "r"(c.y),
+                 "r"(c.z), "r"(c.w), "r"(__float_as_int(cell)), "r"(nmask), "r"(lmask), "r"(0)
+                 : "memory");
+  } else {
+    __stcs(p + 0, a);
+    __stcs(p + 1, b);
+    __stcs(p + 2, c);
+    __stcs(p + 3, make_int4(__float_as_int(cell), nmask, lmask, 0));
+  }
 }
 
 // D18: a single distinct key gives one root node without children.
