@@ -368,6 +368,13 @@ gtc_status pipeline(gtc_ctx* ctx, const float* pts, uint32_t n, float mn, float 
   gtc_status st = resolve_ws(ctx, ws, ws_bytes, pipeline_ws_bytes<K>(n));
   if (st != GTC_OK) return st;
   const Launch L = launch_of(ctx, stream);
+  // A cloud that fits one block's shared memory is built by that block alone
+  // (small.cu).  Stage events and the per-node tree method keep the stage
+  // kernels.
+  if (n <= SMALL_BUILD_MAX && !ctx->profiling && tree_get_method() == 1) {
+    GTC_TRY(ctx, launch_small_build<K>(L, reinterpret_cast<const float4*>(pts), n, mn, rg, *o));
+    return GTC_OK;
+  }
   char* w = reinterpret_cast<char*>(ws);
   K* keys_alt = reinterpret_cast<K*>(w);
   w += align_up((size_t)n * sizeof(K), 256);

@@ -585,6 +585,13 @@ cudaError_t launch_octree_link(const Launch& L, const K* codes, uint32_t m, cons
                                const uint8_t* hll, const uint8_t* hlr, const int32_t* left, const int32_t* parent,
                                const uint32_t* edge, const uint32_t* ps, gtc_octnode* nodes, uint32_t capacity);
 
+// The whole build of a cloud of at most SMALL_BUILD_MAX points by one block
+// (small.cu): every output of the stage kernels, no workspace.
+constexpr uint32_t SMALL_BUILD_MAX = 4096;
+template <class K>
+cudaError_t launch_small_build(const Launch& L, const float4* pts, uint32_t n, float mn, float rg,
+                               const gtc_octree_buffers& out);
+
 inline uint32_t ceil_div(uint64_t a, uint64_t b) { return (uint32_t)((a + b - 1) / b); }
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 

@@ -181,6 +181,43 @@ __device__ __forceinline__ void tw_prefix_or_rows(uint32_t* rows, int lane) {
   rows[lane + 32] = b;
 }
 
+// Smallest of a chunk's 16 prefix lengths.
+__device__ __forceinline__ uint32_t tw_chunk_min(const uint8_t* p) {
+  const uint4 q = *reinterpret_cast<const uint4*>(p);
+  const uint32_t m = __vminu4(__vminu4(q.x, q.y), __vminu4(q.z, q.w));
+  return min(min(m & 0xffu, (m >> 8) & 0xffu), min((m >> 16) & 0xffu, m >> 24));
+}
+
+// The threshold tables, each by one warp.  A table row for threshold v is the
+// OR of the bits of every entry whose minimum is below v: each entry ORs its
+// bit into row min + 1, then a prefix-OR over the 64 rows (two per lane)
+// completes them.
+template <class SH>
+__device__ __forceinline__ void tw_table4(TwSmem<SH>& s, int b) {
+  const int lane = threadIdx.x & 31;
+  s.t4[b][lane] = 0;
+  s.t4[b][lane + 32] = 0;
+  __syncwarp();
+  const uint32_t m = s.cmin[b * 32 + lane];
+  if (m + 1 < TW_TV) atomicOr(&s.t4[b][m + 1], 1u << lane);
+  __syncwarp();
+  tw_prefix_or_rows(s.t4[b], lane);
+}
+// Over the first nwb warp-blocks of the window.
+template <class SH>
+__device__ __forceinline__ void tw_table9(TwSmem<SH>& s, int nwb) {
+  const int lane = threadIdx.x & 31;
+  s.t9[lane] = 0;
+  s.t9[lane + 32] = 0;
+  __syncwarp();
+  if (lane < nwb) {
+    const uint32_t m = min(tw_chunk_min(s.cmin + lane * 32), tw_chunk_min(s.cmin + lane * 32 + 16));
+    if (m + 1 < TW_TV) atomicOr(&s.t9[m + 1], 1u << lane);
+  }
+  __syncwarp();
+  tw_prefix_or_rows(s.t9, lane);
+}
+
 // First / last byte of a 16-byte chunk below t (one exists).
 __device__ __forceinline__ int tw_first_below(const uint8_t* p, uint32_t t) {
   const uint4 q = *reinterpret_cast<const uint4*>(p);
@@ -440,41 +477,12 @@ __global__ void __launch_bounds__(TW_THREADS, 4) radix_tree_window_kernel(
   __syncthreads();
 
   // 2. chunk minima.
-  for (int c = tid; c < SH::NCH; c += TW_THREADS) {
-    const uint4 q = *reinterpret_cast<const uint4*>(s.d + c * TW_C);
-    const uint32_t m = __vminu4(__vminu4(q.x, q.y), __vminu4(q.z, q.w));
-    s.cmin[c] = (uint8_t)min(min(m & 0xffu, (m >> 8) & 0xffu), min((m >> 16) & 0xffu, m >> 24));
-  }
+  for (int c = tid; c < SH::NCH; c += TW_THREADS) s.cmin[c] = (uint8_t)tw_chunk_min(s.d + c * TW_C);
   __syncthreads();
 
-  // 3. the two threshold tables, and the per-lane in-chunk pass.  A table row
-  // for threshold v is the OR of the bits of every entry whose minimum is
-  // below v: each entry ORs its bit into row min + 1, then a prefix-OR over
-  // the 64 rows (two per lane) completes them.
-  for (int b = warp; b < SH::NWB; b += TW_THREADS / 32) {
-    s.t4[b][lane] = 0;
-    s.t4[b][lane + 32] = 0;
-    __syncwarp();
-    const uint32_t m = s.cmin[b * 32 + lane];
-    if (m + 1 < TW_TV) atomicOr(&s.t4[b][m + 1], 1u << lane);
-    __syncwarp();
-    tw_prefix_or_rows(s.t4[b], lane);
-  }
-  if (warp == 0) {
-    s.t9[lane] = 0;
-    s.t9[lane + 32] = 0;
-    __syncwarp();
-    if (lane < SH::NWB) {
-      const uint4 q0 = *reinterpret_cast<const uint4*>(s.cmin + lane * 32);
-      const uint4 q1 = *reinterpret_cast<const uint4*>(s.cmin + lane * 32 + 16);
-      const uint32_t m = __vminu4(__vminu4(__vminu4(q0.x, q0.y), __vminu4(q0.z, q0.w)),
-                                  __vminu4(__vminu4(q1.x, q1.y), __vminu4(q1.z, q1.w)));
-      const uint32_t m9 = min(min(m & 0xffu, (m >> 8) & 0xffu), min((m >> 16) & 0xffu, m >> 24));
-      if (m9 + 1 < TW_TV) atomicOr(&s.t9[m9 + 1], 1u << lane);
-    }
-    __syncwarp();
-    tw_prefix_or_rows(s.t9, lane);
-  }
+  // 3. the two threshold tables, and the per-lane in-chunk pass.
+  for (int b = warp; b < SH::NWB; b += TW_THREADS / 32) tw_table4(s, b);
+  if (warp == 0) tw_table9(s, SH::NWB);
   if (SH::T == TW_THREADS * TW_C || tid < SH::T / TW_C) tw_chunk_stack(s, tid);
   __syncthreads();
 

@@ -37,3 +37,50 @@ def test_tree_window_shapes(ctx, gtc_mod, oracle, key_bits, u):
     assert ctx.device_status() == 0
     for f in want:
         assert torch.equal(got[f], want[f]), f
+
+
+def small_clouds(n):
+    """Clouds of n points that take the one-block build's paths: spread and
+    clustered codes, one or few distinct codes, and runs of codes equal in
+    their top 32 bits around the length one thread sorts (16) and far over."""
+    g = np.random.Generator(np.random.PCG64(n))
+    uniform = W.uniform_points(n, seed=n)
+    yield "uniform", uniform
+    yield "clusters", W.gaussian_mixture_points(n, 3, 2.0, noise=0.1, seed=n)
+    yield "tight", W.gaussian_mixture_points(n, 1, 0.002, noise=0.002, seed=n)  # long runs
+    yield "equal", np.tile(uniform[:1], (n, 1))
+    yield "few", uniform[g.integers(0, min(n, 7), n)]
+    side = 1024.0 / (1 << 11)  # a cell of the top 33 bits holds at most two runs
+    for per in (15, 17):
+        corner = np.floor(g.random((n // per + 1, 3)) * (1 << 11)) * side
+        cube = uniform.copy()
+        cube[:, :3] = np.repeat(corner, per, axis=0)[:n] + g.random((n, 3)) * side
+        cube[:, :3] = np.minimum(cube[:, :3], 1023.99)
+        yield f"runs_{per}", cube[g.permutation(n)]
+
+
+@pytest.mark.parametrize("key_bits", [32, 64])
+@pytest.mark.parametrize("n", [1, 2, 3, 31, 33, 1023, 1024, 1025, 2047, 2048, 2049, 4095, 4096, 4097])
+def test_one_block_build(ctx, gtc_mod, oracle, key_bits, n):
+    """One block up to 4,096 points, the stage kernels above: every output
+    against the oracle, also under capture and at a node capacity one short."""
+    import torch
+
+    from test_gpu_pipeline import _cmp
+
+    for name, pts in small_clouds(n):
+        d = torch.from_numpy(pts).cuda()
+        exp, _ = oracle.build_octree(pts, key_bits)
+        plan = gtc_mod.OctreePlan(ctx, n, key_bits, nodes_capacity=exp["n_oct_nodes"])
+        plan.launch(d)
+        _cmp(plan.result(), exp, key_bits, (name, n))
+        plan.nodes.zero_()
+        plan.capture(d)
+        plan.nodes.zero_()
+        plan.replay()
+        torch.cuda.synchronize()
+        _cmp(plan.result(), exp, key_bits, (name, n, "graph"))
+    short = gtc_mod.OctreePlan(ctx, n, key_bits, nodes_capacity=max(exp["n_oct_nodes"] - 1, 1))
+    short.launch(d)
+    assert short.counts_host()[2] == exp["n_oct_nodes"]
+    assert ctx.device_status_code() == (7 if exp["n_oct_nodes"] > 1 else 0)
