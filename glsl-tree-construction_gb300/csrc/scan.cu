@@ -16,10 +16,171 @@ constexpr int SCAN_THREADS = 512;
 constexpr int SCAN_IPT = 9;  // odd: conflict-free blocked reads of 32-bit words
 constexpr int SCAN_TILE = SCAN_THREADS * SCAN_IPT;
 
-// Workspace: [0] tile counter, [1..63] spare, [64..64+tiles) descriptors.
+// Workspace: [0] tile counter, [1..63] spare, then descriptors: one per tile,
+// or one per block of a row kernel (at most RW_MAX_BLOCKS of them).
+constexpr uint32_t RW_MAX_BLOCKS = 1024;
 size_t scan_workspace_bytes(uint32_t n) {
-  const uint32_t tiles = ceil_div(n > 0 ? n : 1, SCAN_TILE) + 1;
+  const uint32_t tiles = max(ceil_div(n > 0 ? n : 1, SCAN_TILE) + 1, RW_MAX_BLOCKS);
   return align_up((64 + (size_t)tiles) * 4, 256);
+}
+
+// ------------------------------------------------------------ row scans --
+// Sizes that one resident wave of blocks holds in registers: every warp loads
+// its ROWS rows at once, the block posts its total and adds up the totals of
+// the lower blocks (cs_block_prefix), and the rows are written from registers:
+// one read of the input, one round of loads, one wait.  The kernels below read
+// their segments twice, row after row, or chain a look-back from tile to tile.
+// Launch to launch with the memset before it, node offsets and in-place unique
+// of 64-bit keys (us; before: the kernels below):
+//   items        node offsets   before      unique   before
+//   120,000          6.2          6.3          6.2      8.7
+//   1,048,576        8.2         11.4          8.8     17.3
+//   4,000,000       11.1         19.0           -      40.6
+// ROWS is the smallest that keeps the grid within one block per SM: every
+// block polls all lower blocks' totals, so more blocks cost more than more
+// rows (1,048,576 items in 256 blocks: 13.2 and 12.2).  The largest ROWS may
+// take two blocks per SM, which is still faster than the second read.
+
+// Inclusive scan with the node-offset rules of scan_kernel; a row is 128
+// items, one uint4 per lane, so in/out must be 16-byte aligned.  in holds at
+// least n_in items (rows are loaded before the count is known; items past the
+// limit add nothing).  in == out is fine: a warp reads and writes its own rows.
+template <int ROWS>
+__global__ void __launch_bounds__(CS_THREADS) row_scan_kernel(const uint32_t* in,
+                                                              uint32_t* out, uint32_t count_host,
+                                                              const uint32_t* d_u, uint32_t n_in, int node_offsets,
+                                                              uint32_t* ws, uint32_t* d_o, uint32_t* status) {
+  griddep_wait();
+  __shared__ uint32_t s_seg[CS_WARPS];
+  __shared__ uint32_t s_red[CS_WARPS];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t beg = (blockIdx.x * CS_WARPS + warp) * (ROWS * 128) + 4 * lane;
+  uint4 v[ROWS];
+#pragma unroll
+  for (int j = 0; j < ROWS; ++j) {
+    const uint32_t i = beg + j * 128;
+    v[j] = make_uint4(0, 0, 0, 0);
+    if (i + 4 <= n_in) {
+      v[j] = *reinterpret_cast<const uint4*>(in + i);
+    } else if (i < n_in) {
+      v[j].x = in[i];
+      if (i + 1 < n_in) v[j].y = in[i + 1];
+      if (i + 2 < n_in) v[j].z = in[i + 2];
+    }
+  }
+  const uint32_t count = d_u ? *d_u : count_host;
+  const uint32_t limit = node_offsets ? (count > 0 ? count - 1 : 0) : count;
+  uint32_t run = 0;
+#pragma unroll
+  for (int j = 0; j < ROWS; ++j) {  // each row's running sum within the warp's segment
+    const uint32_t i = beg + j * 128;
+    v[j].x = i + 0 < limit ? v[j].x : 0u;
+    v[j].y = (i + 1 < limit ? v[j].y : 0u) + v[j].x;
+    v[j].z = (i + 2 < limit ? v[j].z : 0u) + v[j].y;
+    v[j].w = (i + 3 < limit ? v[j].w : 0u) + v[j].z;
+    const uint32_t inc = warp_inclusive_sum(v[j].w);
+    const uint32_t base = run + inc - v[j].w;
+    v[j].x += base;
+    v[j].y += base;
+    v[j].z += base;
+    v[j].w += base;
+    run += __shfl_sync(0xffffffffu, inc, 31);
+  }
+  if (lane == 0) s_seg[warp] = run;
+  const uint32_t pre = cs_block_prefix(ws + 64, s_seg, s_red, status) + s_seg[warp];
+#pragma unroll
+  for (int j = 0; j < ROWS; ++j) {
+    const uint32_t i = beg + j * 128;
+    v[j].x += pre;
+    v[j].y += pre;
+    v[j].z += pre;
+    v[j].w += pre;
+    if (node_offsets && i == 0) v[j].x = 0;
+    if (i + 4 <= count) {
+      *reinterpret_cast<uint4*>(out + i) = v[j];
+    } else {
+      if (i + 0 < count) out[i + 0] = v[j].x;
+      if (i + 1 < count) out[i + 1] = v[j].y;
+      if (i + 2 < count) out[i + 2] = v[j].z;
+    }
+    if (node_offsets && d_o && count > 0 && i <= count - 1 && count - 1 < i + 4) {
+      const uint32_t q = count - 1 - i;
+      *d_o = 1 + (q == 0 ? v[j].x : q == 1 ? v[j].y : q == 2 ? v[j].z : v[j].w);
+    }
+  }
+  if (node_offsets && d_o && count == 0 && blockIdx.x == 0 && tid == 0) *d_o = 0;
+}
+
+// Unique.  A row is 32 keys.  In place (kin == kout) too: a block writes only
+// below the end of its own input, after every lower block has posted its
+// total, and a block posts only after all its keys and values have arrived
+// (IN_PLACE makes the barrier before the post depend on the values; the count
+// depends on the keys).  A block's first key's predecessor may be rewritten by
+// its own block only with the same key (no key before it dropped).
+template <class K, bool HAS_VALS, int ROWS, bool IN_PLACE>
+__global__ void __launch_bounds__(CS_THREADS) row_unique_kernel(const K* kin, const uint32_t* vin, K* kout,
+                                                                uint32_t* vout, uint32_t n, uint32_t* ws,
+                                                                uint32_t* d_count, uint32_t* status) {
+  griddep_wait();
+  __shared__ uint32_t s_seg[CS_WARPS];
+  __shared__ uint32_t s_red[CS_WARPS];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t lt = (1u << lane) - 1u;
+  const uint32_t beg = (blockIdx.x * CS_WARPS + warp) * (ROWS * 32) + lane;
+  K k[ROWS];
+  uint32_t v[ROWS];
+#pragma unroll
+  for (int j = 0; j < ROWS; ++j) {
+    const uint32_t i = beg + j * 32;
+    k[j] = i < n ? kin[i] : K(0);
+    if (HAS_VALS) v[j] = i < n ? vin[i] : 0u;
+  }
+  K carry = (lane == 0 && beg > 0 && beg < n) ? kin[beg - 1] : K(0);  // lane 0: the key before the row
+  uint32_t keep = 0, cnt = 0;  // bit j: this lane's key of row j stays
+#pragma unroll
+  for (int j = 0; j < ROWS; ++j) {
+    const uint32_t i = beg + j * 32;
+    K prev = (K)__shfl_up_sync(0xffffffffu, k[j], 1);
+    if (lane == 0) prev = carry;
+    const bool kp = i < n && (i == 0 || k[j] != prev);
+    keep |= (uint32_t)kp << j;
+    cnt += __popc(__ballot_sync(0xffffffffu, kp));
+    carry = (K)__shfl_sync(0xffffffffu, k[j], 31);
+  }
+  if (lane == 0) s_seg[warp] = cnt;
+  if (IN_PLACE && HAS_VALS) {
+    uint32_t x = 0;
+#pragma unroll
+    for (int j = 0; j < ROWS; ++j) x |= v[j];
+    if (__syncthreads_or(x == ~0u && cnt > 32u * ROWS)) return;  // never taken (a warp keeps at most its keys)
+  }
+  uint32_t run = cs_block_prefix(ws + 64, s_seg, s_red, status) + s_seg[warp];
+#pragma unroll
+  for (int j = 0; j < ROWS; ++j) {
+    const bool kp = (keep >> j) & 1u;
+    const uint32_t bal = __ballot_sync(0xffffffffu, kp);
+    if (kp) {
+      const uint32_t o = run + __popc(bal & lt);
+      kout[o] = k[j];
+      if (HAS_VALS) vout[o] = v[j];
+    }
+    run += __popc(bal);
+  }
+  // The last warp of the last block ends at n: its running count is u.
+  if (d_count && blockIdx.x == gridDim.x - 1 && warp == CS_WARPS - 1 && lane == 0) *d_count = run;
+}
+
+// Blocks of a row kernel for n items at `per_block` each, or 0 if one
+// resident wave of at most `per_sm` blocks per SM does not hold them.
+static uint32_t row_grid(const Launch& L, const void* kern, uint32_t n, uint32_t per_block, uint32_t per_sm) {
+  const uint32_t g = ceil_div(n, per_block);
+  if (g > RW_MAX_BLOCKS || g > per_sm * (uint32_t)L.num_sms) return 0u;
+  int occ = 0;
+  if (kernel_setup(kern, CS_THREADS, 0, &occ) != cudaSuccess) {
+    cudaGetLastError();
+    return 0u;
+  }
+  return g <= (uint32_t)occ * (uint32_t)L.num_sms ? g : 0u;
 }
 
 // --------------------------------------------------------- segment scans --
@@ -335,15 +496,37 @@ __global__ void __launch_bounds__(SCAN_THREADS) unique_kernel(const K* kin, cons
   if (tid == 0 && base + valid == n && d_count) *d_count = out + total;
 }
 
+// The row kernel of the smallest ROWS that holds n keys; false if none does.
+template <class K, bool HV, bool IP, int ROWS>
+static bool launch_row_unique(const Launch& L, const K* kin, const uint32_t* vin, K* kout, uint32_t* vout, uint32_t n,
+                              uint32_t* d_count, uint32_t* w, cudaError_t* e) {
+  auto kern = row_unique_kernel<K, HV, ROWS, IP>;
+  const uint32_t g = row_grid(L, (const void*)kern, n, ROWS * CS_THREADS, ROWS < 16 ? 1u : 2u);
+  if (g == 0) {
+    if constexpr (ROWS < 16) return launch_row_unique<K, HV, IP, ROWS * 2>(L, kin, vin, kout, vout, n, d_count, w, e);
+    return false;
+  }
+  *e = L.ws_zeroed ? cudaSuccess : cudaMemsetAsync(w, 0, (64 + (size_t)g) * 4, L.stream);
+  if (*e == cudaSuccess)
+    *e = launch_kernel(L, kern, g, CS_THREADS, 0, kin, vin, kout, vout, n, w, d_count, L.status);
+  return true;
+}
+
 template <class K>
 cudaError_t launch_unique(const Launch& L, const K* kin, const uint32_t* vin, K* kout, uint32_t* vout, uint32_t n,
                           uint32_t* d_count, void* ws) {
   uint32_t* w = reinterpret_cast<uint32_t*>(ws);
   const uint32_t tiles = ceil_div(n, SCAN_TILE);
-  cudaError_t e = L.ws_zeroed ? cudaSuccess : cudaMemsetAsync(w, 0, (64 + (size_t)tiles) * 4, L.stream);
-  if (e != cudaSuccess) return e;
+  cudaError_t e = cudaSuccess;
   if (n == 0) return d_count ? cudaMemsetAsync(d_count, 0, 4, L.stream) : cudaSuccess;
-  if (kin != kout && vin != vout) {
+  const bool apart = kin != kout && vin != vout;
+  if (vin ? (apart ? launch_row_unique<K, true, false, 2>(L, kin, vin, kout, vout, n, d_count, w, &e)
+                   : launch_row_unique<K, true, true, 2>(L, kin, vin, kout, vout, n, d_count, w, &e))
+          : launch_row_unique<K, false, false, 2>(L, kin, nullptr, kout, nullptr, n, d_count, w, &e))
+    return e;
+  e = L.ws_zeroed ? cudaSuccess : cudaMemsetAsync(w, 0, (64 + (size_t)tiles) * 4, L.stream);
+  if (e != cudaSuccess) return e;
+  if (apart) {
     const void* kern = vin ? (const void*)chunk_unique_kernel<K, true> : (const void*)chunk_unique_kernel<K, false>;
     const uint32_t g = chunk_grid(L, kern, n);
     if (g) {
@@ -446,13 +629,35 @@ __global__ void __launch_bounds__(SCAN_THREADS) scan_kernel(const uint32_t* in, 
   }
 }
 
+template <int ROWS>
+static bool launch_row_scan(const Launch& L, const uint32_t* in, uint32_t* out, uint32_t count_host,
+                            const uint32_t* d_u, uint32_t n_max, int node_offsets, uint32_t* d_o, uint32_t* w,
+                            cudaError_t* e) {
+  auto kern = row_scan_kernel<ROWS>;
+  const uint32_t g = row_grid(L, (const void*)kern, n_max, ROWS * 128 * CS_WARPS, ROWS < 8 ? 1u : 2u);
+  if (g == 0) {
+    if constexpr (ROWS < 8)
+      return launch_row_scan<ROWS * 2>(L, in, out, count_host, d_u, n_max, node_offsets, d_o, w, e);
+    return false;
+  }
+  *e = L.ws_zeroed ? cudaSuccess : cudaMemsetAsync(w, 0, (64 + (size_t)g) * 4, L.stream);
+  if (*e == cudaSuccess)
+    *e = launch_kernel(L, kern, g, CS_THREADS, 0, in, out, count_host, d_u,
+                       node_offsets ? n_max - 1 : n_max, node_offsets, w, d_o, L.status);
+  return true;
+}
+
 static cudaError_t launch_scan(const Launch& L, const uint32_t* in, uint32_t* out, uint32_t count_host,
                                const uint32_t* d_u, uint32_t n_max, int node_offsets, uint32_t* d_o, void* ws) {
   uint32_t* w = reinterpret_cast<uint32_t*>(ws);
   const uint32_t tiles = ceil_div(n_max > 0 ? n_max : 1, SCAN_TILE);
-  cudaError_t e = L.ws_zeroed ? cudaSuccess : cudaMemsetAsync(w, 0, (64 + (size_t)tiles) * 4, L.stream);
-  if (e != cudaSuccess) return e;
   const bool aligned = ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15u) == 0;
+  cudaError_t e = cudaSuccess;
+  if (aligned &&
+      launch_row_scan<1>(L, in, out, count_host, d_u, n_max, node_offsets, d_o, w, &e))
+    return e;
+  e = L.ws_zeroed ? cudaSuccess : cudaMemsetAsync(w, 0, (64 + (size_t)tiles) * 4, L.stream);
+  if (e != cudaSuccess) return e;
   const uint32_t g = aligned ? chunk_grid(L, (const void*)chunk_scan_kernel, n_max) : 0u;
   if (g)
     return launch_kernel(L, chunk_scan_kernel, g, CS_THREADS, 0, in, out, count_host, d_u, node_offsets, w, d_o,

@@ -84,3 +84,45 @@ def test_one_block_build(ctx, gtc_mod, oracle, key_bits, n):
     short.launch(d)
     assert short.counts_host()[2] == exp["n_oct_nodes"]
     assert ctx.device_status_code() == (7 if exp["n_oct_nodes"] > 1 else 0)
+
+
+# Row kernels: 2..16 rows of 32 keys, 1..8 rows of 128 items per warp, 16 warps
+# per block, one block per SM (two at the most rows); the sizes lie at a warp's,
+# a block's and (for 152 SMs) each form's limit.
+@pytest.mark.parametrize("n", [1, 2, 31, 33, 127, 129, 511, 513, 1023, 1024, 1025, 2048, 2049, 155_648, 155_649,
+                               311_297, 622_593, 1_245_185, 2_490_369, 4_980_737])
+@pytest.mark.parametrize("dups", [1, 40])
+def test_row_scans(ctx, n, dups):
+    """unique in place (both key widths, with and without values), the
+    inclusive scan (aligned, unaligned, in place) and the node offsets, against
+    numpy."""
+    import torch
+
+    g = np.random.Generator(np.random.PCG64(n + dups))
+    for kd, td in ((np.uint32, np.int32), (np.uint64, np.int64)):
+        keys = np.sort(g.integers(0, max(2 * n // dups, 2), n).astype(kd)) + kd(7)
+        want, first = np.unique(keys, return_index=True)
+        for with_vals in (True, False):
+            k = torch.from_numpy(keys.view(td).copy()).cuda()
+            v = torch.arange(n, dtype=torch.int32, device="cuda") if with_vals else None
+            u = int(ctx.unique(k, v).item())
+            assert u == want.size
+            assert np.array_equal(k[:u].cpu().numpy().view(kd), want)
+            if with_vals:
+                assert np.array_equal(v[:u].cpu().numpy(), first)
+    data = g.integers(0, 9, n + 8).astype(np.int32)
+    d = torch.from_numpy(data).cuda()
+    for lo in (0, 3, 4):
+        assert np.array_equal(ctx.partial_sum(d, lo, lo + n).cpu().numpy(), np.cumsum(data[lo:lo + n], dtype=np.int32))
+    e = torch.from_numpy(data[:n]).cuda()
+    ps, o = ctx.node_offsets(e, n)
+    want = np.concatenate((np.cumsum(data[:n], dtype=np.int32), [0]))
+    want[n] = want[n - 1]
+    want[0] = 0
+    assert np.array_equal(ps.cpu().numpy(), want)
+    assert int(o.item()) == 1 + want[n]
+    L = ctx.L
+    ctx.check(L.gtc_partial_sum_u32(ctx.h, d.data_ptr(), 0, n, d.data_ptr(), None, 0,
+                                    torch.cuda.current_stream().cuda_stream))
+    assert np.array_equal(d[:n].cpu().numpy(), np.cumsum(data[:n], dtype=np.int32))
+    assert ctx.device_status() == 0
