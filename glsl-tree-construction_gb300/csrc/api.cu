@@ -246,6 +246,8 @@ gtc_status sort_pairs_impl(gtc_ctx* ctx, K* keys, uint32_t* vals, K* keys_alt, u
   gtc_status st = resolve_ws(ctx, ws, ws_bytes, sort_workspace_bytes(n, passes, 0));
   if (st != GTC_OK) return st;
   const Launch L = launch_of(ctx, stream);
+  Launch Lp = L;  // the passes: programmatic dependent launches (not with stage events between them)
+  Lp.pdl = !ctx->profiling;
   const SortWorkspace Wk = carve_sort_workspace(ws, n, passes, 0);
   GTC_TRY(ctx, cudaMemsetAsync(Wk.header, 0, Wk.header_words * 4, S(stream)));
   if (ctx->skip_first_tile) {
@@ -267,7 +269,7 @@ gtc_status sort_pairs_impl(gtc_ctx* ctx, K* keys, uint32_t* vals, K* keys_alt, u
     std::vector<cudaEvent_t> ev;
     if (ctx->profiling)
       for (int i = 0; i < 2 * passes; ++i) ev.push_back(get_event(ctx));
-    GTC_TRY(ctx, launch_onesweep_passes<K>(L, keys, vals, keys_alt, vals_alt, n, begin_bit, end_bit, Wk, passes,
+    GTC_TRY(ctx, launch_onesweep_passes<K>(Lp, keys, vals, keys_alt, vals_alt, n, begin_bit, end_bit, Wk, passes,
                                            &in_alt, ev.empty() ? nullptr : ev.data(), -1, false, db));
     for (int p = 0; p < (int)ev.size() / 2; ++p) ctx->pending.push_back({ev[2 * p], ev[2 * p + 1], GTC_STAGE_ONESWEEP});
   }

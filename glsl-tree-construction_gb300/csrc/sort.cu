@@ -132,6 +132,7 @@ __global__ void __launch_bounds__(THREADS) global_hist_kernel(const K* __restric
                                                               uint32_t* bin_offsets, uint32_t* done,
                                                               uint32_t* zero_ptr, size_t zero_words,
                                                               const uint32_t* run_if) {
+  griddep_wait();
   if (run_if && *run_if == 0) return;
   __shared__ uint32_t s_hist[MAX_PASSES][RADIX];
   __shared__ uint32_t s_last;
@@ -701,6 +702,112 @@ __global__ void __launch_bounds__(THREADS, MINB) onesweep_kernel(const K* __rest
   }
 }
 
+// ------------------------------------------------- one-wave onesweep ------
+// The same pass for inputs whose tiles are all resident at once: a pass is
+// then one chain of dependent steps, and the chain is what it costs.  Against
+// onesweep_kernel: no ticket (block b takes tile b; it waits only on lower
+// blocks, all resident), keys requested at once, warp counters cleared by
+// their own warp, short tiles (4 or 8 keys per thread: fewer ranking steps in
+// a row, more SMs), and a look-back over 32 descriptors per round trip, since
+// the tiles publish at about the same time.  Whole sorts of uniform pairs,
+// histogram included (us; before: 256 x 16 tiles by ticket):
+//   pairs      u32 before   4 keys   8 keys    u64 before   4 keys   8 keys
+//   16,384        28.3       18.5     20.5        56.4       34.0     37.5
+//   65,536        32.0       24.4     26.5        61.9       43.9     47.4
+//   120,000       33.6       32.9     29.9        65.0       59.4     53.4
+//   250,000       39.3         -      40.4        74.2         -      70.6
+// first_tile: 1 leaves tile 0 unsorted (gtc_debug_skip_first_tile).
+template <class K, int THREADS, int KPT, bool HAS_VALS>
+__global__ void __launch_bounds__(THREADS) onesweep_wave_kernel(const K* __restrict__ kin,
+                                                                const uint32_t* __restrict__ vin,
+                                                                K* __restrict__ kout, uint32_t* __restrict__ vout,
+                                                                uint32_t n, int shift, uint32_t dmask,
+                                                                const uint32_t* __restrict__ bin_off,
+                                                                uint32_t* __restrict__ desc,
+                                                                const uint32_t* __restrict__ first_tile,
+                                                                uint32_t* __restrict__ status,
+                                                                const uint32_t* run_if) {
+  griddep_wait();
+  if (run_if && *run_if == 0) return;
+  using S = OnesweepSmem<K, THREADS, KPT>;
+  constexpr int WARPS = S::WARPS;
+  constexpr int TILE = S::TILE;
+  static_assert(THREADS == RADIX, "one thread per digit");
+  static_assert(TILE <= 65536, "warp ranks are packed in 16 bits");
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  S& s = *reinterpret_cast<S*>(smem_raw);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t lt = (1u << lane) - 1u;
+  const uint32_t tile = blockIdx.x;
+  const uint32_t tile_base = tile * TILE;
+  const uint32_t skip = *first_tile;
+  const uint32_t bin0 = bin_off[tid];
+
+  K key[KPT];
+  uint32_t val[KPT], rank[KPT];
+  const uint32_t wbase = tile_base + warp * 32 * KPT + lane;
+#pragma unroll
+  for (int j = 0; j < KPT; ++j) {
+    const uint32_t pos = wbase + j * 32;
+    key[j] = (pos < n) ? kin[pos] : ~K(0);
+    if (HAS_VALS) val[j] = (pos < n) ? (vin ? vin[pos] : pos) : 0u;
+  }
+  uint32_t* my = s.warp_hist[warp];
+#pragma unroll
+  for (int i = 0; i < RADIX / 32; ++i) my[i * 32 + lane] = 0;
+  __syncwarp();
+#pragma unroll
+  for (int j = 0; j < KPT; ++j) {
+    const uint32_t d = (uint32_t)(key[j] >> shift) & dmask;
+    const uint32_t peers = warp_peers<8>(d);
+    const int leader = 31 - __clz(peers);
+    uint32_t b = 0;
+    if (lane == leader) b = atomicAdd(&my[d], (uint32_t)__popc(peers));
+    b = __shfl_sync(0xffffffffu, b, leader);
+    rank[j] = (b + __popc(peers & lt)) | (d << 16);
+  }
+  __syncthreads();
+  if (tile < skip) return;
+  uint32_t count = 0;
+#pragma unroll
+  for (int w = 0; w < WARPS; ++w) {
+    const uint32_t c = s.warp_hist[w][tid];
+    s.warp_hist[w][tid] = count;
+    count += c;
+  }
+  st_relaxed(desc + (size_t)tile * RADIX + tid, (count << 2) | (tile == 0 ? FLAG_INCLUSIVE : FLAG_AGGREGATE));
+  const uint32_t digit_off = scan256_exclusive<THREADS>(count, s.warp_sums);
+#pragma unroll
+  for (int w = 0; w < WARPS; ++w) s.warp_hist[w][tid] += digit_off;
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < KPT; ++j) {
+    const uint32_t local = my[rank[j] >> 16] + (rank[j] & 0xffffu);
+    s.keys[local] = key[j];
+    if (HAS_VALS) s.vals[local] = val[j];
+  }
+  uint32_t excl = 0;
+  if (tile > 0) {
+    excl = lookback_window<32, RADIX>(desc, tile, tid, status);
+    st_relaxed(desc + (size_t)tile * RADIX + tid, ((excl + count) << 2) | FLAG_INCLUSIVE);
+  }
+  s.global_base[tid] = bin0 + excl - digit_off;
+  __syncthreads();
+  const uint32_t valid = min((uint32_t)TILE, n - tile_base);
+#pragma unroll
+  for (int j = 0; j < KPT; ++j) {
+    const uint32_t i = j * THREADS + tid;
+    if (i < valid) {
+      const K k = s.keys[i];
+      const uint32_t o = s.global_base[(uint32_t)(k >> shift) & dmask] + i;
+      if (o < n) {  // as in onesweep_kernel: only a timed-out look-back gets past n
+        kout[o] = k;
+        if (HAS_VALS) vout[o] = s.vals[i];
+      }
+    }
+  }
+}
+
 // ------------------------------------------- persistent TMA onesweep ------
 // The same pass as onesweep_kernel, restructured so HBM never idles:
 //   * persistent CTAs (a few per SM) pull tile tickets in a loop;
@@ -901,9 +1008,10 @@ __global__ void __launch_bounds__(THREADS, (THREADS <= 256 ? 2 : 1)) onesweep_tm
 // ------------------------------------------------------------- variants ---
 // Tile shapes compiled in.  kind 0: one tile per CTA (onesweep_kernel);
 // kind 1: persistent TMA, __match_any_sync ranks; kind 2: persistent TMA,
-// ballot ranks.  The autotuner times them per key width
-// (gtc_sort_set_variant); TMA kinds need 16-byte aligned inputs and fall back
-// to kind 0 shapes otherwise.
+// ballot ranks; kind 4: kind 0 with L2 hints; kind 5: one resident wave
+// (onesweep_wave_kernel).  The autotuner times them per key width
+// (gtc_sort_set_variant); TMA kinds need 16-byte aligned inputs and kind 5
+// needs all tiles resident, and both fall back to kind 0 shapes otherwise.
 struct Variant {
   int threads;
   int kpt;
@@ -917,17 +1025,44 @@ constexpr Variant kVariants[] = {{256, 16, 0, 3, 0}, {384, 16, 0, 2, 0}, {512, 1
                                  {256, 16, 2, 1, 0}, {512, 8, 2, 1, 0},  {256, 24, 2, 1, 0}, {256, 16, 0, 4, 0},
                                  {512, 8, 0, 2, 0},  {384, 12, 0, 3, 0}, {256, 16, 0, 3, 1}, {384, 16, 0, 2, 1},
                                  {512, 12, 0, 2, 1}, {256, 24, 0, 2, 1}, {256, 16, 4, 3, 0}, {512, 12, 4, 2, 1},
-                                 {256, 16, 4, 3, 2}, {512, 12, 4, 2, 2}, {384, 16, 4, 2, 2}};
+                                 {256, 16, 4, 3, 2}, {512, 12, 4, 2, 2}, {384, 16, 4, 2, 2}, {256, 4, 5, 1, 1},
+                                 {256, 8, 5, 1, 1},  {256, 16, 5, 1, 1}};
 constexpr int kNumVariants = sizeof(kVariants) / sizeof(kVariants[0]);
-static const int g_variant[2] = {0, 2};  // [u32, u64]: measured best on GB300 without tuning
+static const int g_variant[2] = {0, 2};  // [u32, u64]: what gtc_sort_get_variant reports with nothing pinned
 static std::atomic<int> g_pinned[2] = {{-1}, {-1}};  // gtc_sort_set_variant: overrides the tuned choice
+
+// Largest inputs of the one-wave variants (kind 5).  The short tiles' limits
+// bound the look-back descriptors of the workspace (one row of 256 words per
+// tile and pass); every one-wave launch also needs its tiles resident.
+constexpr int WAVE_4 = 19, WAVE_8 = 20, WAVE_16 = 21;  // their places in kVariants
+constexpr uint32_t WAVE_4_MAX = 160 * 1024, WAVE_8_MAX = 200 * 2048;
+constexpr uint32_t WAVE_4_USE = 96 * 1024, WAVE_8_USE = 250000;  // without a tuned or pinned choice
+static_assert(kVariants[WAVE_4].kind == 5 && kVariants[WAVE_4].kpt == 4 && kVariants[WAVE_8].kpt == 8 &&
+                  kVariants[WAVE_16].kpt == 16 && kNumVariants == 22,
+              "variant numbers");
 
 int sort_select_variant(int key_bits, int bits, uint32_t n) {
   const int w = key_bits == 64;
   const int pinned = g_pinned[w].load(std::memory_order_relaxed);
   if (pinned >= 0) return pinned;
   const int t = tuned_variant(key_bits, bits, n);
-  return (t >= 0 && t < kNumVariants) ? t : g_variant[w];
+  if (t >= 0 && t < kNumVariants) return t;
+  // Untuned: the one-wave tiles while the look-back stays short (crossings
+  // measured: 4 against 8 keys per thread at about 100,000 keys, 8 against
+  // the ticketed tiles at about 250,000; onesweep_wave_kernel has the times).
+  if (n <= WAVE_4_USE) return WAVE_4;
+  if (n <= WAVE_8_USE) return WAVE_8;
+  // Above, by how the tiles fill waves (resident tiles on 152 SMs: 304 of
+  // 6,144 keys, 456 of 4,608, 608 of 4,096 with variant 7, whose 64 registers
+  // only 32-bit keys fit without spilling).  Sort of uniform pairs (us):
+  //                  u32: var. 2  var. 9  var. 7    u64: var. 2  var. 9
+  //   1,048,576           63.8     70.5     71.7         123.7    141.1
+  //   2,000,000           85.7     77.4     83.3         177.5    157.1
+  //   4,000,000          132.4    128.3    128.4         280.6    274.5
+  //   16,777,216         433.2    424.4    412.9         942.7    972.0
+  if (n <= 1860000) return 2;
+  if (n <= (w ? 4200000u : 6000000u)) return 9;
+  return w ? 2 : 7;
 }
 
 template <class K, int THREADS, int KPT, bool HV, int MINB, int RANK, bool L2H = false>
@@ -941,6 +1076,23 @@ static cudaError_t launch_one(const Launch& L, const K* kin, const uint32_t* vin
   const uint32_t tiles = ceil_div(n, S::TILE);
   return launch_kernel(L, kern, tiles, THREADS, sizeof(S), kin, vin, kout, vout, n, shift, dmask, bin_off, desc,
                        tile_counter, L.status, L.run_if);
+}
+
+// false: the tiles do not all fit the GPU at once.
+template <class K, int THREADS, int KPT, bool HV>
+static bool launch_wave(const Launch& L, const K* kin, const uint32_t* vin, K* kout, uint32_t* vout, uint32_t n,
+                        int shift, uint32_t dmask, const uint32_t* bin_off, uint32_t* desc, uint32_t* tile_counter,
+                        cudaError_t* e) {
+  using S = OnesweepSmem<K, THREADS, KPT>;
+  auto kern = onesweep_wave_kernel<K, THREADS, KPT, HV>;
+  int per_sm = 1;
+  *e = kernel_setup(kern, THREADS, sizeof(S), &per_sm);
+  if (*e != cudaSuccess) return true;
+  const uint32_t tiles = ceil_div(n, S::TILE);
+  if (tiles > (uint32_t)(per_sm * L.num_sms)) return false;
+  *e = launch_kernel(L, kern, tiles, THREADS, sizeof(S), kin, vin, kout, vout, n, shift, dmask, bin_off, desc,
+                     tile_counter, L.status, L.run_if);
+  return true;
 }
 
 template <class K, int THREADS, int KPT, bool HV, bool MATCH>
@@ -966,6 +1118,16 @@ static cudaError_t launch_variant(int v, bool hv, const Launch& L, const K* kin,
   // one-tile-per-CTA kernel of the same tile width.
   const bool aligned = (reinterpret_cast<uintptr_t>(kin) & 15) == 0 && (!hv || (reinterpret_cast<uintptr_t>(vin) & 15) == 0);
   if ((kVariants[v].kind == 1 || kVariants[v].kind == 2) && (!aligned || (hv && !vin))) v = 0;
+  if (kVariants[v].kind == 5) {
+    cudaError_t e = cudaSuccess;
+#define GTC_WV(P)                                                                                              \
+  (hv ? launch_wave<K, 256, P, true>(L, kin, vin, kout, vout, n, shift, dmask, bin_off, desc, tc, &e)      \
+      : launch_wave<K, 256, P, false>(L, kin, vin, kout, vout, n, shift, dmask, bin_off, desc, tc, &e))
+    const bool done = v == WAVE_4 ? n <= WAVE_4_MAX && GTC_WV(4) : v == WAVE_8 ? n <= WAVE_8_MAX && GTC_WV(8) : GTC_WV(16);
+#undef GTC_WV
+    if (done) return e;
+    v = 0;
+  }
 #define GTC_OS(T, P, MB, RK)                                                                                   \
   return hv ? launch_one<K, T, P, true, MB, RK>(L, kin, vin, kout, vout, n, shift, dmask, bin_off, desc, tc) \
             : launch_one<K, T, P, false, MB, RK>(L, kin, vin, kout, vout, n, shift, dmask, bin_off, desc, tc)
@@ -1001,15 +1163,18 @@ static cudaError_t launch_variant(int v, bool hv, const Launch& L, const K* kin,
 #undef GTC_TMA
 }
 
-// Smallest tile of any variant: sizes the descriptor array for every variant.
-static int min_tile_keys() {
-  int t = 1 << 30;
-  for (const Variant& v : kVariants) t = t < v.threads * v.kpt ? t : v.threads * v.kpt;
-  return t;
+// Smallest tile of any variant that takes n keys: sizes the descriptor array
+// for every variant.
+static int min_tile_keys(uint32_t n) { return n <= WAVE_4_MAX ? 1024 : n <= WAVE_8_MAX ? 2048 : 4096; }
+static constexpr bool tiles_covered() {
+  for (const Variant& v : kVariants)
+    if (v.kind != 5 && v.threads * v.kpt < 4096) return false;
+  return true;
 }
+static_assert(tiles_covered(), "only the limited one-wave variants have tiles below 4,096 keys");
 
 size_t sort_workspace_bytes(uint32_t n, int passes, int /*tile_keys*/) {
-  const uint32_t tiles = ceil_div(n > 0 ? n : 1, (uint32_t)min_tile_keys());
+  const uint32_t tiles = ceil_div(n > 0 ? n : 1, (uint32_t)min_tile_keys(n));
   size_t words = 64 + 2 * (size_t)MAX_PASSES * RADIX;  // header + counts + bin offsets
   words = align_up(words, 64);
   words += (size_t)passes * tiles * RADIX;
@@ -1019,7 +1184,7 @@ size_t sort_workspace_bytes(uint32_t n, int passes, int /*tile_keys*/) {
 SortWorkspace carve_sort_workspace(void* ws, uint32_t n, int passes, int /*tile_keys*/) {
   SortWorkspace W;
   uint32_t* p = reinterpret_cast<uint32_t*>(ws);
-  W.tiles = ceil_div(n > 0 ? n : 1, (uint32_t)min_tile_keys());
+  W.tiles = ceil_div(n > 0 ? n : 1, (uint32_t)min_tile_keys(n));
   W.header = p;                              // [0] done, [1..8] tile counters
   W.counts = p + 64;                         // [passes][256]
   W.bin_offsets = p + 64 + MAX_PASSES * RADIX;
@@ -1030,13 +1195,20 @@ SortWorkspace carve_sort_workspace(void* ws, uint32_t n, int passes, int /*tile_
   return W;
 }
 
+// Blocks of T threads for a pass over n items at per_thread each; up to one
+// block per SM, four items per thread: the pass is then
+// a chain of loads, shared atomics and one round of global ones (120,000 64-bit
+// keys, whole sort: 56.9 us with 16 keys per thread, 52.5 with four).
+static uint32_t hist_blocks(const Launch& L, uint32_t n, uint32_t T, uint32_t per_thread) {
+  return max(ceil_div(n, T * per_thread), min(ceil_div(n, T * 4), (uint32_t)L.num_sms));
+}
+
 template <class K>
 cudaError_t launch_global_hist(const Launch& L, const K* keys, uint32_t n, int begin_bit, int end_bit,
                                const SortWorkspace& W, int passes, int db) {
   if (db < 1 || db > 8 || passes < 1 || passes > MAX_PASSES) return cudaErrorInvalidValue;
   constexpr int T = 512;
-  const uint32_t want = ceil_div(n, T * 16);
-  const uint32_t grid = max(1u, min(want, (uint32_t)L.num_sms * 2));
+  const uint32_t grid = max(1u, min(hist_blocks(L, n, T, 16), (uint32_t)L.num_sms * 2));
   global_hist_kernel<K, T><<<grid, T, 0, L.stream>>>(keys, n, begin_bit, end_bit, passes, db, W.counts,
                                                      W.bin_offsets, W.header, W.desc, W.desc_words, L.run_if);
   return cudaGetLastError();
@@ -1065,8 +1237,7 @@ cudaError_t launch_morton_hist(const Launch& L, const float4* pts, K* keys, uint
     cudaGetLastError();
     occ = 2;
   }
-  const uint32_t want = ceil_div(n, T * 8);
-  const uint32_t grid = max(1u, min(want, (uint32_t)(L.num_sms * occ)));
+  const uint32_t grid = max(1u, min(hist_blocks(L, n, T, 8), (uint32_t)(L.num_sms * occ)));
   return launch_kernel(L, kern, grid, T, 0, pts, keys, n, mn, rg, inv, W.counts, W.bin_offsets, W.header, W.desc,
                        W.desc_words);
 }

@@ -126,3 +126,57 @@ def test_row_scans(ctx, n, dups):
                                     torch.cuda.current_stream().cuda_stream))
     assert np.array_equal(d[:n].cpu().numpy(), np.cumsum(data[:n], dtype=np.int32))
     assert ctx.device_status() == 0
+
+
+@pytest.mark.parametrize("key_bits", [32, 64])
+@pytest.mark.parametrize("variant", [-1, 19, 20, 21])
+def test_one_wave_sort(ctx, key_bits, variant):
+    """The one-wave onesweep pass (default up to 250,000 keys, and pinned):
+    tile edges, the untuned choice's crossings, the variants' own limits and
+    one past them, narrow digits, unaligned inputs, the first-tile switch."""
+    import torch
+
+    kd, td = (np.uint32, np.int32) if key_bits == 32 else (np.uint64, np.int64)
+
+    def check(keys, lo, hi, off=0):
+        k = torch.from_numpy(keys.view(td).copy()).cuda()[off:]
+        v = torch.arange(keys.size, dtype=torch.int32, device="cuda")[off:]
+        want = keys[off:]
+        digits = (want >> kd(lo)) & kd((1 << (hi - lo)) - 1)
+        order = np.argsort(digits, kind="stable")
+        for vals in (v, None):
+            got = k.clone() if off == 0 else k
+            ctx.sort_pairs(got, vals, lo, hi)
+            assert np.array_equal(got.contiguous().cpu().numpy().view(kd), want[order]), (keys.size, lo, hi, off)
+            if vals is not None:
+                assert np.array_equal(vals.contiguous().cpu().numpy(), order.astype(np.int32) + off)
+            if off:
+                break
+
+    try:
+        ctx.set_sort_variant(key_bits, variant)
+        for n in (1, 31, 255, 257, 1023, 1024, 1025, 4097, 98_304, 98_305, 163_840, 163_841, 250_000, 250_001, 409_600,
+                  409_601):
+            check(W.config3_keys(n, key_bits, and_words=n % 4, seed=n), 0, key_bits)
+        for n in (5000, 120_007):
+            keys = W.config3_keys(n, key_bits, seed=n)
+            check(keys, 0, 30 if key_bits == 32 else 63)
+            check(keys, 3, 8)
+            check(keys, 0, key_bits, off=1)
+            check(np.full(n, 7, kd), 0, key_bits)
+        for db in (6, 7):
+            ctx.set_sort_digit_bits(key_bits, db)
+            check(W.config3_keys(70_001, key_bits, seed=db), 0, 40 if key_bits == 64 else 32)
+        ctx.set_sort_digit_bits(key_bits, -1)
+        assert ctx.device_status() == 0
+        ctx.set_spin_limit(1000)
+        ctx.debug_skip_first_tile()
+        k = torch.from_numpy(W.config3_keys(20_000, key_bits, seed=3).view(td)).cuda()
+        ctx.sort_pairs(k, None)
+        assert ctx.device_status_code() == 4  # GTC_ERR_TIMEOUT
+    finally:
+        ctx.set_spin_limit(0)
+        ctx.set_sort_digit_bits(key_bits, -1)
+        ctx.set_sort_variant(key_bits, -1)
+    check(W.config3_keys(20_000, key_bits, seed=3), 0, key_bits)
+    assert ctx.device_status() == 0
