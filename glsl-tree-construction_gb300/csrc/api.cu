@@ -226,7 +226,6 @@ size_t pipeline_ws_bytes(uint32_t n) {
   b += align_up((size_t)n * 4, 256);                  // vals_alt
   b += sort_workspace_bytes(n, passes, 0);
   b += 2 * scan_workspace_bytes(n);                   // unique, node offsets
-  b += 256;                                           // long-range split and run counts
   return b;
 }
 
@@ -388,13 +387,11 @@ gtc_status pipeline(gtc_ctx* ctx, const float* pts, uint32_t n, float mn, float 
   w += scan_workspace_bytes(n);
   void* offsets_ws = w;
   w += scan_workspace_bytes(n);
-  uint32_t* q_count = reinterpret_cast<uint32_t*>(w);  // [0] long-range splits
-  w += 256;
   K* keys = reinterpret_cast<K*>(o->keys);
   const SortWorkspace Wk = carve_sort_workspace(sort_ws, n, passes, 0);
-  // The Morton pass zeroes the sort's look-back descriptors and, in the same
-  // sweep, the unique / node-offset / queue workspaces behind them, so no
-  // memset node sits between the kernels of the build.
+  // The Morton pass zeroes the counts, the sort's look-back descriptors and, in
+  // the same sweep, the unique / node-offset workspaces behind them, so the
+  // sort header's memset is the build's only one.
   SortWorkspace Wz = Wk;
   Wz.desc_words = (size_t)(reinterpret_cast<uint32_t*>(w) - Wk.desc);
   // Every kernel after the first starts under a programmatic dependent
@@ -403,9 +400,6 @@ gtc_status pipeline(gtc_ctx* ctx, const float* pts, uint32_t n, float mn, float 
   Lp.pdl = !ctx->profiling;
   Lp.ws_zeroed = true;
 
-
-
-  GTC_TRY(ctx, cudaMemsetAsync(o->counts, 0, 16, S(stream)));
   GTC_TRY(ctx, cudaMemsetAsync(Wk.header, 0, Wk.header_words * 4, S(stream)));
   // The codes start in whichever pair of buffers makes the last sort pass
   // write the workspace pair (keys_alt, vals_alt): unique then compacts out
@@ -419,7 +413,8 @@ gtc_status pipeline(gtc_ctx* ctx, const float* pts, uint32_t n, float mn, float 
   {
     StageTimer t(ctx, stream, GTC_STAGE_MORTON);
     // No payload written here: the first sort pass makes the iota itself.
-    GTC_TRY(ctx, launch_morton_hist<K>(L, reinterpret_cast<const float4*>(pts), k0, n, mn, rg, Wz, BEGIN, passes));
+    GTC_TRY(ctx, launch_morton_hist<K>(L, reinterpret_cast<const float4*>(pts), k0, n, mn, rg, Wz, BEGIN, passes,
+                                         o->counts));
   }
   {
     bool in_second = false;  // true for odd pass counts: then k1 holds the result, else k0
@@ -441,12 +436,9 @@ gtc_status pipeline(gtc_ctx* ctx, const float* pts, uint32_t n, float mn, float 
     GTC_TRY(ctx, launch_unique<K>(Lp, keys_alt, vals_alt, keys, o->idx, n, o->counts + 0, unique_ws));
   }
   {
-    // vals_alt is free once unique has compacted: it holds the queue of
-    // long-range splits.
     StageTimer t(ctx, stream, GTC_STAGE_RADIX_TREE);
     GTC_TRY(ctx, launch_radix_tree<K>(Lp, keys, o->counts + 0, 0, n, o->prefix_n, o->has_leaf_left,
-                                      o->has_leaf_right, o->left_child, o->parent, o->edge_count, o->counts + 1,
-                                      vals_alt, q_count));
+                                      o->has_leaf_right, o->left_child, o->parent, o->edge_count, o->counts + 1));
   }
   {
     StageTimer t(ctx, stream, GTC_STAGE_PREFIX_SUM);

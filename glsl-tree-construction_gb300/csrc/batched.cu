@@ -809,20 +809,14 @@ gtc_status build_octree_batched_variant(gtc_ctx* ctx, const float* pts, const ui
   {
     Stage t(ctx, stream, GTC_STAGE_RADIX_TREE);
     if (tree_get_method() == 1) {
-      // idx_alt is free after unique: the queue of long-range splits.
-      uint32_t* q_count = W.counters + 16;  // zeroed with the counters
       auto window = [&](auto shape) {
         using SH = decltype(shape);
         radix_tree_window_kernel<uint32_t, true, SH><<<ceil_div(n_total, SH::T), TW_THREADS, 0, s>>>(
             out->keys, nullptr, 0, out->key_offset, S, out->prefix_n, out->has_leaf_left, out->has_leaf_right,
-            out->left_child, out->parent, out->edge_count, nullptr, W.idx_alt, q_count);
+            out->left_child, out->parent, out->edge_count, nullptr);
       };
       if (n_total <= TW_SMALL_MAX) window(TwSmall{});
       else window(TwSegLarge{});
-      BCHK(cudaGetLastError());
-      radix_tree_slow_kernel<uint32_t, true><<<L.num_sms * 2, 256, 0, s>>>(
-          out->keys, nullptr, 0, out->key_offset, S, out->prefix_n, out->has_leaf_left, out->has_leaf_right,
-          out->left_child, out->parent, out->edge_count, W.idx_alt, q_count);
     } else {
       const uint32_t grid = max(1u, min(ceil_div(n_total, 256), (uint32_t)L.num_sms * 8));
       bt_tree_kernel<<<grid, 256, 0, s>>>(out->keys, out->key_offset, S, out->prefix_n, out->has_leaf_left,

@@ -416,7 +416,7 @@ struct Launch {
   // griddep_wait() before its first global memory access, so only the launch
   // and block start-up overlap.
   bool pdl = false;
-  // The unique / scan / tree-queue workspaces of this launch were zeroed by
+  // The unique / scan workspaces of this launch were zeroed by
   // an earlier kernel of the stream: no memset node in front of them.
   bool ws_zeroed = false;
 };
@@ -494,10 +494,10 @@ cudaError_t launch_morton64(const Launch& L, const float4* pts, uint64_t* keys, 
 constexpr int RUN_FIXUP_BITS = 23;  // 5 full 8-bit passes over bits 23..62
 // Fused Morton encode + global histogram for a following sort of bits
 // [begin_bit, 3B) of the code (begin_bit 0 or RUN_FIXUP_BITS; passes must be
-// ceil((3B - begin_bit) / 8)); zeroes W.desc[0, W.desc_words).
+// ceil((3B - begin_bit) / 8)); zeroes W.desc[0, W.desc_words) and zero4[0..3].
 template <class K>
 cudaError_t launch_morton_hist(const Launch& L, const float4* pts, K* keys, uint32_t n, float mn, float rg,
-                               const SortWorkspace& W, int begin_bit, int passes);
+                               const SortWorkspace& W, int begin_bit, int passes, uint32_t* zero4);
 // Completes a stable LSD sort over bits [low_bits, 64) into a sort of the
 // whole key: every run of keys that agree above low_bits is sorted stably by
 // its low bits (1 <= low_bits <= 32), in place; the scratch arrays hold n
@@ -565,9 +565,7 @@ cudaError_t launch_node_offsets(const Launch& L, const uint32_t* edge, uint32_t*
 template <class K>
 cudaError_t launch_radix_tree(const Launch& L, const K* codes, const uint32_t* d_u, int32_t m_host, uint32_t n_max,
                               uint8_t* prefix_n, uint8_t* hll, uint8_t* hlr, int32_t* left, int32_t* parent,
-                              uint32_t* edge, uint32_t* d_m /* nullable: receives m */,
-                              uint32_t* queue = nullptr /* n_max words: long-range splits go to a warp pass */,
-                              uint32_t* q_count = nullptr /* one word, zeroed here */);
+                              uint32_t* edge, uint32_t* d_m /* nullable: receives m */);
 // Radix tree method: 1 split-indexed window kernel (default), 0 per-node Karras.
 int tree_get_method();
 bool tree_set_method(int m);

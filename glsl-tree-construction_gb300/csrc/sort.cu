@@ -176,8 +176,9 @@ template <class K, int THREADS, int Q, int LB>
 __global__ void __launch_bounds__(THREADS, 3) morton_hist_kernel(const float4* __restrict__ pts, K* __restrict__ keys,
                                                               uint32_t n, float mn, float rg, float inv_rg,
                                                               uint32_t* counts, uint32_t* bin_offsets, uint32_t* done,
-                                                              uint32_t* zero_ptr, size_t zero_words) {
+                                                              uint32_t* zero_ptr, size_t zero_words, uint32_t* zero4) {
   griddep_wait();
+  if (blockIdx.x == 0 && threadIdx.x < 4) zero4[threadIdx.x] = 0;
   constexpr int P = (3 * KeyTraits<K>::B - LB + 7) / 8;
   __shared__ uint32_t s_hist[P][RADIX];
   __shared__ uint32_t s_last;
@@ -1220,7 +1221,7 @@ template cudaError_t launch_global_hist<uint64_t>(const Launch&, const uint64_t*
 
 template <class K>
 cudaError_t launch_morton_hist(const Launch& L, const float4* pts, K* keys, uint32_t n, float mn, float rg,
-                               const SortWorkspace& W, int begin_bit, int passes) {
+                               const SortWorkspace& W, int begin_bit, int passes, uint32_t* zero4) {
   constexpr int T = 512;
   constexpr int BITS = 3 * KeyTraits<K>::B;
   if ((begin_bit != 0 && begin_bit != RUN_FIXUP_BITS) || passes != (BITS - begin_bit + 7) / 8)
@@ -1239,12 +1240,12 @@ cudaError_t launch_morton_hist(const Launch& L, const float4* pts, K* keys, uint
   }
   const uint32_t grid = max(1u, min(hist_blocks(L, n, T, 8), (uint32_t)(L.num_sms * occ)));
   return launch_kernel(L, kern, grid, T, 0, pts, keys, n, mn, rg, inv, W.counts, W.bin_offsets, W.header, W.desc,
-                       W.desc_words);
+                       W.desc_words, zero4);
 }
 template cudaError_t launch_morton_hist<uint32_t>(const Launch&, const float4*, uint32_t*, uint32_t, float, float,
-                                                  const SortWorkspace&, int, int);
+                                                  const SortWorkspace&, int, int, uint32_t*);
 template cudaError_t launch_morton_hist<uint64_t>(const Launch&, const float4*, uint64_t*, uint32_t, float, float,
-                                                  const SortWorkspace&, int, int);
+                                                  const SortWorkspace&, int, int, uint32_t*);
 
 template <class K>
 cudaError_t launch_onesweep_passes(const Launch& L, K* keys, uint32_t* vals, K* keys_alt, uint32_t* vals_alt,

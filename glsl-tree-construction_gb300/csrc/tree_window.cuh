@@ -27,9 +27,10 @@
 //   3. a split whose range reaches past the halo (0.04% of the splits of the
 //      10M clustered cloud) is kept in a block-local queue and resolved at
 //      the end of the block by a warp that searches the codes cooperatively,
-//      both range ends together, 32 probes per end per round; splits beyond
-//      the local queue's capacity go to radix_tree_slow_kernel, which does
-//      the same.
+//      both range ends together, 32 probes per end per round.  Such a split is
+//      an ancestor of the key just before or just after the window, and a
+//      root path has fewer than 64 splits (prefix lengths grow along it), so
+//      a block has fewer than 128 of them: the queue always holds them all.
 #pragma once
 
 #include "gtc_internal.cuh"
@@ -40,7 +41,7 @@ constexpr int TW_THREADS = 512;
 constexpr int TW_C = 16;                   // splits per chunk (one lane's in-chunk pass)
 constexpr int TW_TV = 64;                  // prefix lengths are < 64
 constexpr int TW_MAXB = 512;               // cloud starts cached per window (batched)
-constexpr int TW_LQ = 128;                 // long-range splits a block resolves itself
+constexpr int TW_LQ = 128;                 // long-range splits of a block (at most 2 x 63)
 
 // Window shape: T splits per block and a halo of H on each side.  Below about
 // half a million splits the kernel is one dependent chain per block (window,
@@ -282,10 +283,10 @@ __device__ __forceinline__ int tw_prev_tab(const TwSmem<SH>& s, int c, uint32_t 
   return cc * TW_C + tw_last_below(s.d + cc * TW_C, t);
 }
 
-// Global fallbacks.  Largest y in [x + 1, last] with δ(code_x, code_y) >= t,
+// Searches past the window.  Largest y in [x + 1, last] with δ(code_x, code_y) >= t,
 // and smallest y in [first, x] with δ(code_{x+1}, code_y) >= t (δ of a key
 // with keys further away never increases, so both are monotone searches).
-// Single-thread forms (stage API, no queue) and a warp-cooperative form.
+// A warp-cooperative form, and single-thread ones.
 
 // Both range ends of split x (prefix length t) in the cloud [first, last]
 // by the whole warp: the largest hi in [x + 1, last] with δ(code_x, code_hi)
@@ -400,16 +401,12 @@ __device__ __forceinline__ void tw_warp_split(const K* codes, uint32_t x, uint32
 
 // One block: splits [blockIdx.x * T, + T).  SEG: clouds of codes start at
 // uoff[0..S] (uoff[S] = U), indices written are cloud-local, and the last
-// slot of every cloud gets edge 0.  Otherwise one cloud of U codes.  With a
-// queue (capacity: one entry per split), splits whose range reaches past
-// the halo are appended to it for radix_tree_slow_kernel; without one they
-// are searched here by their own thread.
+// slot of every cloud gets edge 0.  Otherwise one cloud of U codes.
 template <class K, bool SEG, class SH>
 __global__ void __launch_bounds__(TW_THREADS, 4) radix_tree_window_kernel(
     const K* __restrict__ codes, const uint32_t* d_u, uint32_t u_host, const uint32_t* uoff, uint32_t S,
     uint8_t* __restrict__ prefix_n, uint8_t* __restrict__ hll, uint8_t* __restrict__ hlr,
-    int32_t* __restrict__ left, int32_t* __restrict__ parent, uint32_t* __restrict__ edge, uint32_t* d_m,
-    uint32_t* queue, uint32_t* q_count) {
+    int32_t* __restrict__ left, int32_t* __restrict__ parent, uint32_t* __restrict__ edge, uint32_t* d_m) {
   griddep_wait();
   constexpr int A = KeyTraits<K>::A;
   __shared__ TwSmem<SH> s;
@@ -518,16 +515,13 @@ __global__ void __launch_bounds__(TW_THREADS, 4) radix_tree_window_kernel(
     }
     const int r = (lr & 15) ? cstart + (int)(lr & 15) : tw_next_tab(s, chunk, t);
     const int l = (lr >> 4) != 15 ? cstart + (int)(lr >> 4) : tw_prev_tab(s, chunk, t);
-    if (r < 0 || l < 0) {  // the range reaches past the window: step 5, or the queue
+    if (r < 0 || l < 0) {  // the range reaches past the window: step 5
       const uint32_t k = atomicAdd(&s.lq_n, 1u);
       if (k < (uint32_t)TW_LQ) {
         s.lq[k] = x;
         continue;
       }
-      if (queue) {
-        queue[atomicAdd(q_count, 1u)] = x;
-        continue;
-      }
+      // Not reached with sorted distinct codes (TW_LQ); searched here otherwise.
     }
     uint32_t hi, dR;
     if (r >= 0) {
@@ -554,31 +548,6 @@ __global__ void __launch_bounds__(TW_THREADS, 4) radix_tree_window_kernel(
   const uint32_t nl = min(s.lq_n, (uint32_t)TW_LQ);
   for (uint32_t q = warp; q < nl; q += TW_THREADS / 32) {  // warp-uniform
     const uint32_t x = s.lq[q];
-    uint32_t U0 = 0, U1 = U;
-    if (SEG) {
-      const uint32_t c = owner(uoff, S, x);
-      U0 = uoff[c];
-      U1 = uoff[c + 1];
-    }
-    tw_warp_split<K>(codes, x, U0, U1, prefix_n, hll, hlr, left, parent, edge);
-  }
-}
-
-// The queued splits, one warp each: both range ends by warp-cooperative
-// search over the codes (the answers the window would give, for ranges of
-// any length).
-template <class K, bool SEG>
-__global__ void __launch_bounds__(256) radix_tree_slow_kernel(const K* __restrict__ codes, const uint32_t* d_u,
-                                                              uint32_t u_host, const uint32_t* uoff, uint32_t S,
-                                                              uint8_t* prefix_n, uint8_t* hll, uint8_t* hlr,
-                                                              int32_t* left, int32_t* parent, uint32_t* edge,
-                                                              const uint32_t* queue, const uint32_t* q_count) {
-  griddep_wait();
-  const uint32_t U = SEG ? uoff[S] : (d_u ? *d_u : u_host);
-  const uint32_t nq = *q_count;
-  const uint32_t warps = gridDim.x * (blockDim.x / 32);
-  for (uint32_t q = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5); q < nq; q += warps) {
-    const uint32_t x = queue[q];
     uint32_t U0 = 0, U1 = U;
     if (SEG) {
       const uint32_t c = owner(uoff, S, x);

@@ -180,3 +180,32 @@ def test_one_wave_sort(ctx, key_bits, variant):
         ctx.set_sort_variant(key_bits, -1)
     check(W.config3_keys(20_000, key_bits, seed=3), 0, key_bits)
     assert ctx.device_status() == 0
+
+
+@pytest.mark.parametrize("key_bits", [32, 64])
+@pytest.mark.parametrize("side", ["right", "left", "both"])
+def test_tree_nested_long_ranges(ctx, gtc_mod, key_bits, side):
+    """Codes whose root paths nest one long range per bit: 700 codes hang off
+    every level of a path to the first code, the last one, or a middle one, so
+    the blocks at its end hold as many splits reaching past their window as
+    there can be."""
+    import torch
+
+    kd = np.uint32 if key_bits == 32 else np.uint64
+    bits = 30 if key_bits == 32 else 63
+    g = np.random.Generator(np.random.PCG64(5))
+    path = {"right": (1 << bits) - 1, "left": 0, "both": 0x2AAAAAAAAAAAAAAA & ((1 << bits) - 1)}[side]
+    parts = [np.array([path], np.uint64)]
+    for b in range(bits - 1, 9, -1):  # the subtree beside the path at bit b
+        base = ((path >> b) ^ 1) << b
+        parts.append(np.uint64(base) + g.choice(1 << min(b, 20), min(700, 1 << b), replace=False).astype(np.uint64))
+    codes = np.unique(np.concatenate(parts)).astype(kd)
+    d = torch.from_numpy(codes.view(np.int32 if key_bits == 32 else np.int64)).cuda()
+    got = ctx.radix_tree(d, codes.size - 1, with_edge=True)
+    try:
+        gtc_mod.lib().gtc_tree_set_method(0)
+        want = ctx.radix_tree(d, codes.size - 1, with_edge=True)
+    finally:
+        gtc_mod.lib().gtc_tree_set_method(1)
+    for f in want:
+        assert torch.equal(got[f], want[f]), f
