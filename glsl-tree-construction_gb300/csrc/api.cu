@@ -501,6 +501,8 @@ cudaEvent_t context_stage_begin(gtc_ctx* ctx, gtc_stream_t stream) {
   cudaEventRecord(a, S(stream));
   return a;
 }
+// No stage events between launches.
+bool context_stage_idle(const gtc_ctx* ctx) { return !ctx->profiling; }
 void context_stage_end(gtc_ctx* ctx, gtc_stream_t stream, cudaEvent_t a, int stage) {
   if (!a) return;
   cudaEvent_t b = get_event(ctx);

@@ -39,6 +39,7 @@ namespace gtc {
 Launch context_launch(gtc_ctx* ctx, gtc_stream_t stream);
 gtc_status context_error(gtc_ctx* ctx, gtc_status s, const char* msg, cudaError_t e);
 cudaEvent_t context_stage_begin(gtc_ctx* ctx, gtc_stream_t stream);
+bool context_stage_idle(const gtc_ctx* ctx);
 void context_stage_end(gtc_ctx* ctx, gtc_stream_t stream, cudaEvent_t a, int stage);
 
 namespace {
@@ -64,22 +65,44 @@ constexpr int BM_THREADS = 512;  // Morton kernel: one block per tile
 struct BtVariant {
   int threads, kpt;
 };
-constexpr BtVariant kBtVariants[] = {{512, 12}, {256, 16}, {384, 16}, {512, 8}, {256, 24}};
+constexpr BtVariant kBtVariants[] = {{512, 12}, {256, 16}, {384, 16}, {512, 8}, {256, 24}, {256, 8}, {256, 16}};
 constexpr int kBtNumVariants = sizeof(kBtVariants) / sizeof(kBtVariants[0]);
-constexpr uint32_t BT_MIN_TILE = 4096;  // smallest tile of any variant: sizes the workspace
-constexpr int BU_THREADS = 512;
-constexpr int BU_IPT = 9;
-constexpr int BU_TILE = BU_THREADS * BU_IPT;  // the scan tile of scan.cu
+// Variant 6 is 256 x 16 held to 64 registers (four blocks per SM), as sort.cu's
+// variant 7; variant 5 has short tiles for small batches, where a pass is one
+// chain of dependent steps, and is limited to BT_SMALL_MAX points, which bounds
+// the workspace's descriptors.  Whole builds (us):
+//   points, clouds         512 x 12   256 x 8   256 x 16 at 4 blocks per SM
+//   300,125, 64                95.6      79.4      94.4
+//   422,794, 200               99.7      92.4     107.7
+//   1,562,588, 20             153.6        -      179.3
+//   3,211,561, 200            288.6        -      279.7
+//   74,044,652, 512          4386.9        -     4274.9
+constexpr int BT_SMALL = 5, BT_LARGE = 6;
+constexpr uint32_t BT_SMALL_MAX = 600000;
+constexpr uint32_t BT_LARGE_MIN = 2000000;  // untuned batches from here on take variant 6
+// Smallest tile of any variant for n points: sizes the workspace.
+constexpr uint32_t bt_min_tile(uint32_t n) { return n <= BT_SMALL_MAX ? 2048 : 4096; }
 constexpr uint32_t MAX_CLOUDS = 1u << 20;
 
 // Tiles per cloud and non-empty clouds, both scanned (one block).  The
 // offsets must partition [0, n): off[0] = 0, non-decreasing, off[S] = n.
 // Otherwise the batch is flagged bad, every later kernel returns at once and
-// the outputs say zero unique codes and zero nodes.
+// the outputs say zero unique codes and zero nodes.  Blocks past the first
+// clear the words that must start at zero (the clouds' digit histograms and
+// the scans' descriptors), in place of a memset each; the first clears the
+// counters, the bad flag among them.
 __global__ void __launch_bounds__(1024) bt_tiles_kernel(const uint32_t* off, uint32_t S, uint32_t n, uint32_t tile,
-                                                        uint32_t* tile_start, uint32_t* ne_start, uint32_t* bad,
-                                                        uint32_t* uoff, uint32_t* status) {
+                                                        uint32_t* tile_start, uint32_t* ne_start, uint32_t* counters,
+                                                        uint32_t* bad, uint32_t* uoff, uint4* zero, size_t zero_vecs,
+                                                        uint32_t* status) {
+  griddep_wait();
+  if (blockIdx.x > 0) {
+    for (size_t i = (size_t)(blockIdx.x - 1) * 1024 + threadIdx.x; i < zero_vecs; i += (size_t)(gridDim.x - 1) * 1024)
+      zero[i] = make_uint4(0, 0, 0, 0);
+    return;
+  }
   __shared__ uint32_t s_t[1024], s_n[1024];
+  if (threadIdx.x < 64) counters[threadIdx.x] = 0;
   const uint32_t per = (S + 1023) / 1024;
   const uint32_t first = threadIdx.x * per, last = min(first + per, S);
   bool ok = threadIdx.x != 0 || (off[0] == 0 && off[S] == n);
@@ -129,50 +152,87 @@ struct TileRange {
   uint32_t cloud, local, base, valid;
 };
 
-__device__ __forceinline__ TileRange tile_range(uint32_t t, const uint32_t* tile_start, const uint32_t* off,
-                                                uint32_t S, uint32_t tile) {
+// Tile t of the batch, its cloud given.
+__device__ __forceinline__ TileRange tile_range(uint32_t t, uint32_t cloud, const uint32_t* tile_start,
+                                                const uint32_t* off, uint32_t tile) {
   TileRange r;
-  r.cloud = owner(tile_start, S, t);
+  r.cloud = cloud;
   r.local = t - tile_start[r.cloud];
   r.base = off[r.cloud] + r.local * tile;
   r.valid = min(tile, off[r.cloud + 1] - r.base);
   return r;
 }
 
-// Morton codes (10 bits per axis), cloud-local payload, per-cloud digit
-// histograms; also clears the look-back descriptors of all passes.
+// Morton codes (10 bits per axis) and per-cloud digit histograms; also clears
+// the look-back descriptors of all passes and records every tile's cloud for
+// the sort.  (No payload is written: the first sort pass makes it.)  A block
+// takes `group` consecutive tiles and adds its histogram to the cloud's only
+// when the cloud changes: the 1,024 global atomics of a flush cost as much as
+// the tile's points.
+template <int Q>
 __global__ void __launch_bounds__(BM_THREADS) bt_morton_kernel(const float4* __restrict__ pts, const uint32_t* off,
                                                                uint32_t S, const uint32_t* tile_start, uint32_t tile,
-                                                               float mn,
-                                                               float rg, float inv_rg, uint32_t* __restrict__ keys,
-                                                               uint32_t* __restrict__ idx, uint32_t* seg_hist,
-                                                               uint32_t* desc, size_t desc_words) {
+                                                               uint32_t group, float mn, float rg, float inv_rg,
+                                                               uint32_t* __restrict__ keys, uint32_t* tile_cloud,
+                                                               uint32_t* seg_hist, uint4* desc, size_t desc_vecs) {
+  griddep_wait();
   __shared__ uint32_t s_hist[BPASSES * BRADIX];
-  for (int i = threadIdx.x; i < BPASSES * BRADIX; i += BM_THREADS) s_hist[i] = 0;
+  __shared__ uint32_t s_cloud;
+  const int tid = threadIdx.x;
+  for (int i = tid; i < BPASSES * BRADIX; i += BM_THREADS) s_hist[i] = 0;
   const size_t stride = (size_t)gridDim.x * BM_THREADS;
-  for (size_t i = (size_t)blockIdx.x * BM_THREADS + threadIdx.x; i < desc_words; i += stride) desc[i] = 0;
+  for (size_t i = (size_t)blockIdx.x * BM_THREADS + tid; i < desc_vecs; i += stride) desc[i] = make_uint4(0, 0, 0, 0);
+  const uint32_t tiles = tile_start[S];
+  const uint32_t t0 = blockIdx.x * group;
+  if (t0 >= tiles) return;
+  if (tid < 32) {
+    const uint32_t c = warp_upper_bound_u32(tile_start, S + 1, t0) - 1;
+    if (tid == 0) s_cloud = c;
+  }
   __syncthreads();
-  if (blockIdx.x >= tile_start[S]) return;
-  const TileRange r = tile_range(blockIdx.x, tile_start, off, S, tile);
-  const uint32_t first = off[r.cloud];
-  for (uint32_t i = threadIdx.x; i < r.valid; i += BM_THREADS) {
-    const uint32_t g = r.base + i;
-    const uint32_t k = encode_point<uint32_t>(__ldcs(pts + g), mn, rg, inv_rg);
-    keys[g] = k;
-    idx[g] = g - first;
+  uint32_t cloud = s_cloud;
+  auto flush = [&] {
+    __syncthreads();
+    uint32_t* h = seg_hist + (size_t)cloud * BPASSES * BRADIX;
+    for (int i = tid; i < BPASSES * BRADIX; i += BM_THREADS) {
+      const uint32_t c = s_hist[i];
+      if (c) atomicAdd(h + i, c);
+      s_hist[i] = 0;
+    }
+    __syncthreads();
+  };
+  for (uint32_t t = t0; t < min(t0 + group, tiles); ++t) {  // block-uniform
+    if (t >= tile_start[cloud + 1]) {
+      flush();
+      while (t >= tile_start[cloud + 1]) ++cloud;  // skips empty clouds
+    }
+    if (tid == 0) tile_cloud[t] = cloud;
+    const TileRange r = tile_range(t, cloud, tile_start, off, tile);
+    for (uint32_t i0 = tid; i0 < r.valid; i0 += 4 * BM_THREADS) {  // four points in flight
+      float4 p[4];
 #pragma unroll
-    for (int p = 0; p < BPASSES; ++p) atomicAdd(&s_hist[p * BRADIX + ((k >> (8 * p)) & 255u)], 1u);
+      for (int q = 0; q < 4; ++q) {
+        const uint32_t i = i0 + q * BM_THREADS;
+        p[q] = i < r.valid ? __ldcs(pts + r.base + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const uint32_t i = i0 + q * BM_THREADS;
+        if (i < r.valid) {
+          const uint32_t k = encode_point<uint32_t, Q>(p[q], mn, rg, inv_rg);
+          keys[r.base + i] = k;
+#pragma unroll
+          for (int d = 0; d < BPASSES; ++d) atomicAdd(&s_hist[d * BRADIX + ((k >> (8 * d)) & 255u)], 1u);
+        }
+      }
+    }
   }
-  __syncthreads();
-  uint32_t* h = seg_hist + (size_t)r.cloud * BPASSES * BRADIX;
-  for (int i = threadIdx.x; i < BPASSES * BRADIX; i += BM_THREADS) {
-    const uint32_t c = s_hist[i];
-    if (c) atomicAdd(h + i, c);
-  }
+  flush();
 }
 
 // Per cloud and pass: digit counts -> global digit bases, in place.
 __global__ void __launch_bounds__(BRADIX) bt_seg_scan_kernel(uint32_t* seg_hist, const uint32_t* off) {
+  griddep_wait();
   __shared__ uint32_t s_w[BRADIX / 32];
   const uint32_t c = blockIdx.x;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -205,15 +265,18 @@ struct BtSmem {
 // confined to one cloud and digit bases from that cloud's histogram.  A
 // cloud's last tile is padded with all-ones keys, which rank last in the tile
 // and are never stored.  Its descriptor counts them, but no tile reads it:
-// the next tile starts another cloud and does not look back.
-template <int THREADS, int KPT>
-__global__ void __launch_bounds__(THREADS) bt_onesweep_kernel(const uint32_t* __restrict__ kin,
+// the next tile starts another cloud and does not look back.  FIRST: the
+// payload is the point's index in its cloud, made here.
+template <int THREADS, int KPT, int MINB, bool FIRST>
+__global__ void __launch_bounds__(THREADS, MINB) bt_onesweep_kernel(const uint32_t* __restrict__ kin,
                                                                  const uint32_t* __restrict__ vin,
                                                                  uint32_t* __restrict__ kout,
                                                                  uint32_t* __restrict__ vout, const uint32_t* off,
-                                                                 uint32_t S, const uint32_t* tile_start, int shift,
+                                                                 uint32_t S, const uint32_t* tile_start,
+                                                                 const uint32_t* tile_cloud, int shift,
                                                                  const uint32_t* seg_base, int pass, uint32_t* desc,
                                                                  uint32_t* tile_counter, uint32_t* status) {
+  griddep_wait();
   using Sm = BtSmem<THREADS, KPT>;
   constexpr int WARPS = Sm::WARPS;
   static_assert(THREADS >= BRADIX, "one thread per digit");
@@ -226,7 +289,7 @@ __global__ void __launch_bounds__(THREADS) bt_onesweep_kernel(const uint32_t* __
   __syncthreads();
   const uint32_t tile = s.tile_id;
   if (tile >= tile_start[S]) return;
-  const TileRange r = tile_range(tile, tile_start, off, S, Sm::TILE);
+  const TileRange r = tile_range(tile, tile_cloud[tile], tile_start, off, Sm::TILE);
 
   uint32_t key[KPT], val[KPT];
   const uint32_t wbase = warp * 32 * KPT + lane;
@@ -234,7 +297,8 @@ __global__ void __launch_bounds__(THREADS) bt_onesweep_kernel(const uint32_t* __
   for (int j = 0; j < KPT; ++j) {
     const uint32_t i = wbase + j * 32;
     key[j] = (i < r.valid) ? kin[r.base + i] : 0xffffffffu;
-    val[j] = (i < r.valid) ? vin[r.base + i] : 0u;
+    if (FIRST) val[j] = r.local * Sm::TILE + i;
+    else val[j] = (i < r.valid) ? vin[r.base + i] : 0u;
   }
   uint32_t* my_hist = s.warp_hist[warp];
 #pragma unroll
@@ -301,107 +365,103 @@ __global__ void __launch_bounds__(THREADS) bt_onesweep_kernel(const uint32_t* __
 }
 
 // Unique with a restart at every cloud start (a cloud's first code is always
-// kept); the thread holding a cloud's first code records U_c.  The same
-// single-pass look-back compaction as scan.cu's unique.
-struct BuSmem {
-  uint32_t keys[BU_TILE];
-  uint32_t vals[BU_TILE];
-  uint32_t ws[BU_THREADS / 32 + 1];
-  uint32_t tile_id, prefix, halo;
+// kept): scan.cu's two resident forms, out of place, on rows of 32 codes per
+// warp.  A warp steps through the clouds that start in its rows, in order, so
+// a row's cloud starts come as a bit mask, and every cloud's U_c is recorded
+// where it starts - an empty cloud's too, which starts where the next one
+// does.  BtStarts is that position: the next cloud to start and its offset.
+struct BtStarts {
+  uint32_t cloud, at;
 };
-
-__global__ void __launch_bounds__(BU_THREADS) bt_unique_kernel(const uint32_t* kin, const uint32_t* vin,
-                                                               uint32_t* kout, uint32_t* vout, uint32_t n,
-                                                               const uint32_t* off, uint32_t S, uint32_t* uoff,
-                                                               uint32_t* ws, const uint32_t* bad, uint32_t* status) {
-  __shared__ BuSmem s;
-  if (*bad) return;
-  uint32_t* desc = ws + 64;
-  const int tid = threadIdx.x;
-  if (tid == 0) s.tile_id = atomicAdd(ws, 1u);
-  __syncthreads();
-  const uint32_t tile = s.tile_id;
-  const uint32_t base = tile * BU_TILE;
-  if (base >= n) return;
-  const uint32_t valid = min((uint32_t)BU_TILE, n - base);
-  for (uint32_t i = tid; i < valid; i += BU_THREADS) {
-    s.keys[i] = kin[base + i];
-    s.vals[i] = vin[base + i];
-  }
-  if (tid == 0) s.halo = base > 0 ? kin[base - 1] : 0u;
-  __syncthreads();
-  const uint32_t first = tid * BU_IPT;
-  const uint32_t c0 = first < valid ? owner(off, S, base + first) : 0u;
-  uint32_t c = c0;
-  uint32_t key[BU_IPT], val[BU_IPT], keep_mask = 0, start_mask = 0, cnt = 0;
-#pragma unroll
-  for (int j = 0; j < BU_IPT; ++j) {
-    const uint32_t i = first + j;
-    if (i < valid) {
-      const uint32_t g = base + i;
-      while (g >= off[c + 1]) ++c;  // off[S] = n > g, so c stays below S
-      const bool start = (g == off[c]);
-      key[j] = s.keys[i];
-      val[j] = s.vals[i];
-      const uint32_t prev = (i == 0) ? s.halo : s.keys[i - 1];
-      const bool keep = start || key[j] != prev;
-      keep_mask |= (uint32_t)keep << j;
-      start_mask |= (uint32_t)start << j;
-      cnt += keep;
-    }
-  }
-  uint32_t total;
-  const uint32_t excl = block_exclusive<BU_THREADS>(cnt, s.ws, &total);
-  if (tid < 32) {
-    const uint32_t pre = tile_lookback(desc, tile, total, status);
-    if (tid == 0) s.prefix = pre;
-  }
-  __syncthreads();
-  const uint32_t out0 = s.prefix;
-  if (start_mask) {
-    c = c0;
-    uint32_t rr = excl;
-#pragma unroll
-    for (int j = 0; j < BU_IPT; ++j) {
-      const uint32_t i = first + j;
-      if (i < valid) {
-        const uint32_t g = base + i;
-        while (g >= off[c + 1]) ++c;
-        if (start_mask & (1u << j)) uoff[c] = out0 + rr;
-        rr += (keep_mask >> j) & 1u;
-      }
-    }
-  }
-  uint32_t r = excl;
-#pragma unroll
-  for (int j = 0; j < BU_IPT; ++j) {
-    if (keep_mask & (1u << j)) {
-      s.keys[r] = key[j];
-      s.vals[r] = val[j];
-      ++r;
-    }
-  }
-  __syncthreads();
-  for (uint32_t i = tid; i < total; i += BU_THREADS) {
-    kout[out0 + i] = s.keys[i];
-    vout[out0 + i] = s.vals[i];
-  }
-  if (tid == 0 && base + valid == n) uoff[S] = out0 + total;
+// The first cloud that starts at or after position r (whole warp).
+__device__ __forceinline__ BtStarts bt_starts_from(const uint32_t* off, uint32_t S, uint32_t r) {
+  const uint32_t c = r > 0 ? warp_upper_bound_u32(off, S + 1, r - 1) : 0u;
+  return BtStarts{c, c <= S ? off[c] : ~0u};
 }
-
-// The resident segment form of the same unique (scan.cu's
-// chunk_unique_kernel, out of place): rows of 32 codes per warp; a warp
-// tracks the cloud of its row (one binary search per segment, then a step
-// per cloud start), so the cloud starts of a row come as a bit mask.
-__device__ __forceinline__ uint32_t bt_row_starts(const uint32_t* off, uint32_t S, uint32_t r, uint32_t& cur) {
-  uint32_t smask = (off[cur] == r) ? 1u : 0u;
-  while (cur + 1 < S && off[cur + 1] < r + 32) {
-    ++cur;
-    smask |= 1u << (off[cur] - r);
+// The cloud starts in [r, r + 32) as a mask; steps past them.
+__device__ __forceinline__ uint32_t bt_row_starts(const uint32_t* off, uint32_t S, uint32_t r, BtStarts& st) {
+  uint32_t smask = 0;
+  while (st.cloud < S && st.at < r + 32) {  // warp-uniform
+    smask |= 1u << (st.at - r);
+    ++st.cloud;
+    st.at = off[st.cloud];
   }
   return smask;
 }
+// Records U_c of the clouds that start in [r, r + 32), and steps past them:
+// bal is the row's kept mask, run its first output position.
+__device__ __forceinline__ void bt_row_record(const uint32_t* off, uint32_t S, uint32_t r, BtStarts& st, uint32_t bal,
+                                              uint32_t run, uint32_t* uoff) {
+  while (st.cloud < S && st.at < r + 32) {
+    if ((threadIdx.x & 31) == 0) uoff[st.cloud] = run + __popc(bal & ((1u << (st.at - r)) - 1u));
+    ++st.cloud;
+    st.at = off[st.cloud];
+  }
+}
+// Past the last row: U_S and the empty clouds behind the last code (lane 0).
+__device__ __forceinline__ void bt_record_end(const uint32_t* off, uint32_t S, uint32_t run, uint32_t* uoff) {
+  uoff[S] = run;
+  for (uint32_t c = S; c > 0 && off[c - 1] == off[S]; --c) uoff[c - 1] = run;
+}
 
+template <int ROWS>
+__global__ void __launch_bounds__(CS_THREADS) bt_row_unique_kernel(const uint32_t* __restrict__ kin,
+                                                                   const uint32_t* __restrict__ vin,
+                                                                   uint32_t* __restrict__ kout,
+                                                                   uint32_t* __restrict__ vout, uint32_t n,
+                                                                   const uint32_t* off, uint32_t S, uint32_t* uoff,
+                                                                   uint32_t* ws, const uint32_t* bad,
+                                                                   uint32_t* status) {
+  griddep_wait();
+  __shared__ uint32_t s_seg[CS_WARPS];
+  __shared__ uint32_t s_red[CS_WARPS];
+  if (*bad) return;  // the same word for every block
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t lt = (1u << lane) - 1u;
+  const uint32_t r0 = (blockIdx.x * CS_WARPS + warp) * (ROWS * 32);
+  uint32_t k[ROWS], v[ROWS];
+#pragma unroll
+  for (int j = 0; j < ROWS; ++j) {
+    const uint32_t i = r0 + j * 32 + lane;
+    k[j] = i < n ? kin[i] : 0u;
+    v[j] = i < n ? vin[i] : 0u;
+  }
+  uint32_t carry = (lane == 0 && r0 > 0 && r0 < n) ? kin[r0 - 1] : 0u;
+  const BtStarts first = bt_starts_from(off, S, min(r0, n));
+  BtStarts st = first;
+  uint32_t keep = 0, cnt = 0;
+#pragma unroll
+  for (int j = 0; j < ROWS; ++j) {
+    const uint32_t r = r0 + j * 32, i = r + lane;
+    const uint32_t smask = r < n ? bt_row_starts(off, S, r, st) : 0u;
+    uint32_t prev = __shfl_up_sync(0xffffffffu, k[j], 1);
+    if (lane == 0) prev = carry;
+    const bool kp = i < n && (k[j] != prev || ((smask >> lane) & 1u));
+    keep |= (uint32_t)kp << j;
+    cnt += __popc(__ballot_sync(0xffffffffu, kp));
+    carry = __shfl_sync(0xffffffffu, k[j], 31);
+  }
+  if (lane == 0) s_seg[warp] = cnt;
+  uint32_t run = cs_block_prefix(ws + 64, s_seg, s_red, status) + s_seg[warp];
+  st = first;
+#pragma unroll
+  for (int j = 0; j < ROWS; ++j) {
+    const uint32_t r = r0 + j * 32;
+    const bool kp = (keep >> j) & 1u;
+    const uint32_t bal = __ballot_sync(0xffffffffu, kp);
+    if (kp) {
+      const uint32_t o = run + __popc(bal & lt);
+      kout[o] = k[j];
+      vout[o] = v[j];
+    }
+    if (r < n) bt_row_record(off, S, r, st, bal, run, uoff);
+    run += __popc(bal);
+  }
+  if (blockIdx.x == gridDim.x - 1 && warp == CS_WARPS - 1 && lane == 0) bt_record_end(off, S, run, uoff);
+}
+
+// Segments of any length, read twice (scan.cu's chunk_unique_kernel), eight
+// rows in flight per warp.
 __global__ void __launch_bounds__(CS_THREADS) bt_chunk_unique_kernel(const uint32_t* __restrict__ kin,
                                                                      const uint32_t* __restrict__ vin,
                                                                      uint32_t* __restrict__ kout,
@@ -409,9 +469,11 @@ __global__ void __launch_bounds__(CS_THREADS) bt_chunk_unique_kernel(const uint3
                                                                      const uint32_t* off, uint32_t S, uint32_t* uoff,
                                                                      uint32_t* ws, const uint32_t* bad,
                                                                      uint32_t* status) {
+  griddep_wait();
   __shared__ uint32_t s_seg[CS_WARPS];
   __shared__ uint32_t s_red[CS_WARPS];
   if (*bad) return;  // the same word for every block
+  constexpr int R = 8;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t lt = (1u << lane) - 1u;
   const uint32_t nseg = gridDim.x * CS_WARPS;
@@ -419,22 +481,31 @@ __global__ void __launch_bounds__(CS_THREADS) bt_chunk_unique_kernel(const uint3
   const uint64_t beg64 = (uint64_t)(blockIdx.x * CS_WARPS + warp) * SL;
   const uint32_t beg = (uint32_t)min(beg64, (uint64_t)n);
   const uint32_t end = (uint32_t)min(beg64 + SL, (uint64_t)n);
-  const uint32_t c_beg = (beg < end) ? owner(off, S, beg) : 0u;
   const uint32_t first_prev = (beg > 0 && beg < end) ? kin[beg - 1] : 0u;
+  const BtStarts first = bt_starts_from(off, S, beg);
+  const uint64_t keep_pol = l2_keep_policy(), drop_pol = l2_drop_policy();
 
-  // 1. kept codes per segment
+  // 1. kept codes per segment (codes tagged to stay in L2 for step 3)
   uint32_t cnt = 0;
   {
-    uint32_t carry = first_prev, cur = c_beg;
-    for (uint32_t r = beg; r < end; r += 32) {
-      const uint32_t i = r + lane;
-      const uint32_t key = (i < end) ? kin[i] : 0u;
-      const uint32_t smask = bt_row_starts(off, S, r, cur);
-      uint32_t prev = __shfl_up_sync(0xffffffffu, key, 1);
-      if (lane == 0) prev = carry;
-      const bool keep = i < end && (i == 0 || key != prev || ((smask >> lane) & 1u));
-      cnt += __popc(__ballot_sync(0xffffffffu, keep));
-      carry = __shfl_sync(0xffffffffu, key, 31);
+    uint32_t carry = first_prev;
+    BtStarts st = first;
+    for (uint32_t r0 = beg; r0 < end; r0 += 32 * R) {
+      uint32_t k[R];
+#pragma unroll
+      for (int j = 0; j < R; ++j) {
+        const uint32_t i = r0 + 32 * j + lane;
+        k[j] = i < end ? ld_hint(kin + i, keep_pol) : 0u;
+      }
+#pragma unroll
+      for (int j = 0; j < R; ++j) {
+        const uint32_t r = r0 + 32 * j, i = r + lane;
+        const uint32_t smask = r < end ? bt_row_starts(off, S, r, st) : 0u;
+        uint32_t prev = __shfl_up_sync(0xffffffffu, k[j], 1);
+        if (lane == 0) prev = carry;
+        cnt += __popc(__ballot_sync(0xffffffffu, i < end && (k[j] != prev || ((smask >> lane) & 1u))));
+        carry = __shfl_sync(0xffffffffu, k[j], 31);
+      }
     }
   }
   if (lane == 0) s_seg[warp] = cnt;
@@ -443,45 +514,47 @@ __global__ void __launch_bounds__(CS_THREADS) bt_chunk_unique_kernel(const uint3
   uint32_t run = cs_block_prefix(ws + 64, s_seg, s_red, status);
   run += s_seg[warp];
 
-  // 3. rescan and write; the lane holding a cloud's first code records U_c
+  // 3. rescan and write, recording every cloud's U_c
   {
-    uint32_t carry = first_prev, cur = c_beg;
-    for (uint32_t r = beg; r < end; r += 32) {
-      const uint32_t i = r + lane;
-      const uint32_t key = (i < end) ? kin[i] : 0u;
-      const uint32_t val = (i < end) ? vin[i] : 0u;
-      const uint32_t smask = bt_row_starts(off, S, r, cur);
-      uint32_t prev = __shfl_up_sync(0xffffffffu, key, 1);
-      if (lane == 0) prev = carry;
-      const bool start = i < end && ((smask >> lane) & 1u);
-      const bool keep = i < end && (i == 0 || key != prev || start);
-      const uint32_t bal = __ballot_sync(0xffffffffu, keep);
-      if (keep) {
-        const uint32_t o = run + __popc(bal & lt);
-        kout[o] = key;
-        vout[o] = val;
-        if (start) uoff[owner(off, S, i)] = o;
+    uint32_t carry = first_prev;
+    BtStarts st = first;
+    for (uint32_t r0 = beg; r0 < end; r0 += 32 * R) {
+      uint32_t k[R], v[R];
+#pragma unroll
+      for (int j = 0; j < R; ++j) {
+        const uint32_t i = r0 + 32 * j + lane;
+        k[j] = i < end ? ld_hint(kin + i, drop_pol) : 0u;
+        v[j] = i < end ? ld_hint(vin + i, drop_pol) : 0u;
       }
-      run += __popc(bal);
-      carry = __shfl_sync(0xffffffffu, key, 31);
+#pragma unroll
+      for (int j = 0; j < R; ++j) {
+        const uint32_t r = r0 + 32 * j, i = r + lane;
+        BtStarts here = st;
+        const uint32_t smask = r < end ? bt_row_starts(off, S, r, st) : 0u;
+        uint32_t prev = __shfl_up_sync(0xffffffffu, k[j], 1);
+        if (lane == 0) prev = carry;
+        const bool kp = i < end && (k[j] != prev || ((smask >> lane) & 1u));
+        const uint32_t bal = __ballot_sync(0xffffffffu, kp);
+        if (kp) {
+          const uint32_t o = run + __popc(bal & lt);
+          kout[o] = k[j];
+          vout[o] = v[j];
+        }
+        if (smask) bt_row_record(off, S, r, here, bal, run, uoff);
+        run += __popc(bal);
+        carry = __shfl_sync(0xffffffffu, k[j], 31);
+      }
     }
   }
   // The last warp of the last block ends at n: its running count is U.
-  if (blockIdx.x == gridDim.x - 1 && warp == CS_WARPS - 1 && lane == 0) uoff[S] = run;
-}
-
-// Empty clouds own no code: their U_c is the next cloud's (one thread; runs
-// from the end, so runs of empty clouds resolve).
-__global__ void bt_uoff_fix_kernel(const uint32_t* off, uint32_t S, uint32_t* uoff, const uint32_t* bad) {
-  if (blockIdx.x != 0 || threadIdx.x != 0 || *bad) return;
-  for (int c = (int)S - 1; c >= 0; --c)
-    if (off[c + 1] == off[c]) uoff[c] = uoff[c + 1];
+  if (blockIdx.x == gridDim.x - 1 && warp == CS_WARPS - 1 && lane == 0) bt_record_end(off, S, run, uoff);
 }
 
 // Radix tree of every cloud, one thread per unique code.
 __global__ void __launch_bounds__(256) bt_tree_kernel(const uint32_t* __restrict__ codes, const uint32_t* uoff,
                                                       uint32_t S, uint8_t* prefix_n, uint8_t* hll, uint8_t* hlr,
                                                       int32_t* left, int32_t* parent, uint32_t* edge) {
+  griddep_wait();
   const uint32_t U = uoff[S];
   const uint32_t stride = gridDim.x * blockDim.x;
   for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < U; g += stride) {
@@ -506,6 +579,7 @@ __global__ void __launch_bounds__(256) bt_tree_kernel(const uint32_t* __restrict
 __global__ void bt_cloud_offsets_kernel(uint32_t* uoff, const uint32_t* ne_start, const uint32_t* ps, uint32_t S,
                                         uint32_t* node_off, uint32_t* cloud_counts, uint4* cinfo,
                                         const uint32_t* bad) {
+  griddep_wait();
   const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= S) return;
   if (*bad) {
@@ -547,6 +621,7 @@ __global__ void __launch_bounds__(BT_OCT_THREADS) bt_octree_kernel(const uint32_
                                                                    float mn, float rg, gtc_octnode* nodes,
                                                                    uint32_t capacity, uint32_t lmask_keep,
                                                                    uint32_t* status) {
+  griddep_wait();
   constexpr int WARPS = BT_OCT_THREADS / 32;
   constexpr int A = KeyTraits<uint32_t>::A;
   __shared__ OctWarp s_warp[WARPS];
@@ -619,34 +694,66 @@ __global__ void __launch_bounds__(BT_OCT_THREADS) bt_octree_kernel(const uint32_
   if (qn > 0) run_batch(qn);
 }
 
-template <int THREADS, int KPT>
-cudaError_t launch_bt_pass(cudaStream_t s, uint32_t grid, const uint32_t* kin, const uint32_t* vin, uint32_t* kout,
-                           uint32_t* vout, const uint32_t* off, uint32_t S, const uint32_t* tile_start, int shift,
-                           const uint32_t* seg_base, int pass, uint32_t* desc, uint32_t* tile_counter,
-                           uint32_t* status) {
+struct BtPass {
+  const uint32_t* kin;
+  const uint32_t* vin;
+  uint32_t* kout;
+  uint32_t* vout;
+  const uint32_t* off;
+  uint32_t S;
+  const uint32_t* tile_start;
+  const uint32_t* tile_cloud;
+  int pass;
+  const uint32_t* seg_base;
+  uint32_t* desc;
+  uint32_t* tile_counter;
+};
+
+template <int THREADS, int KPT, int MINB>
+cudaError_t launch_bt_pass(const Launch& L, uint32_t grid, const BtPass& a) {
   using Sm = BtSmem<THREADS, KPT>;
-  cudaError_t e = kernel_setup(bt_onesweep_kernel<THREADS, KPT>, THREADS, sizeof(Sm));
+  auto kern = a.pass == 0 ? bt_onesweep_kernel<THREADS, KPT, MINB, true> : bt_onesweep_kernel<THREADS, KPT, MINB, false>;
+  cudaError_t e = kernel_setup(kern, THREADS, sizeof(Sm));
   if (e != cudaSuccess) return e;
-  bt_onesweep_kernel<THREADS, KPT><<<grid, THREADS, sizeof(Sm), s>>>(kin, vin, kout, vout, off, S, tile_start, shift,
-                                                                     seg_base, pass, desc, tile_counter, status);
-  return cudaGetLastError();
+  return launch_kernel(L, kern, grid, THREADS, sizeof(Sm), a.kin, a.vin, a.kout, a.vout, a.off, a.S, a.tile_start,
+                       a.tile_cloud, 8 * a.pass, a.seg_base, a.pass, a.desc, a.tile_counter, L.status);
 }
 
-cudaError_t launch_bt_variant(int v, cudaStream_t s, uint32_t grid, const uint32_t* kin, const uint32_t* vin,
-                              uint32_t* kout, uint32_t* vout, const uint32_t* off, uint32_t S,
-                              const uint32_t* tile_start, int shift, const uint32_t* seg_base, int pass,
-                              uint32_t* desc, uint32_t* tile_counter, uint32_t* status) {
-#define GTC_BT(T, K)                                                                                               \
-  return launch_bt_pass<T, K>(s, grid, kin, vin, kout, vout, off, S, tile_start, shift, seg_base, pass, desc, \
-                              tile_counter, status)
+cudaError_t launch_bt_variant(int v, const Launch& L, uint32_t grid, const BtPass& a) {
   switch (v) {
-    case 1: GTC_BT(256, 16);
-    case 2: GTC_BT(384, 16);
-    case 3: GTC_BT(512, 8);
-    case 4: GTC_BT(256, 24);
-    default: GTC_BT(512, 12);
+    case 1: return launch_bt_pass<256, 16, 3>(L, grid, a);
+    case 2: return launch_bt_pass<384, 16, 2>(L, grid, a);
+    case 3: return launch_bt_pass<512, 8, 2>(L, grid, a);
+    case 4: return launch_bt_pass<256, 24, 2>(L, grid, a);
+    case BT_SMALL: return launch_bt_pass<256, 8, 4>(L, grid, a);
+    case BT_LARGE: return launch_bt_pass<256, 16, 4>(L, grid, a);
+    default: return launch_bt_pass<512, 12, 2>(L, grid, a);
   }
-#undef GTC_BT
+}
+
+// Unique by the row kernel of the smallest ROWS whose blocks are all resident
+// at one per SM (two at the most rows; scan.cu has the reason and times), or
+// by segments read twice.
+template <int ROWS>
+cudaError_t launch_bt_unique(const Launch& L, const uint32_t* kin, const uint32_t* vin, uint32_t* kout, uint32_t* vout,
+                             uint32_t n, const uint32_t* off, uint32_t S, uint32_t* uoff, uint32_t* ws,
+                             uint32_t ws_blocks, const uint32_t* bad) {
+  int occ = 1;
+  if constexpr (ROWS <= 16) {
+    auto kern = bt_row_unique_kernel<ROWS>;
+    cudaError_t e = kernel_setup(kern, CS_THREADS, 0, &occ);
+    if (e != cudaSuccess) return e;
+    const uint32_t g = ceil_div(n, ROWS * CS_THREADS);
+    if (g > min(occ, ROWS < 16 ? 1 : 2) * (uint32_t)L.num_sms || g > ws_blocks)
+      return launch_bt_unique<ROWS * 2>(L, kin, vin, kout, vout, n, off, S, uoff, ws, ws_blocks, bad);
+    return launch_kernel(L, kern, g, CS_THREADS, 0, kin, vin, kout, vout, n, off, S, uoff, ws, bad, L.status);
+  } else {
+    cudaError_t e = kernel_setup(bt_chunk_unique_kernel, CS_THREADS, 0, &occ);
+    if (e != cudaSuccess) return e;
+    const uint32_t g = max(1u, min(min((uint32_t)(occ * L.num_sms), ws_blocks), ceil_div(n, CS_THREADS)));
+    return launch_kernel(L, bt_chunk_unique_kernel, g, CS_THREADS, 0, kin, vin, kout, vout, n, off, S, uoff, ws, bad,
+                         L.status);
+  }
 }
 
 std::atomic<int> g_bt_pinned{-1};  // gtc_batched_set_variant
@@ -654,13 +761,16 @@ std::atomic<int> g_bt_pinned{-1};  // gtc_batched_set_variant
 struct BatchWs {
   uint32_t* tile_start;  // [S + 1]
   uint32_t* ne_start;    // [S + 1]
-  uint32_t* seg_hist;    // [S][4][256]
+  uint32_t* tile_cloud;  // [tiles_max]
+  uint32_t* seg_hist;    // [S][4][256], cleared per build, as are the next two
+  void* unique_ws;
+  void* scan_ws;
+  size_t zero_vecs;      // 16-byte words from seg_hist on that are cleared
   uint32_t* counters;    // [0..3] pass tickets
   uint32_t* desc;        // [4][tiles_max][256]
   uint32_t* keys_alt;    // [n]
   uint32_t* idx_alt;     // [n]
   uint32_t* ps;          // [n]
-  void* scan_ws;
   size_t desc_words;
   uint32_t tiles_max;
 };
@@ -668,7 +778,7 @@ struct BatchWs {
 // A cloud of len points has ceil(len / TILE) tiles, so the batch has at most
 // n / TILE + S of them; sized for the smallest tile of any variant.
 size_t batch_layout(uint32_t n, uint32_t S, BatchWs* W, char* p) {
-  const uint32_t tiles_max = ceil_div(n > 0 ? n : 1, BT_MIN_TILE) + S;
+  const uint32_t tiles_max = ceil_div(n > 0 ? n : 1, bt_min_tile(n)) + S;
   size_t o = 0;
   auto take = [&](size_t bytes) {
     char* q = p ? p + o : nullptr;
@@ -678,14 +788,18 @@ size_t batch_layout(uint32_t n, uint32_t S, BatchWs* W, char* p) {
   BatchWs w;
   w.tile_start = reinterpret_cast<uint32_t*>(take(((size_t)S + 1) * 4));
   w.ne_start = reinterpret_cast<uint32_t*>(take(((size_t)S + 1) * 4));
+  w.tile_cloud = reinterpret_cast<uint32_t*>(take((size_t)tiles_max * 4));
+  const size_t zero_from = o;
   w.seg_hist = reinterpret_cast<uint32_t*>(take((size_t)S * BPASSES * BRADIX * 4));
+  w.unique_ws = take(scan_workspace_bytes(n));
+  w.scan_ws = take(scan_workspace_bytes(n));
+  w.zero_vecs = (o - zero_from) / 16;
   w.counters = reinterpret_cast<uint32_t*>(take(256));
   w.desc_words = (size_t)BPASSES * tiles_max * BRADIX;
   w.desc = reinterpret_cast<uint32_t*>(take(w.desc_words * 4));
   w.keys_alt = reinterpret_cast<uint32_t*>(take((size_t)n * 4));
   w.idx_alt = reinterpret_cast<uint32_t*>(take((size_t)n * 4));
   w.ps = reinterpret_cast<uint32_t*>(take((size_t)n * 4));
-  w.scan_ws = take(scan_workspace_bytes(n));
   w.tiles_max = tiles_max;
   if (W) *W = w;
   return o;
@@ -711,7 +825,8 @@ int batched_select_variant(uint32_t n) {
   const int pinned = g_bt_pinned.load(std::memory_order_relaxed);
   if (pinned >= 0) return pinned;
   const int t = tuned_batched_variant(n);
-  return (t >= 0 && t < kBtNumVariants) ? t : 0;
+  if (t >= 0 && t < kBtNumVariants) return t;
+  return n <= BT_SMALL_MAX ? BT_SMALL : n >= BT_LARGE_MIN ? BT_LARGE : 0;
 }
 int batched_num_variants() { return kBtNumVariants; }
 
@@ -723,6 +838,7 @@ gtc_status build_octree_batched_variant(gtc_ctx* ctx, const float* pts, const ui
   if (!ctx) return GTC_ERR_INVALID_ARG;
   if (variant < 0 || variant >= kBtNumVariants)
     return context_error(ctx, GTC_ERR_INVALID_ARG, "no such batched variant", cudaSuccess);
+  if (variant == BT_SMALL && n_total > BT_SMALL_MAX) variant = 0;
   const uint32_t tile = (uint32_t)(kBtVariants[variant].threads * kBtVariants[variant].kpt);
   if (!out || !d_offsets || n_clouds == 0 || n_clouds > MAX_CLOUDS)
     return context_error(ctx, GTC_ERR_INVALID_ARG, "need offsets, outputs and 1..2^20 clouds", cudaSuccess);
@@ -754,20 +870,23 @@ gtc_status build_octree_batched_variant(gtc_ctx* ctx, const float* pts, const ui
     return GTC_OK;
   }
   uint32_t* bad = W.counters + 8;
+  // Every kernel after the first starts under a programmatic dependent launch
+  // (not while stage events are being recorded between them).
+  Launch Lp = L;
+  Lp.pdl = context_stage_idle(ctx);
+  Lp.ws_zeroed = true;
   {
     Stage t(ctx, stream, GTC_STAGE_MORTON);
-    BCHK(cudaMemsetAsync(W.seg_hist, 0, (size_t)S * BPASSES * BRADIX * 4, s));
-    BCHK(cudaMemsetAsync(W.counters, 0, 256, s));
-    bt_tiles_kernel<<<1, 1024, 0, s>>>(d_offsets, S, n_total, tile, W.tile_start, W.ne_start, bad,
-                                       out->key_offset, L.status);
-    BCHK(cudaGetLastError());
-    bt_morton_kernel<<<W.tiles_max, BM_THREADS, 0, s>>>(reinterpret_cast<const float4*>(pts), d_offsets, S,
-                                                        W.tile_start, tile, min_coord, range, pow2_reciprocal(range),
-                                                        W.keys_alt, W.idx_alt,
-                                                        W.seg_hist, W.desc, W.desc_words);
-    BCHK(cudaGetLastError());
-    bt_seg_scan_kernel<<<S, BRADIX, 0, s>>>(W.seg_hist, d_offsets);
-    BCHK(cudaGetLastError());
+    const uint32_t zgrid = (uint32_t)min((W.zero_vecs + 2047) / 2048, (size_t)L.num_sms);
+    BCHK(launch_kernel(L, bt_tiles_kernel, 1 + zgrid, 1024, 0, d_offsets, S, n_total, tile, W.tile_start, W.ne_start,
+                       W.counters, bad, out->key_offset, reinterpret_cast<uint4*>(W.seg_hist), W.zero_vecs, L.status));
+    const float inv = pow2_reciprocal(range);
+    auto kern = inv != 0.0f ? bt_morton_kernel<1> : bt_morton_kernel<2>;
+    const uint32_t group = W.tiles_max > 16u * (uint32_t)L.num_sms ? 4u : 1u;
+    BCHK(launch_kernel(Lp, kern, ceil_div(W.tiles_max, group), BM_THREADS, 0, reinterpret_cast<const float4*>(pts),
+                       d_offsets, S, W.tile_start, tile, group, min_coord, range, inv, W.keys_alt, W.tile_cloud,
+                       W.seg_hist, reinterpret_cast<uint4*>(W.desc), W.desc_words / 4));
+    BCHK(launch_kernel(Lp, bt_seg_scan_kernel, S, BRADIX, 0, W.seg_hist, d_offsets));
   }
   uint32_t* src_k = W.keys_alt;
   uint32_t* src_v = W.idx_alt;
@@ -775,64 +894,42 @@ gtc_status build_octree_batched_variant(gtc_ctx* ctx, const float* pts, const ui
   uint32_t* dst_v = out->idx;
   for (int p = 0; p < BPASSES; ++p) {
     Stage t(ctx, stream, GTC_STAGE_ONESWEEP);
-    BCHK(launch_bt_variant(variant, s, W.tiles_max, src_k, src_v, dst_k, dst_v, d_offsets, S, W.tile_start, 8 * p,
-                           W.seg_hist, p, W.desc + (size_t)p * W.tiles_max * BRADIX, W.counters + p, L.status));
+    BCHK(launch_bt_variant(variant, Lp, W.tiles_max,
+                           BtPass{src_k, src_v, dst_k, dst_v, d_offsets, S, W.tile_start, W.tile_cloud, p, W.seg_hist,
+                                  W.desc + (size_t)p * W.tiles_max * BRADIX, W.counters + p}));
     std::swap(src_k, dst_k);
     std::swap(src_v, dst_v);
   }
   // After 4 passes the sorted pairs are back in the alternate buffers.
   {
     Stage t(ctx, stream, GTC_STAGE_UNIQUE);
-    const uint32_t utiles = ceil_div(n_total, BU_TILE);
-    uint32_t* uws = reinterpret_cast<uint32_t*>(W.scan_ws);
-    // The resident segment form once the batch fills the GPU; its
-    // descriptors fit the workspace's tile count.
-    int occ = 1;  // resident blocks per SM
-    if (kernel_setup(bt_chunk_unique_kernel, CS_THREADS, 0, &occ) != cudaSuccess) {
-      cudaGetLastError();
-      occ = 1;
-    }
-    const uint32_t g = min((uint32_t)(occ * L.num_sms), utiles);
-    if (g >= 64 && (uint64_t)n_total >= (uint64_t)g * CS_WARPS * 256) {
-      BCHK(cudaMemsetAsync(uws, 0, (64 + (size_t)g) * 4, s));
-      bt_chunk_unique_kernel<<<g, CS_THREADS, 0, s>>>(src_k, src_v, out->keys, out->idx, n_total, d_offsets, S,
-                                                      out->key_offset, uws, bad, L.status);
-    } else {
-      BCHK(cudaMemsetAsync(uws, 0, (64 + (size_t)utiles) * 4, s));
-      bt_unique_kernel<<<utiles, BU_THREADS, 0, s>>>(src_k, src_v, out->keys, out->idx, n_total, d_offsets, S,
-                                                     out->key_offset, uws, bad, L.status);
-    }
-    BCHK(cudaGetLastError());
-    bt_uoff_fix_kernel<<<1, 32, 0, s>>>(d_offsets, S, out->key_offset, bad);
-    BCHK(cudaGetLastError());
+    BCHK(launch_bt_unique<2>(Lp, src_k, src_v, out->keys, out->idx, n_total, d_offsets, S, out->key_offset,
+                             reinterpret_cast<uint32_t*>(W.unique_ws),
+                             (uint32_t)(scan_workspace_bytes(n_total) / 4) - 64, bad));
   }
   {
     Stage t(ctx, stream, GTC_STAGE_RADIX_TREE);
     if (tree_get_method() == 1) {
       auto window = [&](auto shape) {
         using SH = decltype(shape);
-        radix_tree_window_kernel<uint32_t, true, SH><<<ceil_div(n_total, SH::T), TW_THREADS, 0, s>>>(
-            out->keys, nullptr, 0, out->key_offset, S, out->prefix_n, out->has_leaf_left, out->has_leaf_right,
-            out->left_child, out->parent, out->edge_count, nullptr);
+        return launch_kernel(Lp, radix_tree_window_kernel<uint32_t, true, SH>, ceil_div(n_total, SH::T), TW_THREADS, 0,
+                             out->keys, nullptr, 0u, out->key_offset, S, out->prefix_n, out->has_leaf_left,
+                             out->has_leaf_right, out->left_child, out->parent, out->edge_count, nullptr);
       };
-      if (n_total <= TW_SMALL_MAX) window(TwSmall{});
-      else window(TwSegLarge{});
+      BCHK(n_total <= TW_SMALL_MAX ? window(TwSmall{}) : window(TwSegLarge{}));
     } else {
       const uint32_t grid = max(1u, min(ceil_div(n_total, 256), (uint32_t)L.num_sms * 8));
-      bt_tree_kernel<<<grid, 256, 0, s>>>(out->keys, out->key_offset, S, out->prefix_n, out->has_leaf_left,
-                                          out->has_leaf_right, out->left_child, out->parent, out->edge_count);
+      BCHK(launch_kernel(Lp, bt_tree_kernel, grid, 256, 0, out->keys, out->key_offset, S, out->prefix_n,
+                         out->has_leaf_left, out->has_leaf_right, out->left_child, out->parent, out->edge_count));
     }
-    BCHK(cudaGetLastError());
   }
   {
     Stage t(ctx, stream, GTC_STAGE_PREFIX_SUM);
-    BCHK(launch_inclusive_scan_dev(L, out->edge_count, W.ps, out->key_offset + S, n_total, W.scan_ws));
+    BCHK(launch_inclusive_scan_dev(Lp, out->edge_count, W.ps, out->key_offset + S, n_total, W.scan_ws));
     // The per-cloud digit histograms are dead after the sort: their space
     // holds the per-cloud octree info.
-    bt_cloud_offsets_kernel<<<ceil_div(S, 256), 256, 0, s>>>(out->key_offset, W.ne_start, W.ps, S,
-                                                            out->node_offset, out->cloud_counts,
-                                                            reinterpret_cast<uint4*>(W.seg_hist), bad);
-    BCHK(cudaGetLastError());
+    BCHK(launch_kernel(Lp, bt_cloud_offsets_kernel, ceil_div(S, 256), 256, 0, out->key_offset, W.ne_start, W.ps, S,
+                       out->node_offset, out->cloud_counts, reinterpret_cast<uint4*>(W.seg_hist), bad));
   }
   {
     Stage t(ctx, stream, GTC_STAGE_OCTREE);
@@ -842,11 +939,10 @@ gtc_status build_octree_batched_variant(gtc_ctx* ctx, const float* pts, const ui
       occ = 4;
     }
     const uint32_t ogrid = max(1u, min(ceil_div(n_total, BT_OCT_THREADS), (uint32_t)(L.num_sms * occ)));
-    bt_octree_kernel<<<ogrid, BT_OCT_THREADS, 0, s>>>(out->keys, out->key_offset, S, reinterpret_cast<const uint4*>(W.seg_hist),
-                                           out->prefix_n, out->has_leaf_left, out->has_leaf_right, out->left_child,
-                                           out->edge_count, W.ps, out->node_offsets, min_coord, range, out->nodes,
-                                           out->nodes_capacity, leaf_mask_keep(), L.status);
-    BCHK(cudaGetLastError());
+    BCHK(launch_kernel(Lp, bt_octree_kernel, ogrid, BT_OCT_THREADS, 0, out->keys, out->key_offset, S,
+                       reinterpret_cast<const uint4*>(W.seg_hist), out->prefix_n, out->has_leaf_left,
+                       out->has_leaf_right, out->left_child, out->edge_count, W.ps, out->node_offsets, min_coord, range,
+                       out->nodes, out->nodes_capacity, leaf_mask_keep(), L.status));
   }
 #undef BCHK
   return GTC_OK;

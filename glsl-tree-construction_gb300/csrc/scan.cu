@@ -36,10 +36,12 @@ size_t scan_workspace_bytes(uint32_t n) {
 //   120,000          6.2          6.3          6.2      8.7
 //   1,048,576        8.2         11.4          8.8     17.3
 //   4,000,000       11.1         19.0           -      40.6
-// ROWS is the smallest that keeps the grid within one block per SM: every
+// ROWS is the smallest that keeps the grid within one block per SM (unique) or
+// 5/8 of one (the scan, whose blocks all arrive at their wait together): every
 // block polls all lower blocks' totals, so more blocks cost more than more
-// rows (1,048,576 items in 256 blocks: 13.2 and 12.2).  The largest ROWS may
-// take two blocks per SM, which is still faster than the second read.
+// rows (1,048,576 items in 256 blocks: 13.2 and 12.2; the scan of 300,000 in
+// 147 blocks 10.2, in 74 blocks 5.7).  The largest ROWS may take two blocks
+// per SM, which is still faster than the second read.
 
 // Inclusive scan with the node-offset rules of scan_kernel; a row is 128
 // items, one uint4 per lane, so in/out must be 16-byte aligned.  in holds at
@@ -170,11 +172,11 @@ __global__ void __launch_bounds__(CS_THREADS) row_unique_kernel(const K* kin, co
   if (d_count && blockIdx.x == gridDim.x - 1 && warp == CS_WARPS - 1 && lane == 0) *d_count = run;
 }
 
-// Blocks of a row kernel for n items at `per_block` each, or 0 if one
-// resident wave of at most `per_sm` blocks per SM does not hold them.
-static uint32_t row_grid(const Launch& L, const void* kern, uint32_t n, uint32_t per_block, uint32_t per_sm) {
+// Blocks of a row kernel for n items at `per_block` each, or 0 if they are
+// more than `most` or than one resident wave.
+static uint32_t row_grid(const Launch& L, const void* kern, uint32_t n, uint32_t per_block, uint32_t most) {
   const uint32_t g = ceil_div(n, per_block);
-  if (g > RW_MAX_BLOCKS || g > per_sm * (uint32_t)L.num_sms) return 0u;
+  if (g > RW_MAX_BLOCKS || g > most) return 0u;
   int occ = 0;
   if (kernel_setup(kern, CS_THREADS, 0, &occ) != cudaSuccess) {
     cudaGetLastError();
@@ -501,7 +503,7 @@ template <class K, bool HV, bool IP, int ROWS>
 static bool launch_row_unique(const Launch& L, const K* kin, const uint32_t* vin, K* kout, uint32_t* vout, uint32_t n,
                               uint32_t* d_count, uint32_t* w, cudaError_t* e) {
   auto kern = row_unique_kernel<K, HV, ROWS, IP>;
-  const uint32_t g = row_grid(L, (const void*)kern, n, ROWS * CS_THREADS, ROWS < 16 ? 1u : 2u);
+  const uint32_t g = row_grid(L, (const void*)kern, n, ROWS * CS_THREADS, (ROWS < 16 ? 1u : 2u) * (uint32_t)L.num_sms);
   if (g == 0) {
     if constexpr (ROWS < 16) return launch_row_unique<K, HV, IP, ROWS * 2>(L, kin, vin, kout, vout, n, d_count, w, e);
     return false;
@@ -634,7 +636,8 @@ static bool launch_row_scan(const Launch& L, const uint32_t* in, uint32_t* out, 
                             const uint32_t* d_u, uint32_t n_max, int node_offsets, uint32_t* d_o, uint32_t* w,
                             cudaError_t* e) {
   auto kern = row_scan_kernel<ROWS>;
-  const uint32_t g = row_grid(L, (const void*)kern, n_max, ROWS * 128 * CS_WARPS, ROWS < 8 ? 1u : 2u);
+  const uint32_t g = row_grid(L, (const void*)kern, n_max, ROWS * 128 * CS_WARPS,
+                              ROWS < 8 ? (uint32_t)L.num_sms * 5 / 8 : 2u * (uint32_t)L.num_sms);
   if (g == 0) {
     if constexpr (ROWS < 8)
       return launch_row_scan<ROWS * 2>(L, in, out, count_host, d_u, n_max, node_offsets, d_o, w, e);

@@ -339,8 +339,11 @@ GTC_API gtc_status gtc_build_octree_batched(gtc_ctx* ctx, const float* pts, cons
 /* Tile shapes of the batch's segmented onesweep compiled into the library
  * (threads per block x keys per thread; the tile also divides the clouds for
  * the Morton pass).  A build uses the pinned variant, else the autotuner's
- * pick for its n_total (gtc_autotune_batched), else variant 0.  Every
- * variant gives identical output.  No reference counterpart. */
+ * pick for its n_total (gtc_autotune_batched), else one by n_total: short
+ * tiles up to 600,000 points, variant 0 below 2 million, variant 6 above.
+ * Every variant gives identical output; variant 5's short tiles are for at
+ * most 600,000 points (larger builds pinned to it take variant 0).  No
+ * reference counterpart. */
 GTC_API int gtc_batched_num_variants(void);
 GTC_API gtc_status gtc_batched_variant_shape(int variant, int* threads, int* keys_per_thread);
 /* Pins one variant for every batched build; variant = -1 unpins. */

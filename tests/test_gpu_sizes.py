@@ -209,3 +209,46 @@ def test_tree_nested_long_ranges(ctx, gtc_mod, key_bits, side):
         gtc_mod.lib().gtc_tree_set_method(1)
     for f in want:
         assert torch.equal(got[f], want[f]), f
+
+
+def _spread_clouds(total, seed):
+    """Clouds that add up to `total` points: empty ones first, last and in
+    runs, single points, equal points across row and tile edges, and the rest
+    split over a few large ones."""
+    g = np.random.Generator(np.random.PCG64(seed))
+    small = [0, 0, 1, 31, 0, 32, 33, 0, 0, 0, 1, 2047, 2048, 2049, 1, 1, 4097]
+    big = total - sum(small)
+    sizes = small + [big // 3, 0, big // 2, 0, big - big // 3 - big // 2, 0, 0]
+    clouds = []
+    for k, n in enumerate(sizes):
+        p = W.uniform_points(n, seed=seed + k) if n else np.zeros((0, 4), np.float32)
+        if n and k % 3 == 0:
+            p = p[g.integers(0, max(n // 5, 1), n)]  # five points per code
+        clouds.append(p)
+    return clouds
+
+
+@pytest.mark.parametrize("total,variant", [(599_999, -1), (600_000, 5), (600_001, 5), (600_001, -1), (1_999_999, -1),
+                                           (2_000_000, -1), (2_700_001, 6), (13_001, 6), (13_001, -1)])
+def test_batched_sizes(ctx, gtc_mod, oracle, total, variant):
+    """Both sides of every size rule of the batch (tile shape, tree window,
+    unique's rows or segments), over a range that is no power of two."""
+    import torch
+
+    from test_gpu_pipeline import _cmp
+
+    clouds = _spread_clouds(total, seed=total)
+    off = np.concatenate(([0], np.cumsum([c.shape[0] for c in clouds]))).astype(np.uint32)
+    pts = np.ascontiguousarray(np.concatenate(clouds))
+    try:
+        gtc_mod.batched_set_variant(variant)
+        res = gtc_mod.build_octree_batched(ctx, torch.from_numpy(pts).cuda(), torch.from_numpy(off.view(np.int32)).cuda(),
+                                           min_coord=-3.0, rng=1100.0)
+    finally:
+        gtc_mod.batched_set_variant(-1)
+    for c, r in enumerate(res):
+        if clouds[c].shape[0] == 0:
+            assert (r.n_unique, r.n_brt_nodes, r.n_oct_nodes) == (0, 0, 0)
+            continue
+        exp, _ = oracle.build_octree(clouds[c], 32, min_coord=-3.0, rng=1100.0, threads=8)
+        _cmp(r, exp, 32, (total, c))
