@@ -435,10 +435,13 @@ gtc_status pipeline(gtc_ctx* ctx, const float* pts, uint32_t n, float mn, float 
     StageTimer t(ctx, stream, GTC_STAGE_UNIQUE);
     GTC_TRY(ctx, launch_unique<K>(Lp, keys_alt, vals_alt, keys, o->idx, n, o->counts + 0, unique_ws));
   }
+  // vals_alt is free once unique has compacted: the window tree leaves the
+  // split records there for the octree.
+  uint32_t* rec = tree_get_method() == 1 ? vals_alt : nullptr;
   {
     StageTimer t(ctx, stream, GTC_STAGE_RADIX_TREE);
     GTC_TRY(ctx, launch_radix_tree<K>(Lp, keys, o->counts + 0, 0, n, o->prefix_n, o->has_leaf_left,
-                                      o->has_leaf_right, o->left_child, o->parent, o->edge_count, o->counts + 1));
+                                      o->has_leaf_right, o->left_child, o->parent, o->edge_count, o->counts + 1, rec));
   }
   {
     StageTimer t(ctx, stream, GTC_STAGE_PREFIX_SUM);
@@ -447,6 +450,12 @@ gtc_status pipeline(gtc_ctx* ctx, const float* pts, uint32_t n, float mn, float 
   }
   {
     StageTimer t(ctx, stream, GTC_STAGE_OCTREE);
+    if (rec) {
+      GTC_TRY(ctx, launch_octree_records<K>(Lp, keys, o->counts + 0, n, rec, o->prefix_n, o->has_leaf_left,
+                                            o->has_leaf_right, o->left_child, o->edge_count, o->node_offsets, mn, rg,
+                                            o->nodes, o->nodes_capacity));
+      return GTC_OK;
+    }
     GTC_TRY(ctx, launch_octree_make<K>(Lp, keys, o->counts + 0, 0, n, o->prefix_n, o->has_leaf_left,
                                        o->has_leaf_right, o->left_child, o->edge_count, o->node_offsets, mn, rg,
                                        o->nodes, o->nodes_capacity, true));

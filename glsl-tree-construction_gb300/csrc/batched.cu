@@ -30,7 +30,7 @@
 #include <utility>
 
 #include "karras.cuh"
-#include "octree_dev.cuh"
+#include "octree_window.cuh"
 #include "scan_dev.cuh"
 #include "tree_window.cuh"
 
@@ -907,14 +907,17 @@ gtc_status build_octree_batched_variant(gtc_ctx* ctx, const float* pts, const ui
                              reinterpret_cast<uint32_t*>(W.unique_ws),
                              (uint32_t)(scan_workspace_bytes(n_total) / 4) - 64, bad));
   }
+  // idx_alt is free after unique: the window tree leaves the split records
+  // there for the octree.
+  uint32_t* rec = tree_get_method() == 1 ? W.idx_alt : nullptr;
   {
     Stage t(ctx, stream, GTC_STAGE_RADIX_TREE);
-    if (tree_get_method() == 1) {
+    if (rec) {
       auto window = [&](auto shape) {
         using SH = decltype(shape);
         return launch_kernel(Lp, radix_tree_window_kernel<uint32_t, true, SH>, ceil_div(n_total, SH::T), TW_THREADS, 0,
                              out->keys, nullptr, 0u, out->key_offset, S, out->prefix_n, out->has_leaf_left,
-                             out->has_leaf_right, out->left_child, out->parent, out->edge_count, nullptr);
+                             out->has_leaf_right, out->left_child, out->parent, out->edge_count, nullptr, rec);
       };
       BCHK(n_total <= TW_SMALL_MAX ? window(TwSmall{}) : window(TwSegLarge{}));
     } else {
@@ -933,6 +936,14 @@ gtc_status build_octree_batched_variant(gtc_ctx* ctx, const float* pts, const ui
   }
   {
     Stage t(ctx, stream, GTC_STAGE_OCTREE);
+    if (rec) {
+      BCHK((launch_octree_window<uint32_t, true>(Lp, out->keys, nullptr, out->key_offset, S,
+                                                 reinterpret_cast<const uint4*>(W.seg_hist), n_total, rec,
+                                                 out->prefix_n, out->has_leaf_left, out->has_leaf_right,
+                                                 out->left_child, out->edge_count, W.ps, out->node_offsets, min_coord,
+                                                 range, out->nodes, out->nodes_capacity)));
+      return GTC_OK;
+    }
     int occ = 4;  // resident blocks per SM
     if (kernel_setup(bt_octree_kernel, BT_OCT_THREADS, 0, &occ) != cudaSuccess) {
       cudaGetLastError();

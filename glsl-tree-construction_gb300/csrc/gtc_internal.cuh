@@ -565,7 +565,8 @@ cudaError_t launch_node_offsets(const Launch& L, const uint32_t* edge, uint32_t*
 template <class K>
 cudaError_t launch_radix_tree(const Launch& L, const K* codes, const uint32_t* d_u, int32_t m_host, uint32_t n_max,
                               uint8_t* prefix_n, uint8_t* hll, uint8_t* hlr, int32_t* left, int32_t* parent,
-                              uint32_t* edge, uint32_t* d_m /* nullable: receives m */);
+                              uint32_t* edge, uint32_t* d_m /* nullable: receives m */,
+                              uint32_t* rec = nullptr /* method 1: n_max split records (split_rec.cuh) */);
 // Radix tree method: 1 split-indexed window kernel (default), 0 per-node Karras.
 int tree_get_method();
 bool tree_set_method(int m);
@@ -578,6 +579,13 @@ cudaError_t launch_octree_make(const Launch& L, const K* codes, const uint32_t* 
                                uint32_t n_max, const uint8_t* prefix_n, const uint8_t* hll, const uint8_t* hlr,
                                const int32_t* left, const uint32_t* edge, const uint32_t* ps, float mn, float rg,
                                gtc_octnode* nodes, uint32_t capacity, bool with_leaves);
+// The fused build's octree, make and link, from the split records of
+// launch_radix_tree (method 1): u codes, u on the device (octree_window.cuh).
+template <class K>
+cudaError_t launch_octree_records(const Launch& L, const K* codes, const uint32_t* d_u, uint32_t n_max,
+                                  const uint32_t* rec, const uint8_t* prefix_n, const uint8_t* hll, const uint8_t* hlr,
+                                  const int32_t* left, const uint32_t* edge, const uint32_t* ps, float mn, float rg,
+                                  gtc_octnode* nodes, uint32_t capacity);
 template <class K>
 cudaError_t launch_octree_link(const Launch& L, const K* codes, uint32_t m, const uint8_t* prefix_n,
                                const uint8_t* hll, const uint8_t* hlr, const int32_t* left, const int32_t* parent,

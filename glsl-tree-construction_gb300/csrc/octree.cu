@@ -2,6 +2,7 @@
 // operator for callers that run make and link as separate stages.
 
 #include "octree_dev.cuh"
+#include "octree_window.cuh"
 
 namespace gtc {
 
@@ -93,6 +94,23 @@ template cudaError_t launch_octree_make<uint64_t>(const Launch&, const uint64_t*
                                                   const uint8_t*, const uint8_t*, const uint8_t*, const int32_t*,
                                                   const uint32_t*, const uint32_t*, float, float, gtc_octnode*,
                                                   uint32_t, bool);
+
+template <class K>
+cudaError_t launch_octree_records(const Launch& L, const K* codes, const uint32_t* d_u, uint32_t n_max,
+                                  const uint32_t* rec, const uint8_t* prefix_n, const uint8_t* hll, const uint8_t* hlr,
+                                  const int32_t* left, const uint32_t* edge, const uint32_t* ps, float mn, float rg,
+                                  gtc_octnode* nodes, uint32_t capacity) {
+  return launch_octree_window<K, false>(L, codes, d_u, nullptr, 0, nullptr, n_max, rec, prefix_n, hll, hlr, left, edge,
+                                        ps, nullptr, mn, rg, nodes, capacity);
+}
+template cudaError_t launch_octree_records<uint32_t>(const Launch&, const uint32_t*, const uint32_t*, uint32_t,
+                                                     const uint32_t*, const uint8_t*, const uint8_t*, const uint8_t*,
+                                                     const int32_t*, const uint32_t*, const uint32_t*, float, float,
+                                                     gtc_octnode*, uint32_t);
+template cudaError_t launch_octree_records<uint64_t>(const Launch&, const uint64_t*, const uint32_t*, uint32_t,
+                                                     const uint32_t*, const uint8_t*, const uint8_t*, const uint8_t*,
+                                                     const int32_t*, const uint32_t*, const uint32_t*, float, float,
+                                                     gtc_octnode*, uint32_t);
 
 // k_LinkLeafNodes (octree.comp:188-222) in push form: each leaf child is
 // stored into the bottom node of the nearest contributing ancestor (the walk

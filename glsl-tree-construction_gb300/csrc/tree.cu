@@ -51,15 +51,15 @@ __global__ void __launch_bounds__(TREE_THREADS) radix_tree_kernel(const K* __res
 template <class K>
 cudaError_t launch_radix_tree(const Launch& L, const K* codes, const uint32_t* d_u, int32_t m_host, uint32_t n_max,
                               uint8_t* prefix_n, uint8_t* hll, uint8_t* hlr, int32_t* left, int32_t* parent,
-                              uint32_t* edge, uint32_t* d_m) {
+                              uint32_t* edge, uint32_t* d_m, uint32_t* rec) {
   const uint32_t work = d_u ? n_max : (uint32_t)max(m_host, 0);
   if (work == 0 && !d_m) return cudaSuccess;
-  if (g_tree_method.load(std::memory_order_relaxed) == 1) {
+  if (rec || g_tree_method.load(std::memory_order_relaxed) == 1) {  // records: the caller chose the window method
     const uint32_t u_host = d_u ? 0u : (uint32_t)max(m_host, 0) + 1;
     auto window = [&](auto shape) {
       using SH = decltype(shape);
       return launch_kernel(L, radix_tree_window_kernel<K, false, SH>, max(1u, ceil_div(work, SH::T)), TW_THREADS, 0,
-                           codes, d_u, u_host, nullptr, 0u, prefix_n, hll, hlr, left, parent, edge, d_m);
+                           codes, d_u, u_host, nullptr, 0u, prefix_n, hll, hlr, left, parent, edge, d_m, rec);
     };
     return work <= TW_SMALL_MAX ? window(TwSmall{}) : window(TwLarge{});
   }
@@ -69,9 +69,11 @@ cudaError_t launch_radix_tree(const Launch& L, const K* codes, const uint32_t* d
   return cudaGetLastError();
 }
 template cudaError_t launch_radix_tree<uint32_t>(const Launch&, const uint32_t*, const uint32_t*, int32_t, uint32_t,
-                                                 uint8_t*, uint8_t*, uint8_t*, int32_t*, int32_t*, uint32_t*, uint32_t*);
+                                                 uint8_t*, uint8_t*, uint8_t*, int32_t*, int32_t*, uint32_t*, uint32_t*,
+                                                 uint32_t*);
 template cudaError_t launch_radix_tree<uint64_t>(const Launch&, const uint64_t*, const uint32_t*, int32_t, uint32_t,
-                                                 uint8_t*, uint8_t*, uint8_t*, int32_t*, int32_t*, uint32_t*, uint32_t*);
+                                                 uint8_t*, uint8_t*, uint8_t*, int32_t*, int32_t*, uint32_t*, uint32_t*,
+                                                 uint32_t*);
 
 // edge_count.comp:30-41 over exactly m nodes, depth = (prefix_n - A) / 3.
 __global__ void edge_count_kernel(const uint8_t* __restrict__ prefix_n, const int32_t* __restrict__ parent,

@@ -34,6 +34,7 @@
 #pragma once
 
 #include "gtc_internal.cuh"
+#include "split_rec.cuh"
 
 namespace gtc {
 
@@ -363,10 +364,11 @@ __device__ __forceinline__ uint32_t tw_range_lo(const K* codes, uint32_t x, uint
 template <int A>
 __device__ __forceinline__ void tw_emit(uint32_t x, uint32_t t, uint32_t lo, uint32_t hi, uint32_t dL, uint32_t dR,
                                         uint32_t U0, uint8_t* prefix_n, uint8_t* hll, uint8_t* hlr, int32_t* left,
-                                        int32_t* parent, uint32_t* edge) {
+                                        int32_t* parent, uint32_t* edge, uint32_t* rec) {
   uint32_t idx;
   uint32_t e = 0;
-  if (dL == 0 && dR == 0) {
+  const bool root = dL == 0 && dR == 0;
+  if (root) {
     idx = U0;  // the root of this cloud (D13: its parent reads 0)
     parent[idx] = 0;
   } else {
@@ -374,6 +376,7 @@ __device__ __forceinline__ void tw_emit(uint32_t x, uint32_t t, uint32_t lo, uin
     e = (t - A) / 3 - (max(dL, dR) - A) / 3;
   }
   if (edge) edge[idx] = e;
+  if (rec) rec[x] = split_pack(x, lo, hi, idx, root ? SPLIT_ROOT : e, (t - A) / 3, dR > dL);
   prefix_n[idx] = (uint8_t)t;
   left[idx] = (int32_t)(x - U0);
   hll[idx] = lo == x;
@@ -387,7 +390,7 @@ __device__ __forceinline__ void tw_emit(uint32_t x, uint32_t t, uint32_t lo, uin
 template <class K>
 __device__ __forceinline__ void tw_warp_split(const K* codes, uint32_t x, uint32_t U0, uint32_t U1,
                                               uint8_t* prefix_n, uint8_t* hll, uint8_t* hlr, int32_t* left,
-                                              int32_t* parent, uint32_t* edge) {
+                                              int32_t* parent, uint32_t* edge, uint32_t* rec) {
   constexpr int A = KeyTraits<K>::A;
   const int t = delta_key(codes[x], codes[x + 1]);
   const uint2 r = tw_warp_range<K>(codes, x, U0, U1 - 1, t);
@@ -395,18 +398,20 @@ __device__ __forceinline__ void tw_warp_split(const K* codes, uint32_t x, uint32
     const uint32_t lo = r.x, hi = r.y;
     const uint32_t dR = (hi + 1 < U1) ? (uint32_t)delta_key(codes[hi], codes[hi + 1]) : 0u;
     const uint32_t dL = (lo > U0) ? (uint32_t)delta_key(codes[lo - 1], codes[lo]) : 0u;
-    tw_emit<A>(x, (uint32_t)t, lo, hi, dL, dR, U0, prefix_n, hll, hlr, left, parent, edge);
+    tw_emit<A>(x, (uint32_t)t, lo, hi, dL, dR, U0, prefix_n, hll, hlr, left, parent, edge, rec);
   }
 }
 
 // One block: splits [blockIdx.x * T, + T).  SEG: clouds of codes start at
 // uoff[0..S] (uoff[S] = U), indices written are cloud-local, and the last
-// slot of every cloud gets edge 0.  Otherwise one cloud of U codes.
+// slot of every cloud gets edge 0.  Otherwise one cloud of U codes.  rec
+// (nullable) receives every split's record (split_rec.cuh).
 template <class K, bool SEG, class SH>
 __global__ void __launch_bounds__(TW_THREADS, 4) radix_tree_window_kernel(
     const K* __restrict__ codes, const uint32_t* d_u, uint32_t u_host, const uint32_t* uoff, uint32_t S,
     uint8_t* __restrict__ prefix_n, uint8_t* __restrict__ hll, uint8_t* __restrict__ hlr,
-    int32_t* __restrict__ left, int32_t* __restrict__ parent, uint32_t* __restrict__ edge, uint32_t* d_m) {
+    int32_t* __restrict__ left, int32_t* __restrict__ parent, uint32_t* __restrict__ edge, uint32_t* d_m,
+    uint32_t* __restrict__ rec) {
   griddep_wait();
   constexpr int A = KeyTraits<K>::A;
   __shared__ TwSmem<SH> s;
@@ -511,6 +516,7 @@ __global__ void __launch_bounds__(TW_THREADS, 4) radix_tree_window_kernel(
     const uint32_t t = s.d[xi];
     if (t == 0) {  // the last key of a cloud: no split here
       if (SEG && edge) edge[x] = 0;
+      if (rec) rec[x] = SPLIT_NONE;
       continue;
     }
     const int r = (lr & 15) ? cstart + (int)(lr & 15) : tw_next_tab(s, chunk, t);
@@ -539,7 +545,7 @@ __global__ void __launch_bounds__(TW_THREADS, 4) radix_tree_window_kernel(
       lo = tw_range_lo<K>(codes, x, U0, (int)t);
       dL = (lo > U0) ? (uint32_t)delta_key(codes[lo - 1], codes[lo]) : 0u;
     }
-    tw_emit<A>(x, t, lo, hi, dL, dR, U0, prefix_n, hll, hlr, left, parent, edge);
+    tw_emit<A>(x, t, lo, hi, dL, dR, U0, prefix_n, hll, hlr, left, parent, edge, rec);
   }
 
   // 5. the block's long-range splits, one warp each (both ends searched
@@ -554,7 +560,7 @@ __global__ void __launch_bounds__(TW_THREADS, 4) radix_tree_window_kernel(
       U0 = uoff[c];
       U1 = uoff[c + 1];
     }
-    tw_warp_split<K>(codes, x, U0, U1, prefix_n, hll, hlr, left, parent, edge);
+    tw_warp_split<K>(codes, x, U0, U1, prefix_n, hll, hlr, left, parent, edge, rec);
   }
 }
 

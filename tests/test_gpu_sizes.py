@@ -252,3 +252,71 @@ def test_batched_sizes(ctx, gtc_mod, oracle, total, variant):
             continue
         exp, _ = oracle.build_octree(clouds[c], 32, min_coord=-3.0, rng=1100.0, threads=8)
         _cmp(r, exp, 32, (total, c))
+
+
+def _nested_cloud(key_bits, side, seed):
+    """Points at the centres of the finest cells whose codes nest one long
+    range per bit (test_tree_nested_long_ranges), in shuffled order: octree
+    nodes of every span, most levels of the path far wider than a block."""
+    axis, bits = (10, 30) if key_bits == 32 else (21, 63)
+    g = np.random.Generator(np.random.PCG64(seed))
+    path = {"right": (1 << bits) - 1, "left": 0, "both": 0x2AAAAAAAAAAAAAAA & ((1 << bits) - 1)}[side]
+    parts = [np.array([path], np.uint64)]
+    for b in range(bits - 1, 8, -1):
+        base = ((path >> b) ^ 1) << b
+        parts.append(np.uint64(base) + g.choice(1 << min(b, 20), min(300, 1 << b), replace=False).astype(np.uint64))
+    codes = np.unique(np.concatenate(parts))
+    pts = np.ones((codes.size, 4), np.float32)
+    for a in range(3):
+        q = np.zeros(codes.size, np.uint64)
+        for b in range(axis):
+            q |= ((codes >> np.uint64(3 * b + a)) & np.uint64(1)) << np.uint64(b)
+        pts[:, a] = (q.astype(np.float64) + 0.5) * (1024.0 / (1 << axis))
+    return pts[g.permutation(codes.size)]
+
+
+@pytest.mark.parametrize("key_bits", [32, 64])
+@pytest.mark.parametrize("side", ["right", "left", "both"])
+def test_octree_window_far_owners(ctx, gtc_mod, oracle, key_bits, side):
+    """Octree nodes assembled in a block's window and those gathered past it,
+    in the single and the batched build, against the oracle."""
+    import torch
+
+    from test_gpu_pipeline import _cmp
+
+    clouds = [_nested_cloud(key_bits, side, 1), W.uniform_points(5000, seed=2), _nested_cloud(key_bits, side, 3)]
+    for c, pts in enumerate(clouds):
+        exp, _ = oracle.build_octree(pts, key_bits, threads=8)
+        _cmp(gtc_mod.build_octree(ctx, torch.from_numpy(pts).cuda(), key_bits), exp, key_bits, (side, c))
+    if key_bits == 32:
+        off = np.concatenate(([0], np.cumsum([c.shape[0] for c in clouds]))).astype(np.int32)
+        res = gtc_mod.build_octree_batched(ctx, torch.from_numpy(np.concatenate(clouds)).cuda(),
+                                           torch.from_numpy(off).cuda())
+        for c, r in enumerate(res):
+            exp, _ = oracle.build_octree(clouds[c], 32, threads=8)
+            _cmp(r, exp, 32, (side, c, "batch"))
+
+
+@pytest.mark.parametrize("key_bits", [32, 64])
+@pytest.mark.parametrize("n", [1888, 1889, 4097, 5665, 9441, 50_001])
+def test_octree_window_tiles(ctx, gtc_mod, oracle, key_bits, n):
+    """Code counts around the octree window's tiles of 1,888 splits (four
+    thousand points and more take the stage kernels; a capacity one short is
+    flagged and the rest written)."""
+    import torch
+
+    from test_gpu_pipeline import _cmp
+
+    pts = np.concatenate((W.gaussian_mixture_points(max(n, 4097), 4, 3.0, noise=0.3, seed=n)[:n],
+                          np.repeat(W.uniform_points(1, seed=n), max(4097 - n, 0), axis=0)))
+    d = torch.from_numpy(np.ascontiguousarray(pts)).cuda()
+    exp, _ = oracle.build_octree(pts, key_bits)
+    plan = gtc_mod.OctreePlan(ctx, pts.shape[0], key_bits, nodes_capacity=exp["n_oct_nodes"])
+    plan.launch(d)
+    _cmp(plan.result(), exp, key_bits, n)
+    short = gtc_mod.OctreePlan(ctx, pts.shape[0], key_bits, nodes_capacity=exp["n_oct_nodes"] - 1)
+    short.launch(d)
+    assert ctx.device_status_code() == 7
+    got = gtc_mod.nodes_to_numpy(short.nodes)
+    same = (got.view(np.int32).reshape(-1, 16) == exp["nodes"][:-1].view(np.int32).reshape(-1, 16)).all(axis=1)
+    assert same.sum() >= same.size - 21  # only nodes that share an owner with the one that did not fit
