@@ -250,8 +250,8 @@ gtc_status sort_pairs_impl(gtc_ctx* ctx, K* keys, uint32_t* vals, K* keys_alt, u
   const SortWorkspace Wk = carve_sort_workspace(ws, n, passes, 0);
   GTC_TRY(ctx, cudaMemsetAsync(Wk.header, 0, Wk.header_words * 4, S(stream)));
   if (ctx->skip_first_tile) {
-    // The LAST pass's tile tickets start at 1 (header word 1 + p is pass p's
-    // counter; byte 0 of the little-endian word): its tile 0 is never sorted
+    // The LAST pass's tiles start at 1 (header word 1 + p is pass p's counter or
+    // first tile; byte 0 of the little-endian word): its tile 0 is never sorted
     // or published.  The last pass reads input whose digit counts match the
     // global histogram, so a tile's writes for digit d land in
     // [bin_off[d] + excl, bin_off[d] + excl + count) and a timed-out look-back

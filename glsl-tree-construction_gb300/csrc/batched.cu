@@ -8,7 +8,7 @@
 // One launch per stage for the whole batch, every size read on the device, so
 // the batch captures into one CUDA graph:
 //   1. tiles:   each cloud is cut into its own tiles; tile_start[c] is the
-//               first tile of cloud c (a device work list pulled by ticket);
+//               first tile of cloud c (a device work list, block b taking tile b);
 //   2. morton:  32-bit codes, cloud-local point index payload, per-cloud
 //               digit histograms of the 4 passes;
 //   3. segmented onesweep, 4 passes: a tile's digit bases come from its own
@@ -258,7 +258,6 @@ struct BtSmem {
   uint32_t warp_hist[WARPS][BRADIX];
   uint32_t gbase[BRADIX];
   uint32_t warp_sums[WARPS + 1];
-  uint32_t tile_id;
 };
 
 // One segmented onesweep pass: the single-cloud pass of sort.cu with tiles
@@ -275,7 +274,7 @@ __global__ void __launch_bounds__(THREADS, MINB) bt_onesweep_kernel(const uint32
                                                                  uint32_t S, const uint32_t* tile_start,
                                                                  const uint32_t* tile_cloud, int shift,
                                                                  const uint32_t* seg_base, int pass, uint32_t* desc,
-                                                                 uint32_t* tile_counter, uint32_t* status) {
+                                                                 uint32_t* status) {
   griddep_wait();
   using Sm = BtSmem<THREADS, KPT>;
   constexpr int WARPS = Sm::WARPS;
@@ -284,10 +283,7 @@ __global__ void __launch_bounds__(THREADS, MINB) bt_onesweep_kernel(const uint32
   Sm& s = *reinterpret_cast<Sm*>(smem_raw);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t lt_mask = (1u << lane) - 1u;
-  for (int i = tid; i < WARPS * BRADIX; i += THREADS) (&s.warp_hist[0][0])[i] = 0;
-  if (tid == 0) s.tile_id = atomicAdd(tile_counter, 1u);
-  __syncthreads();
-  const uint32_t tile = s.tile_id;
+  const uint32_t tile = blockIdx.x;  // blocks start in increasing order (sort.cu)
   if (tile >= tile_start[S]) return;
   const TileRange r = tile_range(tile, tile_cloud[tile], tile_start, off, Sm::TILE);
 
@@ -301,6 +297,9 @@ __global__ void __launch_bounds__(THREADS, MINB) bt_onesweep_kernel(const uint32
     else val[j] = (i < r.valid) ? vin[r.base + i] : 0u;
   }
   uint32_t* my_hist = s.warp_hist[warp];
+#pragma unroll
+  for (int i = 0; i < BRADIX / 32; ++i) my_hist[i * 32 + lane] = 0;
+  __syncwarp();
 #pragma unroll
   for (int j = 0; j < KPT; ++j) {
     const uint32_t d = (key[j] >> shift) & 255u;
@@ -706,7 +705,6 @@ struct BtPass {
   int pass;
   const uint32_t* seg_base;
   uint32_t* desc;
-  uint32_t* tile_counter;
 };
 
 template <int THREADS, int KPT, int MINB>
@@ -716,7 +714,7 @@ cudaError_t launch_bt_pass(const Launch& L, uint32_t grid, const BtPass& a) {
   cudaError_t e = kernel_setup(kern, THREADS, sizeof(Sm));
   if (e != cudaSuccess) return e;
   return launch_kernel(L, kern, grid, THREADS, sizeof(Sm), a.kin, a.vin, a.kout, a.vout, a.off, a.S, a.tile_start,
-                       a.tile_cloud, 8 * a.pass, a.seg_base, a.pass, a.desc, a.tile_counter, L.status);
+                       a.tile_cloud, 8 * a.pass, a.seg_base, a.pass, a.desc, L.status);
 }
 
 cudaError_t launch_bt_variant(int v, const Launch& L, uint32_t grid, const BtPass& a) {
@@ -766,7 +764,7 @@ struct BatchWs {
   void* unique_ws;
   void* scan_ws;
   size_t zero_vecs;      // 16-byte words from seg_hist on that are cleared
-  uint32_t* counters;    // [0..3] pass tickets
+  uint32_t* counters;    // [8] bad batch
   uint32_t* desc;        // [4][tiles_max][256]
   uint32_t* keys_alt;    // [n]
   uint32_t* idx_alt;     // [n]
@@ -896,7 +894,7 @@ gtc_status build_octree_batched_variant(gtc_ctx* ctx, const float* pts, const ui
     Stage t(ctx, stream, GTC_STAGE_ONESWEEP);
     BCHK(launch_bt_variant(variant, Lp, W.tiles_max,
                            BtPass{src_k, src_v, dst_k, dst_v, d_offsets, S, W.tile_start, W.tile_cloud, p, W.seg_hist,
-                                  W.desc + (size_t)p * W.tiles_max * BRADIX, W.counters + p}));
+                                  W.desc + (size_t)p * W.tiles_max * BRADIX}));
     std::swap(src_k, dst_k);
     std::swap(src_v, dst_v);
   }

@@ -428,15 +428,14 @@ struct LpSmem {
   uint32_t warp_hist[WARPS][LP_RADIX];
   uint32_t gbase[LP_RADIX];
   uint32_t warp_sums[LP_RADIX / 32];
-  uint32_t tile_id;
 };
 
 template <bool FIRST, int THREADS, int KPT>
 __global__ void __launch_bounds__(THREADS) learned_pass_kernel(
     const uint64_t* __restrict__ kin, const uint32_t* __restrict__ vin, const uint16_t* __restrict__ bin,
     uint64_t* __restrict__ kout, uint32_t* __restrict__ vout, uint16_t* __restrict__ bout, uint32_t n, int shift,
-    uint32_t mask, const uint32_t* __restrict__ bin_off, uint32_t* __restrict__ desc, uint32_t* tile_counter,
-    uint32_t* status, const uint32_t* flags) {
+    uint32_t mask, const uint32_t* __restrict__ bin_off, uint32_t* __restrict__ desc, uint32_t* status,
+    const uint32_t* flags) {
   if (*flags & (LFLAG_OVERFLOW | LFLAG_BAD_MODEL)) return;
   using Sm = LpSmem<THREADS, KPT>;
   constexpr int WARPS = Sm::WARPS;
@@ -447,9 +446,8 @@ __global__ void __launch_bounds__(THREADS) learned_pass_kernel(
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t lt_mask = (1u << lane) - 1u;
   for (int i = tid; i < WARPS * LP_RADIX; i += THREADS) (&s.warp_hist[0][0])[i] = 0;
-  if (tid == 0) s.tile_id = atomicAdd(tile_counter, 1u);
   __syncthreads();
-  const uint32_t tile = s.tile_id;
+  const uint32_t tile = blockIdx.x;  // blocks start in increasing order (sort.cu); a ticket cost 1% of the sort
   const uint32_t tbase = tile * TILE;
 
   uint64_t key[KPT];
@@ -847,7 +845,6 @@ struct LearnedWorkspace {
   uint32_t* base;     // [B]
   uint64_t* bmin;     // [B]
   uint64_t* bmax;     // [B]
-  uint32_t* misc;     // [1], [2]: pass tile tickets
   uint32_t* off1;     // [128] digit bases of pass 1
   uint32_t* off2;     // [128] digit bases of pass 2
   uint16_t* bid;      // [n] bucket ids
@@ -874,7 +871,6 @@ static size_t learned_ws_layout(uint32_t n, int B, LearnedWorkspace* W, char* p)
   w.base = reinterpret_cast<uint32_t*>(take((size_t)B * 4));
   w.bmin = reinterpret_cast<uint64_t*>(take((size_t)B * 8));
   w.bmax = reinterpret_cast<uint64_t*>(take((size_t)B * 8));
-  w.misc = reinterpret_cast<uint32_t*>(take(256));
   w.off1 = reinterpret_cast<uint32_t*>(take(LP_RADIX * 4));
   w.off2 = reinterpret_cast<uint32_t*>(take(LP_RADIX * 4));
   w.bid = reinterpret_cast<uint16_t*>(take((size_t)n * 2));
@@ -948,22 +944,22 @@ gtc_status launch_count(gtc_ctx* ctx, const gtc_learned_model* m, const uint64_t
 template <bool FIRST, int THREADS, int KPT>
 cudaError_t launch_lp_shape(cudaStream_t s, uint32_t n, const uint64_t* kin, const uint32_t* vin, const uint16_t* bin,
                             uint64_t* kout, uint32_t* vout, uint16_t* bout, int shift, uint32_t mask,
-                            const uint32_t* off, uint32_t* desc, uint32_t* tc, uint32_t* status,
+                            const uint32_t* off, uint32_t* desc, uint32_t* status,
                             const uint32_t* flags) {
   using Sm = LpSmem<THREADS, KPT>;
   cudaError_t e = kernel_setup(learned_pass_kernel<FIRST, THREADS, KPT>, THREADS, sizeof(Sm));
   if (e != cudaSuccess) return e;
   learned_pass_kernel<FIRST, THREADS, KPT><<<ceil_div(n, (uint32_t)Sm::TILE), THREADS, sizeof(Sm), s>>>(
-      kin, vin, bin, kout, vout, bout, n, shift, mask, off, desc, tc, status, flags);
+      kin, vin, bin, kout, vout, bout, n, shift, mask, off, desc, status, flags);
   return cudaGetLastError();
 }
 
 template <bool FIRST>
 cudaError_t launch_lp(int v, cudaStream_t s, uint32_t n, const uint64_t* kin, const uint32_t* vin,
                       const uint16_t* bin, uint64_t* kout, uint32_t* vout, uint16_t* bout, int shift, uint32_t mask,
-                      const uint32_t* off, uint32_t* desc, uint32_t* tc, uint32_t* status, const uint32_t* flags) {
+                      const uint32_t* off, uint32_t* desc, uint32_t* status, const uint32_t* flags) {
 #define GTC_LP(T, K) \
-  return launch_lp_shape<FIRST, T, K>(s, n, kin, vin, bin, kout, vout, bout, shift, mask, off, desc, tc, status, flags)
+  return launch_lp_shape<FIRST, T, K>(s, n, kin, vin, bin, kout, vout, bout, shift, mask, off, desc, status, flags)
   switch (v) {
     case 1: GTC_LP(512, 12);
     case 2: GTC_LP(384, 16);
@@ -1138,7 +1134,6 @@ gtc_status learned_sort_variant(gtc_ctx* ctx, const gtc_learned_model* m, const 
   const int db1 = (lb + 1) / 2, db2 = lb - db1;      // digit widths of the two passes (<= 7 each)
   LTRY(ctx, kernel_setup(bucket_sort_kernel, BS_THREADS, sizeof(BucketSmem)));
   const Launch L0 = context_launch(ctx, stream);
-  LTRY(ctx, cudaMemsetAsync(W.misc, 0, 256, s));
   LTRY(ctx, cudaMemsetAsync(W.totals, 0, (size_t)B * 4, s));
   LTRY(ctx, cudaMemsetAsync(W.desc, 0, 2 * W.desc_words * 4, s));
   gtc_status st = prepare_model(ctx, m, d_flags, s);
@@ -1147,10 +1142,10 @@ gtc_status learned_sort_variant(gtc_ctx* ctx, const gtc_learned_model* m, const 
   learned_scan_kernel<<<1, 1024, 0, s>>>(W.totals, B, db1, m->heights, W.base, W.off1, W.off2, d_flags);
   LTRY(ctx, cudaGetLastError());
   LTRY(ctx, launch_lp<true>(variant, s, n, keys, vals, W.bid, db2 ? W.tkeys : W.ukeys, db2 ? W.tvals : W.uvals,
-                            W.bid2, 0, (1u << db1) - 1, W.off1, W.desc, W.misc + 1, L0.status, d_flags));
+                            W.bid2, 0, (1u << db1) - 1, W.off1, W.desc, L0.status, d_flags));
   if (db2)
     LTRY(ctx, launch_lp<false>(variant, s, n, W.tkeys, W.tvals, W.bid2, W.ukeys, W.uvals, nullptr, db1,
-                               (1u << db2) - 1, W.off2, W.desc + W.desc_words, W.misc + 2, L0.status, d_flags));
+                               (1u << db2) - 1, W.off2, W.desc + W.desc_words, L0.status, d_flags));
   bucket_sort_kernel<<<B, BS_THREADS, sizeof(BucketSmem), s>>>(W.ukeys, W.uvals, W.base, W.totals, keys_out, vals_out,
                                                                W.bmin, W.bmax, d_flags);
   learned_order_check_kernel<<<ceil_div(B, 256), 256, 0, s>>>(W.totals, W.bmin, W.bmax, B, d_flags);

@@ -6,8 +6,12 @@
 // carried alongside the keys and 8-bit digits over [begin_bit, end_bit).
 //
 // One pass over a tile of TILE = THREADS * KPT keys:
-//   1. tile ticket from an atomic counter (tiles start in ticket order, so a
-//      tile only ever waits on tiles that are already running);
+//   1. block b takes tile b: blocks start in increasing order, so a tile only
+//      ever waits on tiles that are already running or done (and every wait is
+//      bounded).  A ticket from an atomic counter costs a tile 2,100 of its
+//      20,000 to 23,000 cycles before its first load; only variant 2 keeps it,
+//      the fastest on 64-bit inputs of tens of millions of keys, where tickets
+//      keep the tiles' order tighter (33.5M pairs: 1809 us, 1854 without);
 //   2. warp-striped coalesced loads (lane l of warp w holds keys
 //      w*32*KPT + j*32 + l), padding past n with all-ones keys (max digit);
 //   3. warp-level multisplit: 8 __ballot_sync per key give the peer mask of
@@ -488,10 +492,11 @@ struct OnesweepSmem {
   uint32_t digit_offset[RADIX];
   uint32_t global_base[RADIX];
   uint32_t warp_sums[8];
-  uint32_t tile_id;
+  uint32_t tile_id;  // TICKET
 };
 
-template <class K, int THREADS, int KPT, bool HAS_VALS, int MINB, int LBW, int RANK, bool L2H = false>
+template <class K, int THREADS, int KPT, bool HAS_VALS, int MINB, int LBW, int RANK, bool L2H = false,
+          bool TICKET = false>
 __global__ void __launch_bounds__(THREADS, MINB) onesweep_kernel(const K* __restrict__ kin, const uint32_t* __restrict__ vin,
                                                            K* __restrict__ kout, uint32_t* __restrict__ vout,
                                                            uint32_t n, int shift, uint32_t dmask,
@@ -513,32 +518,25 @@ __global__ void __launch_bounds__(THREADS, MINB) onesweep_kernel(const K* __rest
   const int lane = tid & 31;
   const int warp = tid >> 5;
 
-  for (int i = tid; i < WARPS * RADIX; i += THREADS) (&s.warp_hist[0][0])[i] = 0;
-  // RANK 2: three rotating per-warp arrays of digit peer masks live in the
-  // key/value staging space, which is free until the scatter; zeroed here.
-  constexpr int MATCH_WORDS = 3 * WARPS * RADIX;
-  if constexpr (RANK == 2) {
-    static_assert(sizeof(s.keys) + sizeof(s.vals) >= MATCH_WORDS * 4, "peer masks fit in the staging space");
-    static_assert(offsetof(S, vals) == sizeof(s.keys), "keys and values are contiguous");
-    uint4* m4 = reinterpret_cast<uint4*>(s.keys);
-    for (int i = tid; i < MATCH_WORDS / 4; i += THREADS) m4[i] = make_uint4(0, 0, 0, 0);
-  }
-  if (tid == 0) s.tile_id = atomicAdd(tile_counter, 1u);
-  // Blocks start in about index order, so the ticket is usually close to
-  // this block's index: warm L2 with that tile while the ticket is in flight
-  // (a hint only; the tile actually processed is the ticket's).
-  {
+  uint32_t tile = blockIdx.x;
+  uint32_t skip = 0;
+  if (TICKET) {
+    if (tid == 0) s.tile_id = atomicAdd(tile_counter, 1u);
+    // The ticket is usually close to this block's index: warm L2 with that
+    // tile while it is in flight (a hint only).
     const uint32_t guess = blockIdx.x * TILE;
     constexpr uint32_t KL = 128 / sizeof(K), VL = 32;  // elements per 128-byte line
     for (uint32_t e = guess + tid * KL; e < guess + TILE && e < n; e += THREADS * KL) prefetch_l2(kin + e);
     if (HAS_VALS && vin)
       for (uint32_t e = guess + tid * VL; e < guess + TILE && e < n; e += THREADS * VL) prefetch_l2(vin + e);
+    __syncthreads();
+    tile = s.tile_id;
+    // Tickets start at 0 but for gtc_debug_skip_first_tile: one past the last
+    // tile has nothing to sort.
+    if (tile >= (n + TILE - 1) / TILE) return;
+  } else {
+    skip = *tile_counter;  // nobody advances it here; needed only after the ranks
   }
-  __syncthreads();
-  const uint32_t tile = s.tile_id;
-  // A ticket past the last tile has nothing to sort (tickets start at 0, so
-  // only a counter advanced on purpose, gtc_debug_skip_first_tile, gets here).
-  if (tile >= (n + TILE - 1) / TILE) return;
   const uint32_t tile_base = tile * TILE;
 
   // 2. warp-striped coalesced loads.
@@ -568,6 +566,22 @@ __global__ void __launch_bounds__(THREADS, MINB) onesweep_kernel(const K* __rest
 
   const uint32_t lt_mask = (1u << lane) - 1u;
   uint32_t* my_hist = s.warp_hist[warp];
+  // Every warp clears its own counters while its keys arrive.
+#pragma unroll
+  for (int i = 0; i < RADIX / 32; ++i) my_hist[i * 32 + lane] = 0;
+  // RANK 2: three rotating per-warp arrays of digit peer masks live in the
+  // key/value staging space, which is free until the scatter; zeroed here.
+  constexpr int MATCH_WORDS = 3 * WARPS * RADIX;
+  if constexpr (RANK == 2) {
+    static_assert(sizeof(s.keys) + sizeof(s.vals) >= MATCH_WORDS * 4, "peer masks fit in the staging space");
+    static_assert(offsetof(S, vals) == sizeof(s.keys), "keys and values are contiguous");
+    uint32_t* mbase = reinterpret_cast<uint32_t*>(s.keys) + warp * RADIX;
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+#pragma unroll
+      for (int i = 0; i < RADIX / 32; ++i) mbase[a * (WARPS * RADIX) + i * 32 + lane] = 0;
+  }
+  __syncwarp();
   uint32_t rank[KPT];  // RANK 1, 2: rank within the warp's digit run | digit << 16
   if (RANK == 0) {
     // 3. early per-warp digit counts: one shared atomic per key (one per warp
@@ -626,6 +640,7 @@ __global__ void __launch_bounds__(THREADS, MINB) onesweep_kernel(const K* __rest
     }
   }
   __syncthreads();
+  if (tile < skip) return;  // gtc_debug_skip_first_tile: tile 0 is never sorted or published
 
   // 4. per-digit counts across warps; publish the tile aggregate; turn the
   // per-warp counts into tile-local start positions.
@@ -706,12 +721,10 @@ __global__ void __launch_bounds__(THREADS, MINB) onesweep_kernel(const K* __rest
 // ------------------------------------------------- one-wave onesweep ------
 // The same pass for inputs whose tiles are all resident at once: a pass is
 // then one chain of dependent steps, and the chain is what it costs.  Against
-// onesweep_kernel: no ticket (block b takes tile b; it waits only on lower
-// blocks, all resident), keys requested at once, warp counters cleared by
-// their own warp, short tiles (4 or 8 keys per thread: fewer ranking steps in
+// onesweep_kernel: short tiles (4 or 8 keys per thread: fewer ranking steps in
 // a row, more SMs), and a look-back over 32 descriptors per round trip, since
 // the tiles publish at about the same time.  Whole sorts of uniform pairs,
-// histogram included (us; before: 256 x 16 tiles by ticket):
+// histogram included (us; before: 256 x 16 tiles):
 //   pairs      u32 before   4 keys   8 keys    u64 before   4 keys   8 keys
 //   16,384        28.3       18.5     20.5        56.4       34.0     37.5
 //   65,536        32.0       24.4     26.5        61.9       43.9     47.4
@@ -1050,28 +1063,30 @@ int sort_select_variant(int key_bits, int bits, uint32_t n) {
   if (t >= 0 && t < kNumVariants) return t;
   // Untuned: the one-wave tiles while the look-back stays short (crossings
   // measured: 4 against 8 keys per thread at about 100,000 keys, 8 against
-  // the ticketed tiles at about 250,000; onesweep_wave_kernel has the times).
+  // the large tiles at about 250,000; onesweep_wave_kernel has the times).
   if (n <= WAVE_4_USE) return WAVE_4;
   if (n <= WAVE_8_USE) return WAVE_8;
   // Above, by how the tiles fill waves (resident tiles on 152 SMs: 304 of
-  // 6,144 keys, 456 of 4,608, 608 of 4,096 with variant 7, whose 64 registers
-  // only 32-bit keys fit without spilling).  Sort of uniform pairs (us):
-  //                  u32: var. 2  var. 9  var. 7    u64: var. 2  var. 9
-  //   1,048,576           63.8     70.5     71.7         123.7    141.1
-  //   2,000,000           85.7     77.4     83.3         177.5    157.1
-  //   4,000,000          132.4    128.3    128.4         280.6    274.5
-  //   16,777,216         433.2    424.4    412.9         942.7    972.0
-  if (n <= 1860000) return 2;
-  if (n <= (w ? 4200000u : 6000000u)) return 9;
-  return w ? 2 : 7;
+  // 6,144 keys, 456 of 4,608 or 4,096, 608 of 4,096 with variant 7, whose 64
+  // registers only 32-bit keys fit without spilling).  Sort of uniform pairs
+  // with the caller's copies in (us):
+  //          u32: var. 0  var. 9  var. 7    u64: var. 2  var. 0  var. 9  var. 14
+  //   1.05M         63.9    68.4    69.3         123.7   116.0   134.1    116.0
+  //   2.0M          83.4    76.6    80.8         177.5   162.0   151.2    162.4
+  //   4.0M         126.7   122.3   124.3         280.6   261.5   263.5    260.5
+  //   8.0M         223.6   217.5   213.0         485.3   475.9   504.1    460.3
+  //   16.8M        431.4   420.8   405.1         942.7   950.7  1027.1    943.2
+  //   33.6M        831.7   810.0   775.4        1809.1  1841.6  2002.2   1850.3
+  if (w) return n <= 1860000 ? 0 : n <= 2100000 ? 9 : n <= 20000000 ? 14 : 2;
+  return n <= 1860000 ? 0 : n <= 6000000 ? 9 : 7;
 }
 
-template <class K, int THREADS, int KPT, bool HV, int MINB, int RANK, bool L2H = false>
+template <class K, int THREADS, int KPT, bool HV, int MINB, int RANK, bool L2H = false, bool TICKET = false>
 static cudaError_t launch_one(const Launch& L, const K* kin, const uint32_t* vin, K* kout, uint32_t* vout,
                               uint32_t n, int shift, uint32_t dmask, const uint32_t* bin_off, uint32_t* desc,
                               uint32_t* tile_counter) {
   using S = OnesweepSmem<K, THREADS, KPT>;
-  auto kern = onesweep_kernel<K, THREADS, KPT, HV, MINB, 8, RANK, L2H>;
+  auto kern = onesweep_kernel<K, THREADS, KPT, HV, MINB, 8, RANK, L2H, TICKET>;
   cudaError_t e = kernel_setup(kern, THREADS, sizeof(S));
   if (e != cudaSuccess) return e;
   const uint32_t tiles = ceil_div(n, S::TILE);
@@ -1135,13 +1150,16 @@ static cudaError_t launch_variant(int v, bool hv, const Launch& L, const K* kin,
 #define GTC_OSH(T, P, MB, RK)                                                                                  \
   return hv ? launch_one<K, T, P, true, MB, RK, true>(L, kin, vin, kout, vout, n, shift, dmask, bin_off, desc, tc) \
             : launch_one<K, T, P, false, MB, RK, true>(L, kin, vin, kout, vout, n, shift, dmask, bin_off, desc, tc)
+#define GTC_OST(T, P, MB, RK)                                                                                  \
+  return hv ? launch_one<K, T, P, true, MB, RK, false, true>(L, kin, vin, kout, vout, n, shift, dmask, bin_off, desc, tc) \
+            : launch_one<K, T, P, false, MB, RK, false, true>(L, kin, vin, kout, vout, n, shift, dmask, bin_off, desc, tc)
 #define GTC_TMA(T, P, M)                                                                                     \
   return hv ? launch_tma<K, T, P, true, M>(L, kin, vin, kout, vout, n, shift, dmask, bin_off, desc, tc)    \
             : launch_tma<K, T, P, false, M>(L, kin, vin, kout, vout, n, shift, dmask, bin_off, desc, tc)
   switch (v) {
     case 0: GTC_OS(256, 16, 3, 0);
     case 1: GTC_OS(384, 16, 2, 0);
-    case 2: GTC_OS(512, 12, 2, 0);
+    case 2: GTC_OST(512, 12, 2, 0);
     case 3: GTC_TMA(256, 16, true);
     case 4: GTC_TMA(256, 16, false);
     case 5: GTC_TMA(512, 8, false);
@@ -1161,6 +1179,7 @@ static cudaError_t launch_variant(int v, bool hv, const Launch& L, const K* kin,
   }
 #undef GTC_OS
 #undef GTC_OSH
+#undef GTC_OST
 #undef GTC_TMA
 }
 
