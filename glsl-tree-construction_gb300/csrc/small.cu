@@ -40,7 +40,7 @@ struct SbSmem {
   static constexpr int WARPS = THREADS / 32;
   static constexpr int MAX = MAX_;
   static constexpr int KPT = MAX / THREADS;  // items per thread of the largest cloud
-  using Shape = TwShape<MAX, 512>;
+  using Shape = TwShape<MAX, 512, 1>;
   static_assert(THREADS % 256 == 0 && MAX % THREADS == 0, "whole digits and items per thread");
   static_assert(MAX <= 1 << 13, "a child's index and two flags fit 16 bits");
   K keys[MAX];

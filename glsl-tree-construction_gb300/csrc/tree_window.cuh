@@ -58,8 +58,9 @@ constexpr int TW_LQ = 128;                 // long-range splits of a block (at m
 //   1,048,576    19.5              18.6             18.6             22.7
 //   4,000,000    56.9              46.9             44.4             49.4
 //   10,000,000  131.2             106.5             96.9            100.5
-template <int T_, int H_>
+template <int T_, int H_, int MINB_>
 struct TwShape {
+  static constexpr int MINB = MINB_;       // blocks per SM that the registers are held to
   static constexpr int T = T_;
   static constexpr int H = H_;
   static constexpr int W = T + 2 * H;      // window positions
@@ -69,10 +70,24 @@ struct TwShape {
   static_assert(T <= TW_THREADS * TW_C, "one in-chunk pass per lane");
   static_assert(NWB <= 32, "one ballot covers the window's warp-blocks");
 };
-using TwSmall = TwShape<1024, 512>;
-using TwLarge = TwShape<4096, 512>;
-using TwSegLarge = TwShape<8192, 1024>;     // batches, where each block also finds its clouds: a build of 83.5M points takes 4.68 ms, 4.73 with TwLarge
-constexpr uint32_t TW_SMALL_MAX = 700000;  // splits up to which TwSmall is the faster shape (table above)
+using TwSmall = TwShape<1024, 512, 3>;
+using TwSmall4 = TwShape<1024, 512, 4>;
+using TwMid = TwShape<4096, 512, 2>;
+using TwMid3 = TwShape<4096, 512, 3>;
+using TwLarge = TwShape<4096, 512, 4>;
+using TwSegLarge = TwShape<8192, 1024, 4>;     // batches, where each block also finds its clouds: a build of 83.5M points takes 4.68 ms, 4.73 with TwLarge
+// Splits up to which each shape is used.  Registers: the longer a block's
+// chain counts, the more its threads may have; TwMid takes 64 while at most
+// two blocks per SM run anyway, TwSmall and TwMid3 40, the others 32.
+// Builds with 32-bit codes (us):
+//   points       1024, 3 per SM   1024, 4   4096, 2   4096, 3   4096, 4
+//   400,000           82.3          83.7
+//   600,000           94.2          92.0       95.0
+//   700,000           98.8          96.3       95.9
+//   1,048,576            -             -     110.7     115.1     119.0
+//   1,700,000            -             -     146.0     140.1     145.8
+//   10M, 64-bit          -             -         -     725       712
+constexpr uint32_t TW_SMALL_MAX = 450000, TW_SMALL4_MAX = 700000, TW_MID_MAX = 1240000, TW_MID3_MAX = 1860000;
 
 // First index in a[0..n) with a[i] > x.
 __device__ __forceinline__ uint32_t upper_bound_u32(const uint32_t* a, uint32_t n, uint32_t x) {
@@ -407,7 +422,7 @@ __device__ __forceinline__ void tw_warp_split(const K* codes, uint32_t x, uint32
 // slot of every cloud gets edge 0.  Otherwise one cloud of U codes.  rec
 // (nullable) receives every split's record (split_rec.cuh).
 template <class K, bool SEG, class SH>
-__global__ void __launch_bounds__(TW_THREADS, 4) radix_tree_window_kernel(
+__global__ void __launch_bounds__(TW_THREADS, SH::MINB) radix_tree_window_kernel(
     const K* __restrict__ codes, const uint32_t* d_u, uint32_t u_host, const uint32_t* uoff, uint32_t S,
     uint8_t* __restrict__ prefix_n, uint8_t* __restrict__ hll, uint8_t* __restrict__ hlr,
     int32_t* __restrict__ left, int32_t* __restrict__ parent, uint32_t* __restrict__ edge, uint32_t* d_m,

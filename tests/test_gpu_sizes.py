@@ -19,7 +19,8 @@ def unique_codes(oracle, n, key_bits, seed):
 
 
 @pytest.mark.parametrize("key_bits", [32, 64])
-@pytest.mark.parametrize("u", [2, 1023, 1024, 1025, 1026, 2049, 4096, 4097, 9000, 700_000, 700_001, 700_002, 708_609])
+@pytest.mark.parametrize("u", [2, 1023, 1024, 1025, 1026, 2049, 4096, 4097, 9000, 450_001, 450_002, 700_001, 700_002,
+                               708_609, 1_240_001, 1_240_002, 1_860_001, 1_860_002])
 def test_tree_window_shapes(ctx, gtc_mod, oracle, key_bits, u):
     """u codes (u - 1 splits) at the tile edges and on both sides of the shape
     rule: the window method against the per-node search."""
@@ -228,7 +229,7 @@ def _spread_clouds(total, seed):
     return clouds
 
 
-@pytest.mark.parametrize("total,variant", [(599_999, -1), (600_000, 5), (600_001, 5), (600_001, -1), (1_999_999, -1),
+@pytest.mark.parametrize("total,variant", [(599_999, -1), (600_000, 5), (600_001, 5), (600_001, -1), (700_001, -1), (1_240_001, -1), (1_999_999, -1),
                                            (2_000_000, -1), (2_700_001, 6), (13_001, 6), (13_001, -1)])
 def test_batched_sizes(ctx, gtc_mod, oracle, total, variant):
     """Both sides of every size rule of the batch (tile shape, tree window,
