@@ -157,7 +157,7 @@ class Context:
     def unique(self, keys, vals=None, ws=None):
         """In-place unique; returns the device count tensor (1 element)."""
         torch = _torch()
-        cnt = torch.zeros(1, dtype=torch.int32, device=keys.device)
+        cnt = torch.empty(1, dtype=torch.int32, device=keys.device)  # always written
         fn = self.L.gtc_unique_u32 if keys.element_size() == 4 else self.L.gtc_unique_u64
         self.check(fn(self.h, _ptr(keys), _ptr(vals), keys.numel(), _ptr(cnt), _ptr(ws),
                       0 if ws is None else ws.numel(), _stream()))
@@ -167,13 +167,12 @@ class Context:
         torch = _torch()
         m = n_brt_nodes
         dev = codes.device
-        out = dict(prefix_n=torch.zeros(max(m, 1), dtype=torch.uint8, device=dev),
-                   has_leaf_left=torch.zeros(max(m, 1), dtype=torch.uint8, device=dev),
-                   has_leaf_right=torch.zeros(max(m, 1), dtype=torch.uint8, device=dev),
-                   left_child=torch.zeros(max(m, 1), dtype=torch.int32, device=dev),
-                   parent=torch.zeros(max(m, 1), dtype=torch.int32, device=dev))
+        # Every entry is written by the kernel: no fill in front of it.
+        out = {k: torch.empty(max(m, 1), dtype=dt, device=dev)
+               for k, dt in (("prefix_n", torch.uint8), ("has_leaf_left", torch.uint8),
+                             ("has_leaf_right", torch.uint8), ("left_child", torch.int32), ("parent", torch.int32))}
         if with_edge:
-            out["edge_count"] = torch.zeros(max(m, 1), dtype=torch.int32, device=dev)
+            out["edge_count"] = torch.empty(max(m, 1), dtype=torch.int32, device=dev)
         fn = self.L.gtc_build_radix_tree_u32 if codes.element_size() == 4 else self.L.gtc_build_radix_tree_u64
         self.check(fn(self.h, _ptr(codes), m, _ptr(out["prefix_n"]), _ptr(out["has_leaf_left"]),
                       _ptr(out["has_leaf_right"]), _ptr(out["left_child"]), _ptr(out["parent"]),
@@ -183,21 +182,21 @@ class Context:
     def edge_count(self, prefix_n, parent, key_bits: int):
         torch = _torch()
         m = prefix_n.numel()
-        edge = torch.zeros(max(m, 1), dtype=torch.int32, device=prefix_n.device)
+        edge = torch.empty(max(m, 1), dtype=torch.int32, device=prefix_n.device)
         self.check(self.L.gtc_edge_count(self.h, _ptr(prefix_n), _ptr(parent), _ptr(edge), m, key_bits, _stream()))
         return edge[:m]
 
     def partial_sum(self, data, first: int, last: int, ws=None):
         torch = _torch()
-        out = torch.zeros(max(last - first, 1), dtype=torch.int32, device=data.device)
+        out = torch.empty(max(last - first, 1), dtype=torch.int32, device=data.device)
         self.check(self.L.gtc_partial_sum_u32(self.h, _ptr(data), first, last, _ptr(out), _ptr(ws),
                                               0 if ws is None else ws.numel(), _stream()))
         return out[: last - first]
 
     def node_offsets(self, edge, n_brt_nodes: int, ws=None):
         torch = _torch()
-        ps = torch.zeros(n_brt_nodes + 1, dtype=torch.int32, device=edge.device)
-        o = torch.zeros(1, dtype=torch.int32, device=edge.device)
+        ps = torch.empty(n_brt_nodes + 1, dtype=torch.int32, device=edge.device)
+        o = torch.empty(1, dtype=torch.int32, device=edge.device)
         self.check(self.L.gtc_node_offsets(self.h, _ptr(edge), n_brt_nodes, _ptr(ps), _ptr(o), _ptr(ws),
                                            0 if ws is None else ws.numel(), _stream()))
         return ps, o
