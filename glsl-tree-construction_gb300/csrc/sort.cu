@@ -724,12 +724,19 @@ __global__ void __launch_bounds__(THREADS, MINB) onesweep_kernel(const K* __rest
 // onesweep_kernel: short tiles (4 or 8 keys per thread: fewer ranking steps in
 // a row, more SMs), and a look-back over 32 descriptors per round trip, since
 // the tiles publish at about the same time.  Whole sorts of uniform pairs,
-// histogram included (us; before: 256 x 16 tiles):
-//   pairs      u32 before   4 keys   8 keys    u64 before   4 keys   8 keys
-//   16,384        28.3       18.5     20.5        56.4       34.0     37.5
-//   65,536        32.0       24.4     26.5        61.9       43.9     47.4
-//   120,000       33.6       32.9     29.9        65.0       59.4     53.4
-//   250,000       39.3         -      40.4        74.2         -      70.6
+// histogram included (us; beside them the 256 x 16 tiles of onesweep_kernel):
+//   pairs     u32: 256 x 16   4 keys   8 keys    u64: 256 x 16   4 keys   8 keys
+//   30,000          27.9       21.0     21.9           54.2       38.5     40.0
+//   65,536          30.4       24.7     26.7           58.4       44.1     47.6
+//   90,000          31.0       28.2     28.7           59.5       51.9     51.9
+//   110,000         31.8       30.9     28.9           61.7       56.8     52.3
+//   180,000         33.1         -      32.4           64.3         -      58.8
+//   220,000         34.5         -      36.0           66.3         -      65.2
+//   260,000         37.8         -      40.6           70.6         -      71.1
+// (16 keys per thread were never the fastest.  Clusters of eight blocks that
+// add up their counts through distributed shared memory and look back once
+// per cluster: 24.0 us for 65,536 u32 pairs, but 19.5 against 16.6 for 4,097
+// and 64.9 against 52.6 for 1M, by this kernel and onesweep_kernel.)
 // first_tile: 1 leaves tile 0 unsorted (gtc_debug_skip_first_tile).
 template <class K, int THREADS, int KPT, bool HAS_VALS>
 __global__ void __launch_bounds__(THREADS) onesweep_wave_kernel(const K* __restrict__ kin,
@@ -1040,7 +1047,7 @@ constexpr Variant kVariants[] = {{256, 16, 0, 3, 0}, {384, 16, 0, 2, 0}, {512, 1
                                  {512, 8, 0, 2, 0},  {384, 12, 0, 3, 0}, {256, 16, 0, 3, 1}, {384, 16, 0, 2, 1},
                                  {512, 12, 0, 2, 1}, {256, 24, 0, 2, 1}, {256, 16, 4, 3, 0}, {512, 12, 4, 2, 1},
                                  {256, 16, 4, 3, 2}, {512, 12, 4, 2, 2}, {384, 16, 4, 2, 2}, {256, 4, 5, 1, 1},
-                                 {256, 8, 5, 1, 1},  {256, 16, 5, 1, 1}};
+                                 {256, 8, 5, 1, 1}};
 constexpr int kNumVariants = sizeof(kVariants) / sizeof(kVariants[0]);
 static const int g_variant[2] = {0, 2};  // [u32, u64]: what gtc_sort_get_variant reports with nothing pinned
 static std::atomic<int> g_pinned[2] = {{-1}, {-1}};  // gtc_sort_set_variant: overrides the tuned choice
@@ -1048,11 +1055,11 @@ static std::atomic<int> g_pinned[2] = {{-1}, {-1}};  // gtc_sort_set_variant: ov
 // Largest inputs of the one-wave variants (kind 5).  The short tiles' limits
 // bound the look-back descriptors of the workspace (one row of 256 words per
 // tile and pass); every one-wave launch also needs its tiles resident.
-constexpr int WAVE_4 = 19, WAVE_8 = 20, WAVE_16 = 21;  // their places in kVariants
+constexpr int WAVE_4 = 19, WAVE_8 = 20;  // their places in kVariants
 constexpr uint32_t WAVE_4_MAX = 160 * 1024, WAVE_8_MAX = 200 * 2048;
-constexpr uint32_t WAVE_4_USE = 96 * 1024, WAVE_8_USE = 250000;  // without a tuned or pinned choice
+constexpr uint32_t WAVE_4_USE = 92000, WAVE_8_USE[2] = {185000, 225000};  // untuned, [u32, u64]
 static_assert(kVariants[WAVE_4].kind == 5 && kVariants[WAVE_4].kpt == 4 && kVariants[WAVE_8].kpt == 8 &&
-                  kVariants[WAVE_16].kpt == 16 && kNumVariants == 22,
+                  kNumVariants == 21,
               "variant numbers");
 
 int sort_select_variant(int key_bits, int bits, uint32_t n) {
@@ -1061,11 +1068,10 @@ int sort_select_variant(int key_bits, int bits, uint32_t n) {
   if (pinned >= 0) return pinned;
   const int t = tuned_variant(key_bits, bits, n);
   if (t >= 0 && t < kNumVariants) return t;
-  // Untuned: the one-wave tiles while the look-back stays short (crossings
-  // measured: 4 against 8 keys per thread at about 100,000 keys, 8 against
-  // the large tiles at about 250,000; onesweep_wave_kernel has the times).
+  // Untuned: the one-wave tiles while the look-back stays short
+  // (onesweep_wave_kernel has the times around the crossings).
   if (n <= WAVE_4_USE) return WAVE_4;
-  if (n <= WAVE_8_USE) return WAVE_8;
+  if (n <= WAVE_8_USE[w]) return WAVE_8;
   // Above, by how the tiles fill waves (resident tiles on 152 SMs: 304 of
   // 6,144 keys, 456 of 4,608 or 4,096, 608 of 4,096 with variant 7, whose 64
   // registers only 32-bit keys fit without spilling).  Sort of uniform pairs
@@ -1139,7 +1145,7 @@ static cudaError_t launch_variant(int v, bool hv, const Launch& L, const K* kin,
 #define GTC_WV(P)                                                                                              \
   (hv ? launch_wave<K, 256, P, true>(L, kin, vin, kout, vout, n, shift, dmask, bin_off, desc, tc, &e)      \
       : launch_wave<K, 256, P, false>(L, kin, vin, kout, vout, n, shift, dmask, bin_off, desc, tc, &e))
-    const bool done = v == WAVE_4 ? n <= WAVE_4_MAX && GTC_WV(4) : v == WAVE_8 ? n <= WAVE_8_MAX && GTC_WV(8) : GTC_WV(16);
+    const bool done = v == WAVE_4 ? n <= WAVE_4_MAX && GTC_WV(4) : n <= WAVE_8_MAX && GTC_WV(8);
 #undef GTC_WV
     if (done) return e;
     v = 0;
