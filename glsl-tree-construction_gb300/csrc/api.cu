@@ -245,6 +245,12 @@ gtc_status sort_pairs_impl(gtc_ctx* ctx, K* keys, uint32_t* vals, K* keys_alt, u
   gtc_status st = resolve_ws(ctx, ws, ws_bytes, sort_workspace_bytes(n, passes, 0));
   if (st != GTC_OK) return st;
   const Launch L = launch_of(ctx, stream);
+  // Few keys: one block sorts them (small.cu).  Stage events, pinned variants
+  // and the first-tile switch are about the passes.
+  if (n <= SMALL_SORT_MAX && !ctx->profiling && !ctx->skip_first_tile && !sort_pinned(W)) {
+    GTC_TRY(ctx, launch_small_sort<K>(L, keys, vals, n, begin_bit, end_bit));
+    return GTC_OK;
+  }
   Launch Lp = L;  // the passes: programmatic dependent launches (not with stage events between them)
   Lp.pdl = !ctx->profiling;
   const SortWorkspace Wk = carve_sort_workspace(ws, n, passes, 0);

@@ -597,6 +597,13 @@ constexpr uint32_t SMALL_BUILD_MAX = 4096;
 template <class K>
 cudaError_t launch_small_build(const Launch& L, const float4* pts, uint32_t n, float mn, float rg,
                                const gtc_octree_buffers& out);
+// The stable sort of at most SMALL_SORT_MAX pairs (vals nullable) in place by
+// one block (small.cu), no workspace.
+constexpr uint32_t SMALL_SORT_MAX = 4096;
+template <class K>
+cudaError_t launch_small_sort(const Launch& L, K* keys, uint32_t* vals, uint32_t n, int begin_bit, int end_bit);
+// A variant or digit width is pinned for that key width (sort.cu).
+bool sort_pinned(int key_bits);
 
 inline uint32_t ceil_div(uint64_t a, uint64_t b) { return (uint32_t)((a + b - 1) / b); }
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }

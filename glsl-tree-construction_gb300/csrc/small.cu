@@ -1,4 +1,5 @@
-// small.cu - the whole build of a small cloud in one block.
+// small.cu - the whole build of a small cloud, and the whole sort of few keys,
+// in one block.
 //
 // The stage kernels (morton.comp .. octree.comp, main.rs:60-170) each cost a
 // launch and a chain of dependent global round trips however few points there
@@ -90,7 +91,7 @@ __device__ __forceinline__ uint32_t sb_scan(uint32_t v, uint32_t (*wsum)[WARPS],
 // holds keys [32 w kpt, 32 (w + 1) kpt) in rows of 32, so that rank order is
 // position order).  Starts and ends with every thread past a barrier.
 template <class S, class K>
-__device__ __forceinline__ void sb_pass(S& s, int kpt, int shift, K*) {
+__device__ __forceinline__ void sb_pass(S& s, int kpt, int shift, K*, uint32_t dmask = 255u) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t lt = (1u << lane) - 1u;
   uint32_t* my = s.hist[warp];
@@ -111,7 +112,7 @@ __device__ __forceinline__ void sb_pass(S& s, int kpt, int shift, K*) {
 #pragma unroll
   for (int j = 0; j < S::KPT; ++j) {
     if (j < kpt) {  // block-uniform
-      const uint32_t d = (uint32_t)(key[j] >> shift) & 255u;
+      const uint32_t d = (uint32_t)(key[j] >> shift) & dmask;
       const uint32_t peers = warp_peers<8>(d);
       const int leader = 31 - __clz(peers);
       uint32_t b = 0;
@@ -440,6 +441,74 @@ __global__ void __launch_bounds__(THREADS, 1) small_build_kernel(const float4* _
     }
   }
 }
+
+// ------------------------------------------------------- sort of few keys --
+// The sort API's whole sort of at most SMALL_SORT_MAX keys in one launch of
+// one block: the build's passes over bits [begin_bit, end_bit) on positions,
+// then the values by position.  (The passes of sort.cu are a memset, a
+// histogram and a launch per digit.)  Back to back, uniform pairs (us):
+//   pairs    u32: passes  one block    u64: passes  one block
+//   100           38.0        7.9           66.7        7.7
+//   512           33.9        7.6           74.8        8.3
+//   1,024         34.7        8.1           74.9       14.4
+//   4,096         42.2       14.4           76.9       25.6
+// (The passes as they were before the one-wave kernel; they take 21.5 and 34.8
+// at 4,097 now.)
+template <class K, int THREADS_, int MAX_>
+struct SsSmem {
+  static constexpr int THREADS = THREADS_;
+  static constexpr int WARPS = THREADS / 32;
+  static constexpr int KPT = MAX_ / THREADS;
+  K keys[MAX_];
+  uint32_t vals[MAX_];
+  uint32_t hist[WARPS][SB_HROW];
+  uint16_t idx[MAX_];
+  uint32_t wsum[2][WARPS];
+};
+
+template <class K, int THREADS, int MAX>
+__global__ void __launch_bounds__(THREADS, 1) small_sort_kernel(K* keys, uint32_t* vals, uint32_t n, int begin_bit,
+                                                                int end_bit) {
+  using S = SsSmem<K, THREADS, MAX>;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  S& s = *reinterpret_cast<S*>(smem_raw);
+  K* const tag = nullptr;
+  const int tid = threadIdx.x;
+  const int kpt = (int)((n + THREADS - 1) / THREADS);
+#pragma unroll
+  for (int j = 0; j < S::KPT; ++j) {
+    const int i = j * THREADS + tid;
+    if (j < kpt) {
+      s.keys[i] = i < (int)n ? keys[i] : ~K(0);  // padding sorts last: it starts last and has the largest digits
+      s.vals[i] = vals && i < (int)n ? vals[i] : 0u;
+      s.idx[i] = (uint16_t)i;
+    }
+  }
+  __syncthreads();
+  for (int sh = begin_bit; sh < end_bit; sh += 8)
+    sb_pass(s, kpt, sh, tag, end_bit - sh < 8 ? (1u << (end_bit - sh)) - 1u : 255u);
+#pragma unroll
+  for (int j = 0; j < S::KPT; ++j) {
+    const int i = j * THREADS + tid;
+    if (i < (int)n) {
+      keys[i] = s.keys[i];
+      if (vals) vals[i] = s.vals[s.idx[i]];
+    }
+  }
+}
+
+template <class K>
+cudaError_t launch_small_sort(const Launch& L, K* keys, uint32_t* vals, uint32_t n, int begin_bit, int end_bit) {
+  if (n == 0 || n > SMALL_SORT_MAX) return cudaErrorInvalidValue;
+  auto run = [&](auto kern, int threads, size_t smem) {
+    cudaError_t e = kernel_setup(kern, threads, smem);
+    return e != cudaSuccess ? e : launch_kernel(L, kern, 1, threads, smem, keys, vals, n, begin_bit, end_bit);
+  };
+  if (n <= 512) return run(small_sort_kernel<K, 256, 512>, 256, sizeof(SsSmem<K, 256, 512>));
+  return run(small_sort_kernel<K, 1024, (int)SMALL_SORT_MAX>, 1024, sizeof(SsSmem<K, 1024, (int)SMALL_SORT_MAX>));
+}
+template cudaError_t launch_small_sort<uint32_t>(const Launch&, uint32_t*, uint32_t*, uint32_t, int, int);
+template cudaError_t launch_small_sort<uint64_t>(const Launch&, uint64_t*, uint32_t*, uint32_t, int, int);
 
 template <class K, int THREADS, int MAX>
 static cudaError_t launch_small(const Launch& L, const float4* pts, uint32_t n, float mn, float rg,

@@ -1330,6 +1330,11 @@ bool sort_set_digit_bits(int key_bits, int db) {
   return true;
 }
 
+bool sort_pinned(int key_bits) {
+  const int w = key_bits == 64;
+  return g_pinned[w].load(std::memory_order_relaxed) >= 0 || g_pinned_db[w].load(std::memory_order_relaxed) > 0;
+}
+
 int sort_max_passes() { return MAX_PASSES; }
 
 int sort_num_variants() { return kNumVariants; }

@@ -321,3 +321,41 @@ def test_octree_window_tiles(ctx, gtc_mod, oracle, key_bits, n):
     got = gtc_mod.nodes_to_numpy(short.nodes)
     same = (got.view(np.int32).reshape(-1, 16) == exp["nodes"][:-1].view(np.int32).reshape(-1, 16)).all(axis=1)
     assert same.sum() >= same.size - 21  # only nodes that share an owner with the one that did not fit
+
+
+@pytest.mark.parametrize("key_bits", [32, 64])
+@pytest.mark.parametrize("n", [1, 2, 31, 33, 255, 511, 512, 513, 1023, 1025, 3073, 4095, 4096, 4097])
+def test_one_block_sort(ctx, key_bits, n):
+    """One block up to 4,096 keys, the passes above: any bit range, with and
+    without values, aligned and not, under capture."""
+    import torch
+
+    kd, td = (np.uint32, np.int32) if key_bits == 32 else (np.uint64, np.int64)
+    for words, lo, hi in ((0, 0, key_bits), (2, 0, key_bits - 2), (0, 5, 9), (4, 0, 1), (1, key_bits - 17, key_bits)):
+        keys = W.config3_keys(n + 1, key_bits, and_words=words, seed=n + words)
+        keys[-1] = keys[0]
+        for off in (0, 1):
+            want = keys[off:off + n]
+            order = np.argsort((want >> kd(lo)) & kd((1 << (hi - lo)) - 1), kind="stable")
+            k = torch.from_numpy(keys.view(td).copy()).cuda()[off:off + n]
+            v = torch.arange(n + 1, dtype=torch.int32, device="cuda")[off:off + n]
+            ctx.sort_pairs(k, v, lo, hi)
+            assert np.array_equal(k.contiguous().cpu().numpy().view(kd), want[order]), (lo, hi, off)
+            assert np.array_equal(v.contiguous().cpu().numpy(), order.astype(np.int32) + off), (lo, hi, off)
+            k = torch.from_numpy(keys.view(td).copy()).cuda()[off:off + n]
+            ctx.sort_pairs(k, None, lo, hi)
+            assert np.array_equal(k.contiguous().cpu().numpy().view(kd), want[order]), (lo, hi, off, "keys only")
+    src = torch.from_numpy(keys[:n].view(td).copy()).cuda()
+    k, alt, ws = src.clone(), torch.empty_like(src), ctx.workspace(1, n, key_bits)
+    ctx.sort_pairs(k, None, ws=ws, keys_alt=alt)
+    torch.cuda.synchronize()
+    g, s = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    with torch.cuda.stream(s):
+        g.capture_begin()
+        ctx.sort_pairs(k, None, ws=ws, keys_alt=alt)
+        g.capture_end()
+    k.copy_(src)
+    g.replay()
+    torch.cuda.synchronize()
+    assert np.array_equal(k.cpu().numpy().view(kd), np.sort(keys[:n]))
+    assert ctx.device_status() == 0
