@@ -34,11 +34,12 @@
 #include <cstdio>
 #include <new>
 
-#include "gtc_internal.cuh"
+#include "scan_dev.cuh"
 
 namespace gtc {
 
 Launch context_launch(gtc_ctx* ctx, gtc_stream_t stream);
+bool context_stage_idle(const gtc_ctx* ctx);
 gtc_status context_error(gtc_ctx* ctx, gtc_status s, const char* msg, cudaError_t e);
 
 constexpr uint32_t LFLAG_OVERFLOW = 1u;   // a bucket exceeds the on-chip sort capacity
@@ -222,6 +223,7 @@ constexpr int LP_RADIX = 128;      // bucket-id digits of at most 7 bits
 // knots in Eytzinger order for the count kernel's search, and the
 // monotonicity check of the heights.
 __global__ void learned_prepare_kernel(const uint64_t* kn, const float* y, int B, uint64_t* eytz, uint32_t* flags) {
+  griddep_wait();
   const int d = 31 - __clz(B);
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < B; i += gridDim.x * blockDim.x) {
     if (flags && !(y[i] <= y[i + 1])) atomicOr(flags, LFLAG_BAD_MODEL);
@@ -272,6 +274,7 @@ __global__ void __launch_bounds__(LC_THREADS, 1) learned_count_kernel(const uint
                                                                       const float* __restrict__ y, int B,
                                                                       uint32_t* totals, uint16_t* __restrict__ bids,
                                                                       uint32_t* flags) {
+  griddep_wait();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   uint32_t* s_hi = reinterpret_cast<uint32_t*>(smem_raw);
   uint32_t* s_lo = s_hi + B;
@@ -369,50 +372,62 @@ __global__ void __launch_bounds__(LC_THREADS, 1) learned_count_kernel(const uint
 
 // 2. one block: bucket bases, the capacity and model checks, and the digit
 // bases of the two passes (low db1 bits of the bucket id, then the rest).
+// The totals are staged in shared memory (one word of padding per 16, so that
+// a thread's run of 16 and its neighbours' fall in different banks): read from
+// global memory in order of use, this one block took 21.5 us for 2^14 buckets.
+__device__ __forceinline__ int ls_at(int i) { return i + (i >> 4); }
+static size_t scan_smem_bytes(int B) { return ((size_t)B + B / 16 + 1) * 4; }
+
 __global__ void __launch_bounds__(1024) learned_scan_kernel(const uint32_t* totals, int B, int db1, const float* y,
                                                             uint32_t* base, uint32_t* off1, uint32_t* off2,
                                                             uint32_t* flags) {
+  griddep_wait();
+  extern __shared__ uint32_t s_tot[];
   __shared__ uint32_t s_part[1024];
+  __shared__ uint32_t s_w[33];
   const int tid = threadIdx.x;
-  const int per = (B + 1023) / 1024;
-  const int first = tid * per, last = min(first + per, B);
-  uint32_t sum = 0;
   bool over = false, bad = false;
-  for (int i = first; i < last; ++i) {
+  for (int i = tid; i < B; i += 1024) {
     const uint32_t t = totals[i];
-    sum += t;
+    s_tot[ls_at(i)] = t;
     over |= t > (uint32_t)BS_CAP;
     bad |= y[i] > y[i + 1];
   }
   if (over) atomicOr(flags, LFLAG_OVERFLOW);
   if (bad) atomicOr(flags, LFLAG_BAD_MODEL);
-  s_part[tid] = sum;
   __syncthreads();
-  for (int o = 1; o < 1024; o <<= 1) {
-    const uint32_t t = (tid >= o) ? s_part[tid - o] : 0u;
-    __syncthreads();
-    s_part[tid] += t;
-    __syncthreads();
-  }
-  uint32_t run = tid > 0 ? s_part[tid - 1] : 0u;
-  for (int i = first; i < last; ++i) {
-    base[i] = run;
-    run += totals[i];
-  }
-  __syncthreads();
-  const int r1 = 1 << db1;
-  if (tid < r1) {
+  // Digit counts of the first pass (bucket id mod 2^db1): 1024 / 2^db1 threads
+  // per digit.
+  const int r1 = 1 << db1, parts = 1024 / r1;
+  {
     uint32_t c = 0;
-    for (int b = tid; b < B; b += r1) c += totals[b];
+    for (int b = tid; b < B; b += 1024) c += s_tot[ls_at(b)];  // b keeps its digit: r1 divides 1024
     s_part[tid] = c;
   }
   __syncthreads();
-  if (tid < r1) {
-    uint32_t pre = 0;
-    for (int d = 0; d < tid; ++d) pre += s_part[d];
-    off1[tid] = pre;
+  uint32_t total;
+  {
+    uint32_t c = 0;
+    if (tid < r1)
+      for (int q = 0; q < parts; ++q) c += s_part[q * r1 + tid];
+    const uint32_t pre = block_exclusive<1024>(c, s_w, &total);
+    if (tid < r1) off1[tid] = pre;
   }
-  if (tid < (B >> db1)) off2[tid] = base[tid << db1];
+  __syncthreads();
+  // Bucket bases.
+  const int per = (B + 1023) / 1024;
+  const int first = tid * per, last = min(first + per, B);
+  uint32_t sum = 0;
+  for (int i = first; i < last; ++i) sum += s_tot[ls_at(i)];
+  uint32_t run = block_exclusive<1024>(sum, s_w, &total);
+  for (int i = first; i < last; ++i) {
+    const uint32_t t = s_tot[ls_at(i)];
+    s_tot[ls_at(i)] = run;
+    run += t;
+  }
+  __syncthreads();
+  for (int i = tid; i < B; i += 1024) base[i] = s_tot[ls_at(i)];
+  if (tid < (B >> db1)) off2[tid] = s_tot[ls_at(tid << db1)];
 }
 
 // 3. one stable pass over the bucket-id digit (bid >> shift) & mask.  FIRST:
@@ -430,12 +445,13 @@ struct LpSmem {
   uint32_t warp_sums[LP_RADIX / 32];
 };
 
-template <bool FIRST, int THREADS, int KPT>
-__global__ void __launch_bounds__(THREADS) learned_pass_kernel(
+template <bool FIRST, int THREADS, int KPT, int MINB>
+__global__ void __launch_bounds__(THREADS, MINB) learned_pass_kernel(
     const uint64_t* __restrict__ kin, const uint32_t* __restrict__ vin, const uint16_t* __restrict__ bin,
     uint64_t* __restrict__ kout, uint32_t* __restrict__ vout, uint16_t* __restrict__ bout, uint32_t n, int shift,
     uint32_t mask, const uint32_t* __restrict__ bin_off, uint32_t* __restrict__ desc, uint32_t* status,
     const uint32_t* flags) {
+  griddep_wait();
   if (*flags & (LFLAG_OVERFLOW | LFLAG_BAD_MODEL)) return;
   using Sm = LpSmem<THREADS, KPT>;
   constexpr int WARPS = Sm::WARPS;
@@ -747,6 +763,7 @@ __global__ void __launch_bounds__(BS_THREADS, 2) bucket_sort_kernel(
     const uint64_t* __restrict__ ukeys, const uint32_t* __restrict__ uvals, const uint32_t* base,
     const uint32_t* totals, uint64_t* __restrict__ out_keys, uint32_t* __restrict__ out_vals, uint64_t* bmin,
     uint64_t* bmax, uint32_t* flags) {
+  griddep_wait();
   if (*flags & (LFLAG_OVERFLOW | LFLAG_BAD_MODEL)) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   BucketSmem& s = *reinterpret_cast<BucketSmem*>(smem_raw);
@@ -820,6 +837,7 @@ __global__ void __launch_bounds__(BS_THREADS, 2) bucket_sort_kernel(
 // Consecutive non-empty buckets must hold strictly increasing key ranges.
 __global__ void learned_order_check_kernel(const uint32_t* totals, const uint64_t* bmin, const uint64_t* bmax, int B,
                                            uint32_t* flags) {
+  griddep_wait();
   if (*flags) return;
   for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < B; b += gridDim.x * blockDim.x) {
     if (totals[b] == 0) continue;
@@ -832,6 +850,7 @@ __global__ void learned_order_check_kernel(const uint32_t* totals, const uint64_
 // Fallback preparation: with any flag set, copy the input to the output.
 __global__ void cond_copy_kernel(const uint64_t* keys, const uint32_t* vals, uint64_t* keys_out, uint32_t* vals_out,
                                  uint32_t n, const uint32_t* flags) {
+  griddep_wait();
   if (*flags == 0) return;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
     keys_out[i] = keys[i];
@@ -921,52 +940,57 @@ gtc_status cuda_fail(gtc_ctx* ctx, const char* what, cudaError_t e) {
 size_t count_smem_bytes(int B) { return (size_t)B * 14 + 4; }
 
 // Derives the sort-time model arrays from the knots and heights.
-gtc_status prepare_model(gtc_ctx* ctx, const gtc_learned_model* m, uint32_t* d_flags, cudaStream_t s) {
-  learned_prepare_kernel<<<ceil_div(m->B, 256), 256, 0, s>>>(m->knots, m->heights, m->B, m->eytz, d_flags);
-  LTRY(ctx, cudaGetLastError());
+gtc_status prepare_model(gtc_ctx* ctx, const Launch& L, const gtc_learned_model* m, uint32_t* d_flags) {
+  LTRY(ctx, launch_kernel(L, learned_prepare_kernel, ceil_div(m->B, 256), 256, 0, m->knots, m->heights, m->B, m->eytz,
+                          d_flags));
   return GTC_OK;
 }
 
 // The count kernel over the keys: one resident CTA per SM.
-gtc_status launch_count(gtc_ctx* ctx, const gtc_learned_model* m, const uint64_t* keys, uint32_t n, uint32_t* totals,
-                        uint16_t* bids, uint32_t* d_flags, cudaStream_t s) {
+gtc_status launch_count(gtc_ctx* ctx, const Launch& L, const gtc_learned_model* m, const uint64_t* keys, uint32_t n,
+                        uint32_t* totals, uint16_t* bids, uint32_t* d_flags) {
   const int B = m->B;
   LTRY(ctx, kernel_setup(learned_count_kernel, LC_THREADS, count_smem_bytes(MAX_BUCKETS)));
-  const Launch L = context_launch(ctx, reinterpret_cast<gtc_stream_t>(s));
   const uint32_t grid = max(1u, min((uint32_t)L.num_sms, ceil_div(n, LC_THREADS * LC_ILP)));
-  learned_count_kernel<<<grid, LC_THREADS, count_smem_bytes(B), s>>>(keys, n, m->eytz, m->knots, m->heights, B,
-                                                                     totals, bids, d_flags);
-  LTRY(ctx, cudaGetLastError());
+  LTRY(ctx, launch_kernel(L, learned_count_kernel, grid, LC_THREADS, count_smem_bytes(B), keys, n, m->eytz, m->knots,
+                          m->heights, B, totals, bids, d_flags));
   return GTC_OK;
 }
 
 // One grouping pass with the tile shape of variant v.
-template <bool FIRST, int THREADS, int KPT>
-cudaError_t launch_lp_shape(cudaStream_t s, uint32_t n, const uint64_t* kin, const uint32_t* vin, const uint16_t* bin,
-                            uint64_t* kout, uint32_t* vout, uint16_t* bout, int shift, uint32_t mask,
-                            const uint32_t* off, uint32_t* desc, uint32_t* status,
-                            const uint32_t* flags) {
+struct LpPass {
+  uint32_t n;
+  const uint64_t* kin;
+  const uint32_t* vin;
+  const uint16_t* bin;
+  uint64_t* kout;
+  uint32_t* vout;
+  uint16_t* bout;
+  int shift;
+  uint32_t mask;
+  const uint32_t* off;
+  uint32_t* desc;
+  const uint32_t* flags;
+};
+
+template <bool FIRST, int THREADS, int KPT, int MINB>
+cudaError_t launch_lp_shape(const Launch& L, const LpPass& a) {
   using Sm = LpSmem<THREADS, KPT>;
-  cudaError_t e = kernel_setup(learned_pass_kernel<FIRST, THREADS, KPT>, THREADS, sizeof(Sm));
+  auto kern = learned_pass_kernel<FIRST, THREADS, KPT, MINB>;
+  cudaError_t e = kernel_setup(kern, THREADS, sizeof(Sm));
   if (e != cudaSuccess) return e;
-  learned_pass_kernel<FIRST, THREADS, KPT><<<ceil_div(n, (uint32_t)Sm::TILE), THREADS, sizeof(Sm), s>>>(
-      kin, vin, bin, kout, vout, bout, n, shift, mask, off, desc, status, flags);
-  return cudaGetLastError();
+  return launch_kernel(L, kern, ceil_div(a.n, (uint32_t)Sm::TILE), THREADS, sizeof(Sm), a.kin, a.vin, a.bin, a.kout,
+                       a.vout, a.bout, a.n, a.shift, a.mask, a.off, a.desc, L.status, a.flags);
 }
 
 template <bool FIRST>
-cudaError_t launch_lp(int v, cudaStream_t s, uint32_t n, const uint64_t* kin, const uint32_t* vin,
-                      const uint16_t* bin, uint64_t* kout, uint32_t* vout, uint16_t* bout, int shift, uint32_t mask,
-                      const uint32_t* off, uint32_t* desc, uint32_t* status, const uint32_t* flags) {
-#define GTC_LP(T, K) \
-  return launch_lp_shape<FIRST, T, K>(s, n, kin, vin, bin, kout, vout, bout, shift, mask, off, desc, status, flags)
+cudaError_t launch_lp(int v, const Launch& L, const LpPass& a) {
   switch (v) {
-    case 1: GTC_LP(512, 12);
-    case 2: GTC_LP(384, 16);
-    case 3: GTC_LP(512, 8);
-    default: GTC_LP(256, 16);
+    case 1: return launch_lp_shape<FIRST, 512, 12, 2>(L, a);
+    case 2: return launch_lp_shape<FIRST, 384, 16, 2>(L, a);
+    case 3: return launch_lp_shape<FIRST, 512, 8, 2>(L, a);
+    default: return launch_lp_shape<FIRST, 256, 16, 3>(L, a);
   }
-#undef GTC_LP
 }
 
 std::atomic<int> g_lp_pinned{-1};  // gtc_learned_set_variant
@@ -1092,9 +1116,10 @@ GTC_API gtc_status gtc_learned_histogram_u64(gtc_ctx* ctx, const gtc_learned_mod
   const int B = m->B;
   LTRY(ctx, cudaMemsetAsync(d_counts, 0, (size_t)B * 4, s));
   if (n == 0) return GTC_OK;
-  gtc_status st = prepare_model(ctx, m, nullptr, s);
+  const Launch L = context_launch(ctx, stream);
+  gtc_status st = prepare_model(ctx, L, m, nullptr);
   if (st != GTC_OK) return st;
-  return launch_count(ctx, m, keys, n, d_counts, nullptr, nullptr, s);
+  return launch_count(ctx, L, m, keys, n, d_counts, nullptr, nullptr);
 }
 
 }  // extern "C"
@@ -1104,7 +1129,10 @@ int learned_select_variant(uint32_t n) {
   const int pinned = g_lp_pinned.load(std::memory_order_relaxed);
   if (pinned >= 0) return pinned;
   const int t = tuned_learned_variant(n);
-  return (t >= 0 && t < kLpNumVariants) ? t : 0;
+  if (t >= 0 && t < kLpNumVariants) return t;
+  // Untuned: 512 x 8 (whole sorts, 4M / 16.8M / 67M keys: 297 / 710 / 2603 us;
+  // 256 x 16 308 / 749 / 2664, 512 x 12 309 / 716 / 2646).
+  return n >= 2000000 ? 3 : 0;
 }
 int learned_num_variants() { return kLpNumVariants; }
 
@@ -1136,26 +1164,32 @@ gtc_status learned_sort_variant(gtc_ctx* ctx, const gtc_learned_model* m, const 
   const Launch L0 = context_launch(ctx, stream);
   LTRY(ctx, cudaMemsetAsync(W.totals, 0, (size_t)B * 4, s));
   LTRY(ctx, cudaMemsetAsync(W.desc, 0, 2 * W.desc_words * 4, s));
-  gtc_status st = prepare_model(ctx, m, d_flags, s);
-  if (st == GTC_OK) st = launch_count(ctx, m, keys, n, W.totals, W.bid, d_flags, s);
-  if (st != GTC_OK) return st;
-  learned_scan_kernel<<<1, 1024, 0, s>>>(W.totals, B, db1, m->heights, W.base, W.off1, W.off2, d_flags);
-  LTRY(ctx, cudaGetLastError());
-  LTRY(ctx, launch_lp<true>(variant, s, n, keys, vals, W.bid, db2 ? W.tkeys : W.ukeys, db2 ? W.tvals : W.uvals,
-                            W.bid2, 0, (1u << db1) - 1, W.off1, W.desc, L0.status, d_flags));
-  if (db2)
-    LTRY(ctx, launch_lp<false>(variant, s, n, W.tkeys, W.tvals, W.bid2, W.ukeys, W.uvals, nullptr, db1,
-                               (1u << db2) - 1, W.off2, W.desc + W.desc_words, L0.status, d_flags));
-  bucket_sort_kernel<<<B, BS_THREADS, sizeof(BucketSmem), s>>>(W.ukeys, W.uvals, W.base, W.totals, keys_out, vals_out,
-                                                               W.bmin, W.bmax, d_flags);
-  learned_order_check_kernel<<<ceil_div(B, 256), 256, 0, s>>>(W.totals, W.bmin, W.bmax, B, d_flags);
-  LTRY(ctx, cudaGetLastError());
-  // Fallback: copy + plain onesweep, all gated on the flag word.
-  cond_copy_kernel<<<L0.num_sms * 4, 256, 0, s>>>(keys, vals, keys_out, vals_out, n, d_flags);
-  Launch L = L0;
-  L.run_if = d_flags;
   const SortWorkspace SW = carve_sort_workspace(W.sort_ws, n, 8, 0);
   LTRY(ctx, cudaMemsetAsync(SW.header, 0, SW.header_words * 4, s));
+  // Everything after the first kernel is a programmatic dependent launch.
+  Launch Lp = L0;
+  Lp.pdl = context_stage_idle(ctx);
+  gtc_status st = prepare_model(ctx, L0, m, d_flags);
+  if (st == GTC_OK) st = launch_count(ctx, Lp, m, keys, n, W.totals, W.bid, d_flags);
+  if (st != GTC_OK) return st;
+  LTRY(ctx, kernel_setup(learned_scan_kernel, 1024, scan_smem_bytes(MAX_BUCKETS)));
+  LTRY(ctx, launch_kernel(Lp, learned_scan_kernel, 1, 1024, scan_smem_bytes(B), W.totals, B, db1, m->heights, W.base,
+                          W.off1, W.off2, d_flags));
+  LTRY(ctx, launch_lp<true>(variant, Lp,
+                            LpPass{n, keys, vals, W.bid, db2 ? W.tkeys : W.ukeys, db2 ? W.tvals : W.uvals, W.bid2, 0,
+                                   (1u << db1) - 1, W.off1, W.desc, d_flags}));
+  if (db2)
+    LTRY(ctx, launch_lp<false>(variant, Lp,
+                               LpPass{n, W.tkeys, W.tvals, W.bid2, W.ukeys, W.uvals, nullptr, db1, (1u << db2) - 1,
+                                      W.off2, W.desc + W.desc_words, d_flags}));
+  LTRY(ctx, launch_kernel(Lp, bucket_sort_kernel, B, BS_THREADS, sizeof(BucketSmem), W.ukeys, W.uvals, W.base,
+                          W.totals, keys_out, vals_out, W.bmin, W.bmax, d_flags));
+  LTRY(ctx, launch_kernel(Lp, learned_order_check_kernel, ceil_div(B, 256), 256, 0, W.totals, W.bmin, W.bmax, B,
+                          d_flags));
+  // Fallback: copy + plain onesweep, all gated on the flag word.
+  LTRY(ctx, launch_kernel(Lp, cond_copy_kernel, L0.num_sms * 4, 256, 0, keys, vals, keys_out, vals_out, n, d_flags));
+  Launch L = Lp;
+  L.run_if = d_flags;
   LTRY(ctx, launch_global_hist<uint64_t>(L, keys_out, n, 0, 64, SW, 8));
   bool in_alt = false;
   // Variant 4 is a persistent kernel (one resident wave of CTAs pulling

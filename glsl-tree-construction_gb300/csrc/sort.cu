@@ -1235,9 +1235,8 @@ cudaError_t launch_global_hist(const Launch& L, const K* keys, uint32_t n, int b
   if (db < 1 || db > 8 || passes < 1 || passes > MAX_PASSES) return cudaErrorInvalidValue;
   constexpr int T = 512;
   const uint32_t grid = max(1u, min(hist_blocks(L, n, T, 16), (uint32_t)L.num_sms * 2));
-  global_hist_kernel<K, T><<<grid, T, 0, L.stream>>>(keys, n, begin_bit, end_bit, passes, db, W.counts,
-                                                     W.bin_offsets, W.header, W.desc, W.desc_words, L.run_if);
-  return cudaGetLastError();
+  return launch_kernel(L, global_hist_kernel<K, T>, grid, T, 0, keys, n, begin_bit, end_bit, passes, db, W.counts,
+                       W.bin_offsets, W.header, W.desc, W.desc_words, L.run_if);
 }
 template cudaError_t launch_global_hist<uint32_t>(const Launch&, const uint32_t*, uint32_t, int, int,
                                                   const SortWorkspace&, int, int);

@@ -419,8 +419,8 @@ GTC_API gtc_status gtc_learned_sort_u64(gtc_ctx* ctx, const gtc_learned_model* m
 /* Tile shapes of the learned sort's two bucket-id grouping passes compiled
  * into the library (threads per block x keys per thread).  A sort uses the
  * pinned variant, else the autotuner's pick for its n
- * (gtc_autotune_learned), else variant 0.  Every variant gives identical
- * output.  No reference counterpart. */
+ * (gtc_autotune_learned), else variant 3 from 2 million keys on and 0 below.
+ * Every variant gives identical output.  No reference counterpart. */
 GTC_API int gtc_learned_num_variants(void);
 GTC_API gtc_status gtc_learned_variant_shape(int variant, int* threads, int* keys_per_thread);
 /* Pins one variant for every learned sort; variant = -1 unpins. */
