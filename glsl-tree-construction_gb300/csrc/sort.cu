@@ -721,19 +721,19 @@ __global__ void __launch_bounds__(THREADS, MINB) onesweep_kernel(const K* __rest
 // ------------------------------------------------- one-wave onesweep ------
 // The same pass for inputs whose tiles are all resident at once: a pass is
 // then one chain of dependent steps, and the chain is what it costs.  Against
-// onesweep_kernel: short tiles (4 or 8 keys per thread: fewer ranking steps in
-// a row, more SMs), and a look-back over 32 descriptors per round trip, since
+// onesweep_kernel: short tiles of 4 keys per thread (fewer ranking steps in a
+// row, more SMs), and a look-back over 32 descriptors per round trip, since
 // the tiles publish at about the same time.  Whole sorts of uniform pairs,
-// histogram included (us; beside them the 256 x 16 tiles of onesweep_kernel):
-//   pairs     u32: 256 x 16   4 keys   8 keys    u64: 256 x 16   4 keys   8 keys
-//   30,000          27.9       21.0     21.9           54.2       38.5     40.0
-//   65,536          30.4       24.7     26.7           58.4       44.1     47.6
-//   90,000          31.0       28.2     28.7           59.5       51.9     51.9
-//   110,000         31.8       30.9     28.9           61.7       56.8     52.3
-//   180,000         33.1         -      32.4           64.3         -      58.8
-//   220,000         34.5         -      36.0           66.3         -      65.2
-//   260,000         37.8         -      40.6           70.6         -      71.1
-// (16 keys per thread were never the fastest.  Clusters of eight blocks that
+// histogram included (us; beside them the 256 x 16 and 256 x 8 tiles of
+// onesweep_kernel and of this one):
+//   pairs     u32: 256 x 16  256 x 4  256 x 8  512 x 4   u64: 256 x 16  256 x 4  256 x 8  512 x 4
+//   16,384          27.1      19.7     21.9     20.6           52.0      34.7     38.6     37.7
+//   65,536          30.4      24.6     26.9     25.5           58.5      43.8     47.4     46.3
+//   92,000          31.2      28.6     28.7     27.5           59.4      51.9     51.6     50.1
+//   150,000         32.3      35.5     30.4     29.1           61.9      65.7     54.6     53.2
+//   185,000         32.6         -     33.0     31.8           62.9         -     59.3     58.4
+//   225,000         34.7         -     36.5     35.7           66.1         -     66.2     66.1
+// (256 x 16 in this form was never the fastest.  Clusters of eight blocks that
 // add up their counts through distributed shared memory and look back once
 // per cluster: 24.0 us for 65,536 u32 pairs, but 19.5 against 16.6 for 4,097
 // and 64.9 against 52.6 for 1M, by this kernel and onesweep_kernel.)
@@ -753,7 +753,7 @@ __global__ void __launch_bounds__(THREADS) onesweep_wave_kernel(const K* __restr
   using S = OnesweepSmem<K, THREADS, KPT>;
   constexpr int WARPS = S::WARPS;
   constexpr int TILE = S::TILE;
-  static_assert(THREADS == RADIX, "one thread per digit");
+  static_assert(THREADS >= RADIX, "one thread per digit");
   static_assert(TILE <= 65536, "warp ranks are packed in 16 bits");
   extern __shared__ __align__(16) unsigned char smem_raw[];
   S& s = *reinterpret_cast<S*>(smem_raw);
@@ -762,7 +762,7 @@ __global__ void __launch_bounds__(THREADS) onesweep_wave_kernel(const K* __restr
   const uint32_t tile = blockIdx.x;
   const uint32_t tile_base = tile * TILE;
   const uint32_t skip = *first_tile;
-  const uint32_t bin0 = bin_off[tid];
+  const uint32_t bin0 = tid < RADIX ? bin_off[tid] : 0u;
 
   K key[KPT];
   uint32_t val[KPT], rank[KPT];
@@ -790,16 +790,20 @@ __global__ void __launch_bounds__(THREADS) onesweep_wave_kernel(const K* __restr
   __syncthreads();
   if (tile < skip) return;
   uint32_t count = 0;
+  if (tid < RADIX) {
 #pragma unroll
-  for (int w = 0; w < WARPS; ++w) {
-    const uint32_t c = s.warp_hist[w][tid];
-    s.warp_hist[w][tid] = count;
-    count += c;
+    for (int w = 0; w < WARPS; ++w) {
+      const uint32_t c = s.warp_hist[w][tid];
+      s.warp_hist[w][tid] = count;
+      count += c;
+    }
+    st_relaxed(desc + (size_t)tile * RADIX + tid, (count << 2) | (tile == 0 ? FLAG_INCLUSIVE : FLAG_AGGREGATE));
   }
-  st_relaxed(desc + (size_t)tile * RADIX + tid, (count << 2) | (tile == 0 ? FLAG_INCLUSIVE : FLAG_AGGREGATE));
   const uint32_t digit_off = scan256_exclusive<THREADS>(count, s.warp_sums);
+  if (tid < RADIX) {
 #pragma unroll
-  for (int w = 0; w < WARPS; ++w) s.warp_hist[w][tid] += digit_off;
+    for (int w = 0; w < WARPS; ++w) s.warp_hist[w][tid] += digit_off;
+  }
   __syncthreads();
 #pragma unroll
   for (int j = 0; j < KPT; ++j) {
@@ -807,12 +811,14 @@ __global__ void __launch_bounds__(THREADS) onesweep_wave_kernel(const K* __restr
     s.keys[local] = key[j];
     if (HAS_VALS) s.vals[local] = val[j];
   }
-  uint32_t excl = 0;
-  if (tile > 0) {
-    excl = lookback_window<32, RADIX>(desc, tile, tid, status);
-    st_relaxed(desc + (size_t)tile * RADIX + tid, ((excl + count) << 2) | FLAG_INCLUSIVE);
+  if (tid < RADIX) {
+    uint32_t excl = 0;
+    if (tile > 0) {
+      excl = lookback_window<32, RADIX>(desc, tile, tid, status);
+      st_relaxed(desc + (size_t)tile * RADIX + tid, ((excl + count) << 2) | FLAG_INCLUSIVE);
+    }
+    s.global_base[tid] = bin0 + excl - digit_off;
   }
-  s.global_base[tid] = bin0 + excl - digit_off;
   __syncthreads();
   const uint32_t valid = min((uint32_t)TILE, n - tile_base);
 #pragma unroll
@@ -1047,7 +1053,7 @@ constexpr Variant kVariants[] = {{256, 16, 0, 3, 0}, {384, 16, 0, 2, 0}, {512, 1
                                  {512, 8, 0, 2, 0},  {384, 12, 0, 3, 0}, {256, 16, 0, 3, 1}, {384, 16, 0, 2, 1},
                                  {512, 12, 0, 2, 1}, {256, 24, 0, 2, 1}, {256, 16, 4, 3, 0}, {512, 12, 4, 2, 1},
                                  {256, 16, 4, 3, 2}, {512, 12, 4, 2, 2}, {384, 16, 4, 2, 2}, {256, 4, 5, 1, 1},
-                                 {256, 8, 5, 1, 1}};
+                                 {512, 4, 5, 1, 1},  {1024, 4, 0, 1, 0}};
 constexpr int kNumVariants = sizeof(kVariants) / sizeof(kVariants[0]);
 static const int g_variant[2] = {0, 2};  // [u32, u64]: what gtc_sort_get_variant reports with nothing pinned
 static std::atomic<int> g_pinned[2] = {{-1}, {-1}};  // gtc_sort_set_variant: overrides the tuned choice
@@ -1055,11 +1061,12 @@ static std::atomic<int> g_pinned[2] = {{-1}, {-1}};  // gtc_sort_set_variant: ov
 // Largest inputs of the one-wave variants (kind 5).  The short tiles' limits
 // bound the look-back descriptors of the workspace (one row of 256 words per
 // tile and pass); every one-wave launch also needs its tiles resident.
-constexpr int WAVE_4 = 19, WAVE_8 = 20;  // their places in kVariants
-constexpr uint32_t WAVE_4_MAX = 160 * 1024, WAVE_8_MAX = 200 * 2048;
-constexpr uint32_t WAVE_4_USE = 92000, WAVE_8_USE[2] = {185000, 225000};  // untuned, [u32, u64]
-static_assert(kVariants[WAVE_4].kind == 5 && kVariants[WAVE_4].kpt == 4 && kVariants[WAVE_8].kpt == 8 &&
-                  kNumVariants == 21,
+constexpr int WAVE_1K = 19, WAVE_2K = 20;  // their places in kVariants, by keys per tile
+constexpr uint32_t WAVE_1K_MAX = 160 * 1024, WAVE_2K_MAX = 200 * 2048;
+constexpr uint32_t WAVE_1K_USE = 78000, WAVE_2K_USE[2] = {175000, 200000};  // untuned, [u32, u64]
+static_assert(kVariants[WAVE_1K].kind == 5 && kVariants[WAVE_1K].threads * kVariants[WAVE_1K].kpt == 1024 &&
+                  kVariants[WAVE_2K].kind == 5 && kVariants[WAVE_2K].threads * kVariants[WAVE_2K].kpt == 2048 &&
+                  kNumVariants == 22,
               "variant numbers");
 
 int sort_select_variant(int key_bits, int bits, uint32_t n) {
@@ -1069,22 +1076,35 @@ int sort_select_variant(int key_bits, int bits, uint32_t n) {
   const int t = tuned_variant(key_bits, bits, n);
   if (t >= 0 && t < kNumVariants) return t;
   // Untuned: the one-wave tiles while the look-back stays short
-  // (onesweep_wave_kernel has the times around the crossings).
-  if (n <= WAVE_4_USE) return WAVE_4;
-  if (n <= WAVE_8_USE[w]) return WAVE_8;
+  // (onesweep_wave_kernel has the times).  Above them, as many threads per
+  // tile as keep every tile resident, since a tile is a chain of dependent
+  // steps: 1,024 (152 tiles of 4,096 at one per SM), 512 (304 at two), then
+  // larger tiles (304 of 6,144).  Sort of uniform pairs alone (us):
+  //          u32: 256 x 16  512 x 8  1024 x 4  384 x 16   u64: 256 x 16  512 x 8  1024 x 4  384 x 16
+  //   185K            32.6     30.8      31.4      36.3           62.9     59.1      60.9      70.0
+  //   225K            34.7     33.6      32.5      36.9           66.1     63.1      62.7      70.7
+  //   300K            37.9     34.5      33.4      39.8           70.6     65.0      64.3      75.2
+  //   400K            40.2     37.2      35.9      41.2           75.8     72.5      68.4      77.4
+  //   700K            46.5     43.1      50.9      48.0           95.5     85.4     104.3      98.3
+  //   1.05M           52.6     46.9      60.1      51.7          104.5     94.5     123.6     105.6
+  //   1.7M            59.7     68.6         -      57.9          121.2    140.0         -     117.4
+  if (n <= WAVE_1K_USE) return WAVE_1K;
+  if (n <= WAVE_2K_USE[w]) return WAVE_2K;
+  if (n <= 152 * 4096) return 21;
+  if (n <= 304 * 4096) return 8;
+  if (n <= 304 * 6144) return 1;
   // Above, by how the tiles fill waves (resident tiles on 152 SMs: 304 of
   // 6,144 keys, 456 of 4,608 or 4,096, 608 of 4,096 with variant 7, whose 64
-  // registers only 32-bit keys fit without spilling).  Sort of uniform pairs
-  // with the caller's copies in (us):
+  // registers only 32-bit keys fit without spilling).  With the caller's
+  // copies in (us):
   //          u32: var. 0  var. 9  var. 7    u64: var. 2  var. 0  var. 9  var. 14
-  //   1.05M         63.9    68.4    69.3         123.7   116.0   134.1    116.0
   //   2.0M          83.4    76.6    80.8         177.5   162.0   151.2    162.4
   //   4.0M         126.7   122.3   124.3         280.6   261.5   263.5    260.5
   //   8.0M         223.6   217.5   213.0         485.3   475.9   504.1    460.3
   //   16.8M        431.4   420.8   405.1         942.7   950.7  1027.1    943.2
   //   33.6M        831.7   810.0   775.4        1809.1  1841.6  2002.2   1850.3
-  if (w) return n <= 1860000 ? 0 : n <= 2100000 ? 9 : n <= 20000000 ? 14 : 2;
-  return n <= 1860000 ? 0 : n <= 6000000 ? 9 : 7;
+  if (w) return n <= 2100000 ? 9 : n <= 20000000 ? 14 : 2;
+  return n <= 6000000 ? 9 : 7;
 }
 
 template <class K, int THREADS, int KPT, bool HV, int MINB, int RANK, bool L2H = false, bool TICKET = false>
@@ -1142,10 +1162,10 @@ static cudaError_t launch_variant(int v, bool hv, const Launch& L, const K* kin,
   if ((kVariants[v].kind == 1 || kVariants[v].kind == 2) && (!aligned || (hv && !vin))) v = 0;
   if (kVariants[v].kind == 5) {
     cudaError_t e = cudaSuccess;
-#define GTC_WV(P)                                                                                              \
-  (hv ? launch_wave<K, 256, P, true>(L, kin, vin, kout, vout, n, shift, dmask, bin_off, desc, tc, &e)      \
-      : launch_wave<K, 256, P, false>(L, kin, vin, kout, vout, n, shift, dmask, bin_off, desc, tc, &e))
-    const bool done = v == WAVE_4 ? n <= WAVE_4_MAX && GTC_WV(4) : n <= WAVE_8_MAX && GTC_WV(8);
+#define GTC_WV(T, P)                                                                                              \
+  (hv ? launch_wave<K, T, P, true>(L, kin, vin, kout, vout, n, shift, dmask, bin_off, desc, tc, &e)      \
+      : launch_wave<K, T, P, false>(L, kin, vin, kout, vout, n, shift, dmask, bin_off, desc, tc, &e))
+    const bool done = v == WAVE_1K ? n <= WAVE_1K_MAX && GTC_WV(256, 4) : n <= WAVE_2K_MAX && GTC_WV(512, 4);
 #undef GTC_WV
     if (done) return e;
     v = 0;
@@ -1181,7 +1201,8 @@ static cudaError_t launch_variant(int v, bool hv, const Launch& L, const K* kin,
     case 15: GTC_OSH(512, 12, 2, 1);
     case 16: GTC_OSH(256, 16, 3, 2);
     case 17: GTC_OSH(512, 12, 2, 2);
-    default: GTC_OSH(384, 16, 2, 2);
+    case 18: GTC_OSH(384, 16, 2, 2);
+    default: GTC_OS(1024, 4, 1, 0);
   }
 #undef GTC_OS
 #undef GTC_OSH
@@ -1191,7 +1212,7 @@ static cudaError_t launch_variant(int v, bool hv, const Launch& L, const K* kin,
 
 // Smallest tile of any variant that takes n keys: sizes the descriptor array
 // for every variant.
-static int min_tile_keys(uint32_t n) { return n <= WAVE_4_MAX ? 1024 : n <= WAVE_8_MAX ? 2048 : 4096; }
+static int min_tile_keys(uint32_t n) { return n <= WAVE_1K_MAX ? 1024 : n <= WAVE_2K_MAX ? 2048 : 4096; }
 static constexpr bool tiles_covered() {
   for (const Variant& v : kVariants)
     if (v.kind != 5 && v.threads * v.kpt < 4096) return false;

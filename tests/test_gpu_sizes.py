@@ -130,9 +130,10 @@ def test_row_scans(ctx, n, dups):
 
 
 @pytest.mark.parametrize("key_bits", [32, 64])
-@pytest.mark.parametrize("variant", [-1, 19, 20])
+@pytest.mark.parametrize("variant", [-1, 19, 20, 21])
 def test_one_wave_sort(ctx, key_bits, variant):
-    """The one-wave onesweep pass (default up to 185,000 or 225,000 keys, and pinned):
+    """The one-wave onesweep pass (default up to 175,000 or 200,000 keys, and pinned)
+    and the shapes above it:
     tile edges, the untuned choice's crossings, the variants' own limits and
     one past them, narrow digits, unaligned inputs, the first-tile switch."""
     import torch
@@ -156,8 +157,8 @@ def test_one_wave_sort(ctx, key_bits, variant):
 
     try:
         ctx.set_sort_variant(key_bits, variant)
-        for n in (1, 31, 255, 257, 1023, 1024, 1025, 4097, 92_000, 92_001, 163_840, 163_841, 185_000, 185_001, 225_000,
-                  225_001, 409_600, 409_601):
+        for n in (1, 31, 255, 257, 1023, 1024, 1025, 4097, 78_000, 78_001, 163_840, 163_841, 175_000, 175_001, 200_000,
+                  200_001, 409_600, 409_601, 622_592, 622_593, 1_245_185, 1_867_777):
             check(W.config3_keys(n, key_bits, and_words=n % 4, seed=n), 0, key_bits)
         for n in (5000, 120_007):
             keys = W.config3_keys(n, key_bits, seed=n)
