@@ -65,18 +65,22 @@ constexpr int BM_THREADS = 512;  // Morton kernel: one block per tile
 struct BtVariant {
   int threads, kpt;
 };
-constexpr BtVariant kBtVariants[] = {{512, 12}, {256, 16}, {384, 16}, {512, 8}, {256, 24}, {256, 8}, {256, 16}};
+constexpr BtVariant kBtVariants[] = {{512, 12}, {256, 16}, {384, 16}, {512, 8}, {256, 24}, {512, 4}, {256, 16}};
 constexpr int kBtNumVariants = sizeof(kBtVariants) / sizeof(kBtVariants[0]);
 // Variant 6 is 256 x 16 held to 64 registers (four blocks per SM), as sort.cu's
 // variant 7; variant 5 has short tiles for small batches, where a pass is one
 // chain of dependent steps, and is limited to BT_SMALL_MAX points, which bounds
 // the workspace's descriptors.  Whole builds (us):
-//   points, clouds         512 x 12   256 x 8   256 x 16 at 4 blocks per SM
-//   300,125, 64                95.6      79.4      94.4
-//   422,794, 200               99.7      92.4     107.7
-//   1,562,588, 20             153.6        -      179.3
-//   3,211,561, 200            288.6        -      279.7
-//   74,044,652, 512          4386.9        -     4274.9
+//   points, clouds         512 x 12   512 x 4   256 x 16 at 4 blocks per SM
+//   9,293, 16                  55.5      48.3      56.5
+//   300,125, 64                90.3      74.8      81.6
+//   422,794, 200               93.5      83.3      94.9
+//   598,201, 16                98.7      89.7     101.7
+//   1,562,588, 20             154.5        -      172.3
+//   3,211,561, 200            257.7        -      247.3
+//   74,044,652, 512          3640.1        -     3552.9
+// (512 x 4 took over from 256 x 8: 77.0 -> 74.6 us for 64 clouds of 300 to
+// 20,000 points as a graph, the same tile with half the ranking steps.)
 constexpr int BT_SMALL = 5, BT_LARGE = 6;
 constexpr uint32_t BT_SMALL_MAX = 600000;
 constexpr uint32_t BT_LARGE_MIN = 2000000;  // untuned batches from here on take variant 6
@@ -723,7 +727,7 @@ cudaError_t launch_bt_variant(int v, const Launch& L, uint32_t grid, const BtPas
     case 2: return launch_bt_pass<384, 16, 2>(L, grid, a);
     case 3: return launch_bt_pass<512, 8, 2>(L, grid, a);
     case 4: return launch_bt_pass<256, 24, 2>(L, grid, a);
-    case BT_SMALL: return launch_bt_pass<256, 8, 4>(L, grid, a);
+    case BT_SMALL: return launch_bt_pass<512, 4, 2>(L, grid, a);
     case BT_LARGE: return launch_bt_pass<256, 16, 4>(L, grid, a);
     default: return launch_bt_pass<512, 12, 2>(L, grid, a);
   }
