@@ -234,7 +234,8 @@ __global__ void __launch_bounds__(BM_THREADS) bt_morton_kernel(const float4* __r
   flush();
 }
 
-// Per cloud and pass: digit counts -> global digit bases, in place.
+// Per cloud and pass: digit counts -> global digit bases, in place.  Only the
+// 64-register tiles of large batches want it (bt_onesweep_kernel).
 __global__ void __launch_bounds__(BRADIX) bt_seg_scan_kernel(uint32_t* seg_hist, const uint32_t* off) {
   griddep_wait();
   __shared__ uint32_t s_w[BRADIX / 32];
@@ -261,23 +262,28 @@ struct BtSmem {
   uint32_t vals[TILE];
   uint32_t warp_hist[WARPS][BRADIX];
   uint32_t gbase[BRADIX];
+  uint32_t hist_sums[BRADIX / 32];
   uint32_t warp_sums[WARPS + 1];
 };
 
 // One segmented onesweep pass: the single-cloud pass of sort.cu with tiles
-// confined to one cloud and digit bases from that cloud's histogram.  A
+// confined to one cloud and digit bases from that cloud's histogram.  Every
+// tile scans that for itself, behind its keys' loads, which saves a launch:
+// 64 clouds of 300 to 20,000 points 74.6 -> 71.5 us.  SCANNED takes the bases
+// from bt_seg_scan_kernel: in variant 6 the scan in the tile spills, and
+// 512 clouds of 74M points took 3641 us against 3566.  A
 // cloud's last tile is padded with all-ones keys, which rank last in the tile
 // and are never stored.  Its descriptor counts them, but no tile reads it:
 // the next tile starts another cloud and does not look back.  FIRST: the
 // payload is the point's index in its cloud, made here.
-template <int THREADS, int KPT, int MINB, bool FIRST>
+template <int THREADS, int KPT, int MINB, bool FIRST, bool SCANNED>
 __global__ void __launch_bounds__(THREADS, MINB) bt_onesweep_kernel(const uint32_t* __restrict__ kin,
                                                                  const uint32_t* __restrict__ vin,
                                                                  uint32_t* __restrict__ kout,
                                                                  uint32_t* __restrict__ vout, const uint32_t* off,
                                                                  uint32_t S, const uint32_t* tile_start,
                                                                  const uint32_t* tile_cloud, int shift,
-                                                                 const uint32_t* seg_base, int pass, uint32_t* desc,
+                                                                 const uint32_t* seg_hist, int pass, uint32_t* desc,
                                                                  uint32_t* status) {
   griddep_wait();
   using Sm = BtSmem<THREADS, KPT>;
@@ -299,6 +305,12 @@ __global__ void __launch_bounds__(THREADS, MINB) bt_onesweep_kernel(const uint32
     key[j] = (i < r.valid) ? kin[r.base + i] : 0xffffffffu;
     if (FIRST) val[j] = r.local * Sm::TILE + i;
     else val[j] = (i < r.valid) ? vin[r.base + i] : 0u;
+  }
+  if (!SCANNED && tid < BRADIX) {  // the cloud's keys of smaller digits, but for earlier warps' digits
+    const uint32_t h = seg_hist[((size_t)r.cloud * BPASSES + pass) * BRADIX + tid];
+    const uint32_t incl = warp_inclusive_sum(h);
+    s.gbase[tid] = incl - h;
+    if (lane == 31) s.hist_sums[warp] = incl;
   }
   uint32_t* my_hist = s.warp_hist[warp];
 #pragma unroll
@@ -351,7 +363,13 @@ __global__ void __launch_bounds__(THREADS, MINB) bt_onesweep_kernel(const uint32
       excl = lookback_window<8, BRADIX>(desc, tile, tid, status);
       st_relaxed(desc + (size_t)tile * BRADIX + tid, ((excl + count) << 2) | FLAG_INCLUSIVE);
     }
-    s.gbase[tid] = seg_base[((size_t)r.cloud * BPASSES + pass) * BRADIX + tid] + excl - doff;
+    if constexpr (SCANNED) {
+      s.gbase[tid] = seg_hist[((size_t)r.cloud * BPASSES + pass) * BRADIX + tid] + excl - doff;
+    } else {
+      uint32_t base = r.base - r.local * Sm::TILE + excl - doff;
+      for (int w = 0; w < warp; ++w) base += s.hist_sums[w];
+      s.gbase[tid] += base;
+    }
   }
   __syncthreads();
   // o stays inside the cloud while every look-back completes; after one ran
@@ -707,18 +725,19 @@ struct BtPass {
   const uint32_t* tile_start;
   const uint32_t* tile_cloud;
   int pass;
-  const uint32_t* seg_base;
+  const uint32_t* seg_hist;
   uint32_t* desc;
 };
 
-template <int THREADS, int KPT, int MINB>
+template <int THREADS, int KPT, int MINB, bool SCANNED = false>
 cudaError_t launch_bt_pass(const Launch& L, uint32_t grid, const BtPass& a) {
   using Sm = BtSmem<THREADS, KPT>;
-  auto kern = a.pass == 0 ? bt_onesweep_kernel<THREADS, KPT, MINB, true> : bt_onesweep_kernel<THREADS, KPT, MINB, false>;
+  auto kern = a.pass == 0 ? bt_onesweep_kernel<THREADS, KPT, MINB, true, SCANNED>
+                          : bt_onesweep_kernel<THREADS, KPT, MINB, false, SCANNED>;
   cudaError_t e = kernel_setup(kern, THREADS, sizeof(Sm));
   if (e != cudaSuccess) return e;
   return launch_kernel(L, kern, grid, THREADS, sizeof(Sm), a.kin, a.vin, a.kout, a.vout, a.off, a.S, a.tile_start,
-                       a.tile_cloud, 8 * a.pass, a.seg_base, a.pass, a.desc, L.status);
+                       a.tile_cloud, 8 * a.pass, a.seg_hist, a.pass, a.desc, L.status);
 }
 
 cudaError_t launch_bt_variant(int v, const Launch& L, uint32_t grid, const BtPass& a) {
@@ -728,7 +747,7 @@ cudaError_t launch_bt_variant(int v, const Launch& L, uint32_t grid, const BtPas
     case 3: return launch_bt_pass<512, 8, 2>(L, grid, a);
     case 4: return launch_bt_pass<256, 24, 2>(L, grid, a);
     case BT_SMALL: return launch_bt_pass<512, 4, 2>(L, grid, a);
-    case BT_LARGE: return launch_bt_pass<256, 16, 4>(L, grid, a);
+    case BT_LARGE: return launch_bt_pass<256, 16, 4, true>(L, grid, a);
     default: return launch_bt_pass<512, 12, 2>(L, grid, a);
   }
 }
@@ -888,7 +907,7 @@ gtc_status build_octree_batched_variant(gtc_ctx* ctx, const float* pts, const ui
     BCHK(launch_kernel(Lp, kern, ceil_div(W.tiles_max, group), BM_THREADS, 0, reinterpret_cast<const float4*>(pts),
                        d_offsets, S, W.tile_start, tile, group, min_coord, range, inv, W.keys_alt, W.tile_cloud,
                        W.seg_hist, reinterpret_cast<uint4*>(W.desc), W.desc_words / 4));
-    BCHK(launch_kernel(Lp, bt_seg_scan_kernel, S, BRADIX, 0, W.seg_hist, d_offsets));
+    if (variant == BT_LARGE) BCHK(launch_kernel(Lp, bt_seg_scan_kernel, S, BRADIX, 0, W.seg_hist, d_offsets));
   }
   uint32_t* src_k = W.keys_alt;
   uint32_t* src_v = W.idx_alt;
