@@ -940,10 +940,7 @@ gtc_status build_octree_batched_variant(gtc_ctx* ctx, const float* pts, const ui
                              out->keys, nullptr, 0u, out->key_offset, S, out->prefix_n, out->has_leaf_left,
                              out->has_leaf_right, out->left_child, out->parent, out->edge_count, nullptr, rec);
       };
-      BCHK(n_total <= TW_SMALL_MAX    ? window(TwSmall{})
-           : n_total <= TW_SMALL4_MAX ? window(TwSmall4{})
-           : n_total <= TW_MID_MAX    ? window(TwMid{})
-                                      : window(TwSegLarge{}));
+      BCHK(n_total <= TW_TWO_MAX ? tw_window_two(n_total, window) : window(TwSegLarge{}));
     } else {
       const uint32_t grid = max(1u, min(ceil_div(n_total, 256), (uint32_t)L.num_sms * 8));
       BCHK(launch_kernel(Lp, bt_tree_kernel, grid, 256, 0, out->keys, out->key_offset, S, out->prefix_n,

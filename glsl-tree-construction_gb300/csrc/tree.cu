@@ -61,11 +61,11 @@ cudaError_t launch_radix_tree(const Launch& L, const K* codes, const uint32_t* d
       return launch_kernel(L, radix_tree_window_kernel<K, false, SH>, max(1u, ceil_div(work, SH::T)), TW_THREADS, 0,
                            codes, d_u, u_host, nullptr, 0u, prefix_n, hll, hlr, left, parent, edge, d_m, rec);
     };
-    return work <= TW_SMALL_MAX    ? window(TwSmall{})
-           : work <= TW_SMALL4_MAX ? window(TwSmall4{})
-           : work <= TW_MID_MAX    ? window(TwMid{})
-           : work <= TW_MID3_MAX   ? window(TwMid3{})
-                                   : window(TwLarge{});
+    return work <= TW_TWO_MAX             ? tw_window_two(work, window)
+           : work <= 3 * TW_SMS * 3072    ? window(TwShape<3072, 512, 3>{})
+           : work <= 3 * TW_SMS * 3584    ? window(TwShape<3584, 512, 3>{})
+           : work <= TW_WAVE_MAX          ? window(TwShape<4096, 512, 3>{})
+                                          : window(TwLarge{});
   }
   const uint32_t grid = max(1u, min(ceil_div(work, TREE_THREADS), (uint32_t)L.num_sms * 8));
   radix_tree_kernel<K><<<grid, TREE_THREADS, 0, L.stream>>>(codes, d_u, m_host, prefix_n, hll, hlr, left, parent,

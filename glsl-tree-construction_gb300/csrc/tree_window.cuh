@@ -70,24 +70,45 @@ struct TwShape {
   static_assert(T <= TW_THREADS * TW_C, "one in-chunk pass per lane");
   static_assert(NWB <= 32, "one ballot covers the window's warp-blocks");
 };
-using TwSmall = TwShape<1024, 512, 3>;
-using TwSmall4 = TwShape<1024, 512, 4>;
-using TwMid = TwShape<4096, 512, 2>;
-using TwMid3 = TwShape<4096, 512, 3>;
 using TwLarge = TwShape<4096, 512, 4>;
 using TwSegLarge = TwShape<8192, 1024, 4>;     // batches, where each block also finds its clouds: a build of 83.5M points takes 4.68 ms, 4.73 with TwLarge
-// Splits up to which each shape is used.  Registers: the longer a block's
-// chain counts, the more its threads may have; TwMid takes 64 while at most
-// two blocks per SM run anyway, TwSmall and TwMid3 40, the others 32.
-// Builds with 32-bit codes (us):
-//   points       1024, 3 per SM   1024, 4   4096, 2   4096, 3   4096, 4
-//   400,000           82.3          83.7
-//   600,000           94.2          92.0       95.0
-//   700,000           98.8          96.3       95.9
-//   1,048,576            -             -     110.7     115.1     119.0
-//   1,700,000            -             -     146.0     140.1     145.8
-//   10M, 64-bit          -             -         -     725       712
-constexpr uint32_t TW_SMALL_MAX = 450000, TW_SMALL4_MAX = 700000, TW_MID_MAX = 1240000, TW_MID3_MAX = 1860000;
+
+// One wave: up to 1.87M splits the shape is one whose blocks all run at once,
+// spread evenly over 152 SMs - the shortest tile of that kind, since an SM
+// with one more block than its neighbour is what the kernel then takes, with
+// as many registers as that residency leaves (two blocks per SM: 64, three:
+// 40, four: 32).  Whole builds of uniform points as graphs (us; tile / blocks
+// per SM, in brackets the shape of its neighbours in size):
+//              32-bit codes                      64-bit codes
+//   120,000    512/2  52.0   (1024/3  53.4)      512/2  59.5   (1024/3  59.9)
+//   200,000    512/3  55.7   (1024/3  59.7)      512/3  69.1   (1024/3  73.6)
+//   400,000   1024/3  67.6   (1024/4  69.8)     1024/3  83.9   (1024/4  86.2)
+//   600,000   1024/4  80.0   (4096/2  84.8)     1024/4  92.7   (4096/2  96.3)
+//   780,000   2560/2  87.9   (4096/2  90.8)     2560/2 112.4   (4096/2 113.0)
+//   930,000   3072/2  97.2   (4096/2 101.7)     3072/2 115.7   (4096/2 121.5)
+//   1.05M     3584/2 100.7   (4096/2 103.0)     3584/2 119.6   (4096/2 121.9)
+//   1.24M     4096/2 110.9   (3072/3 111.8)     4096/2 128.8   (3072/3 130.0)
+//   1.40M     3072/3 117.4   (4096/3 124.3)     3072/3 143.5   (4096/3 151.5)
+//   1.63M     3584/3 129.7   (4096/3 131.0)     3584/3 161.1   (4096/3 160.6)
+//   1.86M     4096/3 138.6   (4096/2 145.1)     4096/3 165.3   (4096/2 169.6)
+//   10M                                         4096/4 712     (4096/3 725)
+// (1024/4 is taken up to 700,000, where some SMs have a fifth block: 85.0
+// against 86.3 of 2560/2, and 104.3 against 105.0.)
+constexpr uint32_t TW_SMS = 152;
+constexpr uint32_t TW_TWO_MAX = 2 * TW_SMS * 4096, TW_WAVE_MAX = 3 * TW_SMS * 4096;
+
+// Calls window(shape) with the one-wave shape for work <= TW_TWO_MAX splits.
+template <class F>
+cudaError_t tw_window_two(uint32_t work, F&& window) {
+  return work <= 2 * TW_SMS * 512    ? window(TwShape<512, 512, 2>{})
+         : work <= 3 * TW_SMS * 512  ? window(TwShape<512, 512, 3>{})
+         : work <= 3 * TW_SMS * 1024 ? window(TwShape<1024, 512, 3>{})
+         : work <= 700000            ? window(TwShape<1024, 512, 4>{})
+         : work <= 2 * TW_SMS * 2560 ? window(TwShape<2560, 512, 2>{})
+         : work <= 2 * TW_SMS * 3072 ? window(TwShape<3072, 512, 2>{})
+         : work <= 2 * TW_SMS * 3584 ? window(TwShape<3584, 512, 2>{})
+                                     : window(TwShape<4096, 512, 2>{});
+}
 
 // First index in a[0..n) with a[i] > x.
 __device__ __forceinline__ uint32_t upper_bound_u32(const uint32_t* a, uint32_t n, uint32_t x) {

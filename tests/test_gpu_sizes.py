@@ -19,8 +19,10 @@ def unique_codes(oracle, n, key_bits, seed):
 
 
 @pytest.mark.parametrize("key_bits", [32, 64])
-@pytest.mark.parametrize("u", [2, 1023, 1024, 1025, 1026, 2049, 4096, 4097, 9000, 450_001, 450_002, 700_001, 700_002,
-                               708_609, 1_240_001, 1_240_002, 1_860_001, 1_860_002])
+@pytest.mark.parametrize("u", [2, 511, 512, 513, 514, 1025, 1026, 4097, 9000, 155_649, 155_650, 233_473, 233_474,
+                               466_945, 466_946, 700_001, 700_002, 778_241, 778_242, 933_889, 933_890, 1_089_537,
+                               1_089_538, 1_245_185, 1_245_186, 1_400_833, 1_400_834, 1_634_305, 1_634_306,
+                               1_867_777, 1_867_778])
 def test_tree_window_shapes(ctx, gtc_mod, oracle, key_bits, u):
     """u codes (u - 1 splits) at the tile edges and on both sides of the shape
     rule: the window method against the per-node search."""
@@ -230,7 +232,8 @@ def _spread_clouds(total, seed):
     return clouds
 
 
-@pytest.mark.parametrize("total,variant", [(599_999, -1), (600_000, 5), (600_001, 5), (600_001, -1), (700_001, -1), (1_240_001, -1), (1_999_999, -1),
+@pytest.mark.parametrize("total,variant", [(155_649, -1), (233_472, -1), (466_945, -1), (599_999, -1), (600_000, 5), (600_001, 5), (600_001, -1), (700_001, -1),
+                                           (800_001, -1), (1_000_001, -1), (1_245_185, -1), (1_999_999, -1),
                                            (2_000_000, -1), (2_700_001, 6), (13_001, 6), (13_001, -1)])
 def test_batched_sizes(ctx, gtc_mod, oracle, total, variant):
     """Both sides of every size rule of the batch (tile shape, tree window,
