@@ -387,14 +387,13 @@ gtc_status pipeline(gtc_ctx* ctx, const float* pts, uint32_t n, float mn, float 
   w += align_up((size_t)n * sizeof(K), 256);
   uint32_t* vals_alt = reinterpret_cast<uint32_t*>(w);
   w += align_up((size_t)n * 4, 256);
-  void* sort_ws = w;
-  w += sort_workspace_bytes(n, passes, 0);
+  const SortWorkspace Wk = carve_sort_workspace(w, n, passes, 0);
+  w = reinterpret_cast<char*>(Wk.desc + Wk.desc_words);  // whole digit rows: 256-byte aligned
   void* unique_ws = w;
   w += scan_workspace_bytes(n);
   void* offsets_ws = w;
   w += scan_workspace_bytes(n);
   K* keys = reinterpret_cast<K*>(o->keys);
-  const SortWorkspace Wk = carve_sort_workspace(sort_ws, n, passes, 0);
   // The Morton pass zeroes the counts, the sort's look-back descriptors and, in
   // the same sweep, the unique / node-offset workspaces behind them, so the
   // sort header's memset is the build's only one.

@@ -481,6 +481,8 @@ struct SortWorkspace {
   uint32_t tiles;
 };
 
+// Enough for every sort of up to n keys (never less for more keys); the carve
+// lays out what a sort of exactly n keys uses, its descriptors last.
 size_t sort_workspace_bytes(uint32_t n, int passes, int tile_keys);
 SortWorkspace carve_sort_workspace(void* ws, uint32_t n, int passes, int tile_keys);
 

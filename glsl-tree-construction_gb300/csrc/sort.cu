@@ -1212,7 +1212,21 @@ static cudaError_t launch_variant(int v, bool hv, const Launch& L, const K* kin,
 
 // Smallest tile of any variant that takes n keys: sizes the descriptor array
 // for every variant.
-static int min_tile_keys(uint32_t n) { return n <= WAVE_1K_MAX ? 1024 : n <= WAVE_2K_MAX ? 2048 : 4096; }
+static constexpr uint32_t min_tile_keys(uint32_t n) {
+  return n <= WAVE_1K_MAX ? 1024 : n <= WAVE_2K_MAX ? 2048 : 4096;
+}
+static constexpr uint32_t max_tiles(uint32_t n) {
+  return ((n > 0 ? n : 1) + min_tile_keys(n) - 1) / min_tile_keys(n);
+}
+// The most tiles of any sort of up to n keys.  A workspace made for n keys
+// also serves fewer, and fewer keys may have more tiles: just past each of the
+// short tiles' limits the count halves.
+static constexpr uint32_t max_tiles_up_to(uint32_t n) {
+  uint32_t t = max_tiles(n);
+  if (n > WAVE_1K_MAX && max_tiles(WAVE_1K_MAX) > t) t = max_tiles(WAVE_1K_MAX);
+  if (n > WAVE_2K_MAX && max_tiles(WAVE_2K_MAX) > t) t = max_tiles(WAVE_2K_MAX);
+  return t;
+}
 static constexpr bool tiles_covered() {
   for (const Variant& v : kVariants)
     if (v.kind != 5 && v.threads * v.kpt < 4096) return false;
@@ -1220,24 +1234,22 @@ static constexpr bool tiles_covered() {
 }
 static_assert(tiles_covered(), "only the limited one-wave variants have tiles below 4,096 keys");
 
+// Words in front of the look-back descriptors: header, counts, bin offsets.
+constexpr size_t SORT_FRONT_WORDS = (64 + 2 * (size_t)MAX_PASSES * RADIX + 63) / 64 * 64;
+
 size_t sort_workspace_bytes(uint32_t n, int passes, int /*tile_keys*/) {
-  const uint32_t tiles = ceil_div(n > 0 ? n : 1, (uint32_t)min_tile_keys(n));
-  size_t words = 64 + 2 * (size_t)MAX_PASSES * RADIX;  // header + counts + bin offsets
-  words = align_up(words, 64);
-  words += (size_t)passes * tiles * RADIX;
-  return align_up(words * 4, 256);
+  return align_up((SORT_FRONT_WORDS + (size_t)passes * max_tiles_up_to(n) * RADIX) * 4, 256);
 }
 
 SortWorkspace carve_sort_workspace(void* ws, uint32_t n, int passes, int /*tile_keys*/) {
   SortWorkspace W;
   uint32_t* p = reinterpret_cast<uint32_t*>(ws);
-  W.tiles = ceil_div(n > 0 ? n : 1, (uint32_t)min_tile_keys(n));
+  W.tiles = max_tiles(n);
   W.header = p;                              // [0] done, [1..8] tile counters
   W.counts = p + 64;                         // [passes][256]
   W.bin_offsets = p + 64 + MAX_PASSES * RADIX;
-  W.header_words = 64 + (size_t)MAX_PASSES * RADIX;  // header + counts zeroed per call
-  const size_t desc_off = align_up(64 + 2 * (size_t)MAX_PASSES * RADIX, 64);
-  W.desc = p + desc_off;
+  W.desc = p + SORT_FRONT_WORDS;             // [passes][tiles][256]
+  W.header_words = 64 + MAX_PASSES * RADIX;  // header + counts
   W.desc_words = (size_t)passes * W.tiles * RADIX;
   return W;
 }

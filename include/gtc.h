@@ -120,8 +120,9 @@ typedef enum gtc_op {
   GTC_OP_GLOBAL_HISTOGRAM = 5,
   GTC_OP_LEARNED_SORT = 6
 } gtc_op;
-/* Bytes of device workspace `op` needs for n elements of key_bits-wide keys.
- * Workspace pointers must be 256-byte aligned. */
+/* Bytes of device workspace `op` needs for up to n elements of key_bits-wide
+ * keys (never less for a larger n).  Workspace pointers must be 256-byte
+ * aligned. */
 GTC_API gtc_status gtc_workspace_size(gtc_ctx* ctx, gtc_op op, uint32_t n, int key_bits, size_t* bytes);
 
 /* ----------------------------------------------------- stage operators --- */
