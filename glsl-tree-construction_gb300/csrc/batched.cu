@@ -84,8 +84,15 @@ constexpr int kBtNumVariants = sizeof(kBtVariants) / sizeof(kBtVariants[0]);
 constexpr int BT_SMALL = 5, BT_LARGE = 6;
 constexpr uint32_t BT_SMALL_MAX = 600000;
 constexpr uint32_t BT_LARGE_MIN = 2000000;  // untuned batches from here on take variant 6
-// Smallest tile of any variant for n points: sizes the workspace.
-constexpr uint32_t bt_min_tile(uint32_t n) { return n <= BT_SMALL_MAX ? 2048 : 4096; }
+// Most whole tiles of any variant for n points, and for up to n points: a
+// workspace made for n also serves fewer, which may have more (short) tiles.
+constexpr uint32_t bt_tiles(uint32_t n) {
+  const uint32_t tile = n <= BT_SMALL_MAX ? 2048 : 4096;
+  return ((n > 0 ? n : 1) + tile - 1) / tile;
+}
+constexpr uint32_t bt_tiles_up_to(uint32_t n) {
+  return n > BT_SMALL_MAX && bt_tiles(n) < bt_tiles(BT_SMALL_MAX) ? bt_tiles(BT_SMALL_MAX) : bt_tiles(n);
+}
 constexpr uint32_t MAX_CLOUDS = 1u << 20;
 
 // Tiles per cloud and non-empty clouds, both scanned (one block).  The
@@ -797,9 +804,11 @@ struct BatchWs {
 };
 
 // A cloud of len points has ceil(len / TILE) tiles, so the batch has at most
-// n / TILE + S of them; sized for the smallest tile of any variant.
+// n / TILE + S of them, for the smallest tile of any variant.  Room is taken
+// for the tiles of up to n points, so the size never shrinks as n grows.
 size_t batch_layout(uint32_t n, uint32_t S, BatchWs* W, char* p) {
-  const uint32_t tiles_max = ceil_div(n > 0 ? n : 1, bt_min_tile(n)) + S;
+  const uint32_t tiles_max = bt_tiles(n) + S;
+  const uint32_t tiles_room = bt_tiles_up_to(n) + S;
   size_t o = 0;
   auto take = [&](size_t bytes) {
     char* q = p ? p + o : nullptr;
@@ -809,7 +818,7 @@ size_t batch_layout(uint32_t n, uint32_t S, BatchWs* W, char* p) {
   BatchWs w;
   w.tile_start = reinterpret_cast<uint32_t*>(take(((size_t)S + 1) * 4));
   w.ne_start = reinterpret_cast<uint32_t*>(take(((size_t)S + 1) * 4));
-  w.tile_cloud = reinterpret_cast<uint32_t*>(take((size_t)tiles_max * 4));
+  w.tile_cloud = reinterpret_cast<uint32_t*>(take((size_t)tiles_room * 4));
   const size_t zero_from = o;
   w.seg_hist = reinterpret_cast<uint32_t*>(take((size_t)S * BPASSES * BRADIX * 4));
   w.unique_ws = take(scan_workspace_bytes(n));
@@ -817,7 +826,7 @@ size_t batch_layout(uint32_t n, uint32_t S, BatchWs* W, char* p) {
   w.zero_vecs = (o - zero_from) / 16;
   w.counters = reinterpret_cast<uint32_t*>(take(256));
   w.desc_words = (size_t)BPASSES * tiles_max * BRADIX;
-  w.desc = reinterpret_cast<uint32_t*>(take(w.desc_words * 4));
+  w.desc = reinterpret_cast<uint32_t*>(take((size_t)BPASSES * tiles_room * BRADIX * 4));
   w.keys_alt = reinterpret_cast<uint32_t*>(take((size_t)n * 4));
   w.idx_alt = reinterpret_cast<uint32_t*>(take((size_t)n * 4));
   w.ps = reinterpret_cast<uint32_t*>(take((size_t)n * 4));

@@ -31,6 +31,15 @@ def test_workspace_never_shrinks(gtc_mod, op, key_bits):
         last = (n, b.value)
 
 
+@pytest.mark.parametrize("clouds", [1, 16, 64, 1000])
+def test_batched_workspace_never_shrinks(gtc_mod, clouds):
+    b, last = ctypes.c_size_t(), (0, 0)
+    for n in sizes_around((600_000,)):
+        assert gtc_mod.lib().gtc_batched_workspace_size(n, clouds, ctypes.byref(b)) == 0
+        assert b.value >= last[1], (n, last)
+        last = (n, b.value)
+
+
 # (capacity, items): the items' own workspace has more tiles than the capacity's.
 REUSE = [(170_000, 160_000), (180_000, 163_840), (190_000, 163_841), (420_000, 400_000), (440_000, 409_600),
          (440_000, 409_601)]
@@ -123,4 +132,24 @@ def test_learned_sort_with_a_larger_workspace(gtc_mod, cap, n):
     model.train(prior, stride=10)
     out = model.sort(keys, ws=c.workspace(gtc_mod.OP_LEARNED_SORT, cap, 64))
     assert torch.equal(out[0], prior)
+    c.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("cap,clouds_cap,n,clouds", [(600_001, 16, 600_000, 16), (640_000, 16, 600_000, 16),
+                                                     (640_000, 64, 599_999, 63), (640_000, 64, 600_001, 64)])
+def test_batch_plan_with_fewer_points(gtc_mod, oracle, cap, clouds_cap, n, clouds):
+    import torch
+
+    from test_gpu_pipeline import _cmp
+
+    c = gtc_mod.Context(0)
+    plan = gtc_mod.BatchPlan(c, cap, clouds_cap)
+    for m, s in ((cap, clouds_cap), (n, clouds)):
+        off = np.linspace(0, m, s + 1).astype(np.int64)
+        pts = W.gaussian_mixture_points(m, 8, 10.0, noise=0.2, seed=m + s)
+        plan.launch(torch.from_numpy(pts).cuda(), torch.from_numpy(off.astype(np.int32)).cuda())
+        for k, r in enumerate(plan.clouds()):
+            exp, _ = oracle.build_octree(np.ascontiguousarray(pts[off[k]:off[k + 1]]), 32, threads=8)
+            _cmp(r, exp, 32, (m, k))
     c.close()
