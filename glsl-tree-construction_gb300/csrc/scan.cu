@@ -33,8 +33,8 @@ size_t scan_workspace_bytes(uint32_t n) {
 // Launch to launch with the memset before it, node offsets and in-place unique
 // of 64-bit keys (us; before: the kernels below):
 //   items        node offsets   before      unique   before
-//   120,000          6.2          6.3          6.2      8.7
-//   1,048,576        8.2         11.4          8.8     17.3
+//   120,000          6.2          6.3          8.1      8.7
+//   1,048,576        8.2         11.4         10.5     17.3
 //   4,000,000       11.1         19.0           -      40.6
 // ROWS is the smallest that keeps the grid within one block per SM (unique) or
 // 5/8 of one (the scan, whose blocks all arrive at their wait together): every
@@ -114,15 +114,19 @@ __global__ void __launch_bounds__(CS_THREADS) row_scan_kernel(const uint32_t* in
 }
 
 // Unique.  A row is 32 keys.  In place (kin == kout) too: a block writes only
-// below the end of its own input, after every lower block has posted its
-// total, and a block posts only after all its keys and values have arrived
-// (IN_PLACE makes the barrier before the post depend on the values; the count
-// depends on the keys).  A block's first key's predecessor may be rewritten by
-// its own block only with the same key (no key before it dropped).
+// below the end of its own input, at places that depend on every lower block's
+// total, and a total depends on every key and value that its block has loaded:
+// on the keys by the count, on the values by `zero`, which is 0 at run time,
+// unknown to the compiler (a test of the values that the compiler can see to
+// be false goes away, and the dependence with it).  Fences in place of the
+// dependence, a release at the post and an acquire behind the polls, cost 2 us
+// more (u64 pairs, 120,000 10.2 against 8.2 us, 1M 12.4 against 10.5).  A
+// block's first key's predecessor may be rewritten by its own block only with
+// the same key (no key before it dropped).
 template <class K, bool HAS_VALS, int ROWS, bool IN_PLACE>
 __global__ void __launch_bounds__(CS_THREADS) row_unique_kernel(const K* kin, const uint32_t* vin, K* kout,
                                                                 uint32_t* vout, uint32_t n, uint32_t* ws,
-                                                                uint32_t* d_count, uint32_t* status) {
+                                                                uint32_t* d_count, uint32_t* status, uint32_t zero) {
   griddep_wait();
   __shared__ uint32_t s_seg[CS_WARPS];
   __shared__ uint32_t s_red[CS_WARPS];
@@ -149,13 +153,13 @@ __global__ void __launch_bounds__(CS_THREADS) row_unique_kernel(const K* kin, co
     cnt += __popc(__ballot_sync(0xffffffffu, kp));
     carry = (K)__shfl_sync(0xffffffffu, k[j], 31);
   }
-  if (lane == 0) s_seg[warp] = cnt;
   if (IN_PLACE && HAS_VALS) {
     uint32_t x = 0;
 #pragma unroll
     for (int j = 0; j < ROWS; ++j) x |= v[j];
-    if (__syncthreads_or(x == ~0u && cnt > 32u * ROWS)) return;  // never taken (a warp keeps at most its keys)
+    cnt += __reduce_or_sync(0xffffffffu, x & zero);
   }
+  if (lane == 0) s_seg[warp] = cnt;
   uint32_t run = cs_block_prefix(ws + 64, s_seg, s_red, status) + s_seg[warp];
 #pragma unroll
   for (int j = 0; j < ROWS; ++j) {
@@ -510,7 +514,7 @@ static bool launch_row_unique(const Launch& L, const K* kin, const uint32_t* vin
   }
   *e = L.ws_zeroed ? cudaSuccess : cudaMemsetAsync(w, 0, (64 + (size_t)g) * 4, L.stream);
   if (*e == cudaSuccess)
-    *e = launch_kernel(L, kern, g, CS_THREADS, 0, kin, vin, kout, vout, n, w, d_count, L.status);
+    *e = launch_kernel(L, kern, g, CS_THREADS, 0, kin, vin, kout, vout, n, w, d_count, L.status, 0u);
   return true;
 }
 
