@@ -181,7 +181,7 @@ __device__ __forceinline__ TileRange tile_range(uint32_t t, uint32_t cloud, cons
 // when the cloud changes: the 1,024 global atomics of a flush cost as much as
 // the tile's points.
 template <int Q>
-__global__ void __launch_bounds__(BM_THREADS) bt_morton_kernel(const float4* __restrict__ pts, const uint32_t* off,
+__global__ void __launch_bounds__(BM_THREADS) bt_morton_kernel(const float4* pts, const uint32_t* off,
                                                                uint32_t S, const uint32_t* tile_start, uint32_t tile,
                                                                uint32_t group, float mn, float rg, float inv_rg,
                                                                uint32_t* __restrict__ keys, uint32_t* tile_cloud,
@@ -284,8 +284,8 @@ struct BtSmem {
 // the next tile starts another cloud and does not look back.  FIRST: the
 // payload is the point's index in its cloud, made here.
 template <int THREADS, int KPT, int MINB, bool FIRST, bool SCANNED>
-__global__ void __launch_bounds__(THREADS, MINB) bt_onesweep_kernel(const uint32_t* __restrict__ kin,
-                                                                 const uint32_t* __restrict__ vin,
+__global__ void __launch_bounds__(THREADS, MINB) bt_onesweep_kernel(const uint32_t* kin,
+                                                                 const uint32_t* vin,
                                                                  uint32_t* __restrict__ kout,
                                                                  uint32_t* __restrict__ vout, const uint32_t* off,
                                                                  uint32_t S, const uint32_t* tile_start,
@@ -433,8 +433,8 @@ __device__ __forceinline__ void bt_record_end(const uint32_t* off, uint32_t S, u
 }
 
 template <int ROWS>
-__global__ void __launch_bounds__(CS_THREADS) bt_row_unique_kernel(const uint32_t* __restrict__ kin,
-                                                                   const uint32_t* __restrict__ vin,
+__global__ void __launch_bounds__(CS_THREADS) bt_row_unique_kernel(const uint32_t* kin,
+                                                                   const uint32_t* vin,
                                                                    uint32_t* __restrict__ kout,
                                                                    uint32_t* __restrict__ vout, uint32_t n,
                                                                    const uint32_t* off, uint32_t S, uint32_t* uoff,
@@ -490,8 +490,8 @@ __global__ void __launch_bounds__(CS_THREADS) bt_row_unique_kernel(const uint32_
 
 // Segments of any length, read twice (scan.cu's chunk_unique_kernel), eight
 // rows in flight per warp.
-__global__ void __launch_bounds__(CS_THREADS) bt_chunk_unique_kernel(const uint32_t* __restrict__ kin,
-                                                                     const uint32_t* __restrict__ vin,
+__global__ void __launch_bounds__(CS_THREADS) bt_chunk_unique_kernel(const uint32_t* kin,
+                                                                     const uint32_t* vin,
                                                                      uint32_t* __restrict__ kout,
                                                                      uint32_t* __restrict__ vout, uint32_t n,
                                                                      const uint32_t* off, uint32_t S, uint32_t* uoff,
@@ -579,7 +579,7 @@ __global__ void __launch_bounds__(CS_THREADS) bt_chunk_unique_kernel(const uint3
 }
 
 // Radix tree of every cloud, one thread per unique code.
-__global__ void __launch_bounds__(256) bt_tree_kernel(const uint32_t* __restrict__ codes, const uint32_t* uoff,
+__global__ void __launch_bounds__(256) bt_tree_kernel(const uint32_t* codes, const uint32_t* uoff,
                                                       uint32_t S, uint8_t* prefix_n, uint8_t* hll, uint8_t* hlr,
                                                       int32_t* left, int32_t* parent, uint32_t* edge) {
   griddep_wait();
@@ -640,7 +640,7 @@ __global__ void bt_cloud_offsets_kernel(uint32_t* uoff, const uint32_t* ne_start
 // (octree_warp_batch), each lane with its own cloud.
 constexpr int BT_OCT_THREADS = 256;
 
-__global__ void __launch_bounds__(BT_OCT_THREADS) bt_octree_kernel(const uint32_t* __restrict__ codes,
+__global__ void __launch_bounds__(BT_OCT_THREADS) bt_octree_kernel(const uint32_t* codes,
                                                                    const uint32_t* uoff, uint32_t S,
                                                                    const uint4* cinfo, const uint8_t* prefix_n,
                                                                    const uint8_t* hll, const uint8_t* hlr,

@@ -80,18 +80,18 @@ __device__ __forceinline__ uint64_t l2_drop_policy() {
 }
 __device__ __forceinline__ uint32_t ld_hint(const uint32_t* p, uint64_t pol) {
   uint32_t v;
-  asm volatile("ld.global.nc.L2::cache_hint.u32 %0, [%1], %2;" : "=r"(v) : "l"(p), "l"(pol));
+  asm volatile("ld.global.L2::cache_hint.u32 %0, [%1], %2;" : "=r"(v) : "l"(p), "l"(pol));
   return v;
 }
 __device__ __forceinline__ uint64_t ld_hint(const uint64_t* p, uint64_t pol) {
   uint64_t v;
-  asm volatile("ld.global.nc.L2::cache_hint.u64 %0, [%1], %2;" : "=l"(v) : "l"(p), "l"(pol));
+  asm volatile("ld.global.L2::cache_hint.u64 %0, [%1], %2;" : "=l"(v) : "l"(p), "l"(pol));
   return v;
 }
 
 __device__ __forceinline__ uint4 ld_hint(const uint4* p, uint64_t pol) {
   uint4 v;
-  asm volatile("ld.global.nc.L2::cache_hint.v4.u32 {%0, %1, %2, %3}, [%4], %5;"
+  asm volatile("ld.global.L2::cache_hint.v4.u32 {%0, %1, %2, %3}, [%4], %5;"
                : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
                : "l"(p), "l"(pol));
   return v;
@@ -424,7 +424,10 @@ struct Launch {
 // Start of every kernel that may run under a programmatic dependent launch:
 // wait until the previous grid has completed and its writes are visible
 // (a no-op for a normal launch), then let the next grid's blocks be
-// scheduled.
+// scheduled.  Such a kernel's grid overlaps the one that writes its inputs, so
+// it reads them with plain loads: a non-coherent load (__ldg, or what the
+// compiler makes of a const pointer marked __restrict__) is for memory that
+// does not change while the kernel runs, and need not stay behind the wait.
 __device__ __forceinline__ void griddep_wait() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

@@ -268,10 +268,10 @@ __device__ __forceinline__ int leaf_bucket(uint64_t key, uint32_t leaf, const ui
   return pwl_bucket(key, k0, k1, s_y[seg], s_y[seg + 1], B);
 }
 
-__global__ void __launch_bounds__(LC_THREADS, 1) learned_count_kernel(const uint64_t* __restrict__ keys, uint32_t n,
-                                                                      const uint64_t* __restrict__ eytz,
-                                                                      const uint64_t* __restrict__ kn,
-                                                                      const float* __restrict__ y, int B,
+__global__ void __launch_bounds__(LC_THREADS, 1) learned_count_kernel(const uint64_t* keys, uint32_t n,
+                                                                      const uint64_t* eytz,
+                                                                      const uint64_t* kn,
+                                                                      const float* y, int B,
                                                                       uint32_t* totals, uint16_t* __restrict__ bids,
                                                                       uint32_t* flags) {
   griddep_wait();
@@ -447,9 +447,9 @@ struct LpSmem {
 
 template <bool FIRST, int THREADS, int KPT, int MINB>
 __global__ void __launch_bounds__(THREADS, MINB) learned_pass_kernel(
-    const uint64_t* __restrict__ kin, const uint32_t* __restrict__ vin, const uint16_t* __restrict__ bin,
+    const uint64_t* kin, const uint32_t* vin, const uint16_t* bin,
     uint64_t* __restrict__ kout, uint32_t* __restrict__ vout, uint16_t* __restrict__ bout, uint32_t n, int shift,
-    uint32_t mask, const uint32_t* __restrict__ bin_off, uint32_t* __restrict__ desc, uint32_t* status,
+    uint32_t mask, const uint32_t* bin_off, uint32_t* __restrict__ desc, uint32_t* status,
     const uint32_t* flags) {
   griddep_wait();
   if (*flags & (LFLAG_OVERFLOW | LFLAG_BAD_MODEL)) return;
@@ -760,7 +760,7 @@ __device__ __forceinline__ int bucket_sort_body(BucketSmem& s, uint32_t cnt, int
 // longer run sends the bucket through full passes over all its varying bits
 // instead.
 __global__ void __launch_bounds__(BS_THREADS, 2) bucket_sort_kernel(
-    const uint64_t* __restrict__ ukeys, const uint32_t* __restrict__ uvals, const uint32_t* base,
+    const uint64_t* ukeys, const uint32_t* uvals, const uint32_t* base,
     const uint32_t* totals, uint64_t* __restrict__ out_keys, uint32_t* __restrict__ out_vals, uint64_t* bmin,
     uint64_t* bmax, uint32_t* flags) {
   griddep_wait();

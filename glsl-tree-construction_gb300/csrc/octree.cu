@@ -15,13 +15,13 @@ constexpr int OCT_THREADS = 256;
 // of them (octree_warp_batch: breadth-first descents, every lane busy).  No
 // block barriers; 16-byte stores straight to HBM.
 template <class K, bool WITH_LEAVES>
-__global__ void __launch_bounds__(OCT_THREADS) octree_make_kernel(const K* __restrict__ codes, const uint32_t* d_u,
-                                                                  uint32_t u_host, const uint8_t* __restrict__ prefix_n,
-                                                                  const uint8_t* __restrict__ hll,
-                                                                  const uint8_t* __restrict__ hlr,
-                                                                  const int32_t* __restrict__ left,
-                                                                  const uint32_t* __restrict__ edge,
-                                                                  const uint32_t* __restrict__ ps, float mn, float rg,
+__global__ void __launch_bounds__(OCT_THREADS) octree_make_kernel(const K* codes, const uint32_t* d_u,
+                                                                  uint32_t u_host, const uint8_t* prefix_n,
+                                                                  const uint8_t* hll,
+                                                                  const uint8_t* hlr,
+                                                                  const int32_t* left,
+                                                                  const uint32_t* edge,
+                                                                  const uint32_t* ps, float mn, float rg,
                                                                   gtc_octnode* __restrict__ nodes, uint32_t capacity,
                                                                   uint32_t lmask_keep, uint32_t* status) {
   griddep_wait();

@@ -132,10 +132,10 @@ struct OctCloud {
 
 template <class K, bool WITH_LEAVES>
 __device__ __forceinline__ void octree_warp_batch(OctWarp& S, bool valid, uint32_t k, const OctCloud& cl,
-                                                  const K* __restrict__ codes, const uint8_t* __restrict__ prefix_n,
-                                                  const uint8_t* __restrict__ hll, const uint8_t* __restrict__ hlr,
-                                                  const int32_t* __restrict__ left, const uint32_t* __restrict__ edge,
-                                                  const uint32_t* __restrict__ ps, float mn, float rg,
+                                                  const K* codes, const uint8_t* prefix_n,
+                                                  const uint8_t* hll, const uint8_t* hlr,
+                                                  const int32_t* left, const uint32_t* edge,
+                                                  const uint32_t* ps, float mn, float rg,
                                                   uint32_t lmask_keep, uint32_t* status) {
   constexpr int A = KeyTraits<K>::A;
   const int lane = threadIdx.x & 31;

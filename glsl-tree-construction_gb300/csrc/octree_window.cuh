@@ -85,10 +85,10 @@ __device__ __forceinline__ void ow_sync() { asm volatile("bar.sync 1, 480;" ::: 
 // offsets (ps minus the bias) are written here.
 template <class K, bool SEG>
 __global__ void __launch_bounds__(OW_THREADS + 32, 3) octree_window_kernel(
-    const K* __restrict__ codes, const uint32_t* d_u, const uint32_t* __restrict__ uoff, uint32_t S,
-    const uint4* __restrict__ cinfo, const uint32_t* __restrict__ rec, const uint8_t* __restrict__ prefix_n,
-    const uint8_t* __restrict__ hll, const uint8_t* __restrict__ hlr, const int32_t* __restrict__ left,
-    const uint32_t* __restrict__ edge, const uint32_t* __restrict__ ps, uint32_t* __restrict__ node_offsets, float mn,
+    const K* codes, const uint32_t* d_u, const uint32_t* uoff, uint32_t S,
+    const uint4* cinfo, const uint32_t* rec, const uint8_t* prefix_n,
+    const uint8_t* hll, const uint8_t* hlr, const int32_t* left,
+    const uint32_t* edge, const uint32_t* ps, uint32_t* __restrict__ node_offsets, float mn,
     float rg, gtc_octnode* __restrict__ nodes, uint32_t capacity, uint32_t lmask_keep, uint32_t* status) {
   griddep_wait();
   constexpr int A = KeyTraits<K>::A;
@@ -161,18 +161,18 @@ __global__ void __launch_bounds__(OW_THREADS + 32, 3) octree_window_kernel(
 #pragma unroll
       for (int q = 0; q < OW_PER; ++q) {
         const uint32_t x = (uint32_t)(w0 + q * OW_THREADS + tid);
-        r[q] = __ldg(rec + x);
-        pv[q] = __ldg(ps + x);
-        cx[q] = __ldg(codes + x);
+        r[q] = rec[x];
+        pv[q] = ps[x];
+        cx[q] = codes[x];
       }
     } else {
 #pragma unroll
       for (int q = 0; q < OW_PER; ++q) {
         const int x = w0 + q * OW_THREADS + tid;
         const bool in = x >= 0 && x < (int)U;
-        r[q] = in && (SEG || x < m) ? __ldg(rec + x) : SPLIT_NONE;
-        pv[q] = in ? __ldg(ps + x) : 0u;
-        cx[q] = in ? __ldg(codes + x) : K(0);
+        r[q] = in && (SEG || x < m) ? rec[x] : SPLIT_NONE;
+        pv[q] = in ? ps[x] : 0u;
+        cx[q] = in ? codes[x] : K(0);
       }
     }
     if (tid == 0) {

@@ -205,7 +205,7 @@ static uint32_t row_grid(const Launch& L, const void* kern, uint32_t n, uint32_t
 // Inclusive scan with the node-offset rules of scan_kernel.  Rows of 128
 // items (one uint4 per lane); S is a multiple of 128, so rows never straddle
 // segments and in/out must be 16-byte aligned.
-__global__ void __launch_bounds__(CS_THREADS) chunk_scan_kernel(const uint32_t* __restrict__ in,
+__global__ void __launch_bounds__(CS_THREADS) chunk_scan_kernel(const uint32_t* in,
                                                                 uint32_t* __restrict__ out, uint32_t count_host,
                                                                 const uint32_t* d_u, int node_offsets, uint32_t* ws,
                                                                 uint32_t* d_o, uint32_t* status) {
@@ -293,8 +293,8 @@ __global__ void __launch_bounds__(CS_THREADS) chunk_scan_kernel(const uint32_t* 
 // may land on input not yet re-read).  Rows of 32 keys; keep = first key or
 // different from its predecessor; kept keys of a row are written contiguously.
 template <class K, bool HAS_VALS>
-__global__ void __launch_bounds__(CS_THREADS) chunk_unique_kernel(const K* __restrict__ kin,
-                                                                  const uint32_t* __restrict__ vin,
+__global__ void __launch_bounds__(CS_THREADS) chunk_unique_kernel(const K* kin,
+                                                                  const uint32_t* vin,
                                                                   K* __restrict__ kout, uint32_t* __restrict__ vout,
                                                                   uint32_t n, uint32_t* ws, uint32_t* d_count,
                                                                   uint32_t* status) {

@@ -131,7 +131,7 @@ __device__ __forceinline__ void zero_region(uint32_t* p, size_t words) {
 }
 
 template <class K, int THREADS>
-__global__ void __launch_bounds__(THREADS) global_hist_kernel(const K* __restrict__ keys, uint32_t n, int begin_bit,
+__global__ void __launch_bounds__(THREADS) global_hist_kernel(const K* keys, uint32_t n, int begin_bit,
                                                               int end_bit, int passes, int db, uint32_t* counts,
                                                               uint32_t* bin_offsets, uint32_t* done,
                                                               uint32_t* zero_ptr, size_t zero_words,
@@ -177,7 +177,7 @@ __device__ __forceinline__ void hist_add_code(uint32_t (*s_hist)[RADIX], K k) {
 // the points once and leaves the sort ready to run (its first pass makes
 // the index payload itself).
 template <class K, int THREADS, int Q, int LB>
-__global__ void __launch_bounds__(THREADS, 3) morton_hist_kernel(const float4* __restrict__ pts, K* __restrict__ keys,
+__global__ void __launch_bounds__(THREADS, 3) morton_hist_kernel(const float4* pts, K* __restrict__ keys,
                                                               uint32_t n, float mn, float rg, float inv_rg,
                                                               uint32_t* counts, uint32_t* bin_offsets, uint32_t* done,
                                                               uint32_t* zero_ptr, size_t zero_words, uint32_t* zero4) {
@@ -497,10 +497,10 @@ struct OnesweepSmem {
 
 template <class K, int THREADS, int KPT, bool HAS_VALS, int MINB, int LBW, int RANK, bool L2H = false,
           bool TICKET = false>
-__global__ void __launch_bounds__(THREADS, MINB) onesweep_kernel(const K* __restrict__ kin, const uint32_t* __restrict__ vin,
+__global__ void __launch_bounds__(THREADS, MINB) onesweep_kernel(const K* kin, const uint32_t* vin,
                                                            K* __restrict__ kout, uint32_t* __restrict__ vout,
                                                            uint32_t n, int shift, uint32_t dmask,
-                                                           const uint32_t* __restrict__ bin_off,
+                                                           const uint32_t* bin_off,
                                                            uint32_t* __restrict__ desc,
                                                            uint32_t* __restrict__ tile_counter,
                                                            uint32_t* __restrict__ status,
@@ -739,13 +739,13 @@ __global__ void __launch_bounds__(THREADS, MINB) onesweep_kernel(const K* __rest
 // and 64.9 against 52.6 for 1M, by this kernel and onesweep_kernel.)
 // first_tile: 1 leaves tile 0 unsorted (gtc_debug_skip_first_tile).
 template <class K, int THREADS, int KPT, bool HAS_VALS>
-__global__ void __launch_bounds__(THREADS) onesweep_wave_kernel(const K* __restrict__ kin,
-                                                                const uint32_t* __restrict__ vin,
+__global__ void __launch_bounds__(THREADS) onesweep_wave_kernel(const K* kin,
+                                                                const uint32_t* vin,
                                                                 K* __restrict__ kout, uint32_t* __restrict__ vout,
                                                                 uint32_t n, int shift, uint32_t dmask,
-                                                                const uint32_t* __restrict__ bin_off,
+                                                                const uint32_t* bin_off,
                                                                 uint32_t* __restrict__ desc,
-                                                                const uint32_t* __restrict__ first_tile,
+                                                                const uint32_t* first_tile,
                                                                 uint32_t* __restrict__ status,
                                                                 const uint32_t* run_if) {
   griddep_wait();
@@ -873,10 +873,10 @@ __device__ __forceinline__ uint32_t peer_mask(uint32_t d) {
 }
 
 template <class K, int THREADS, int KPT, bool HV, bool MATCH>
-__global__ void __launch_bounds__(THREADS, (THREADS <= 256 ? 2 : 1)) onesweep_tma_kernel(const K* __restrict__ kin,
-                                                               const uint32_t* __restrict__ vin, K* __restrict__ kout,
+__global__ void __launch_bounds__(THREADS, (THREADS <= 256 ? 2 : 1)) onesweep_tma_kernel(const K* kin,
+                                                               const uint32_t* vin, K* __restrict__ kout,
                                                                uint32_t* __restrict__ vout, uint32_t n, int shift,
-                                                               uint32_t dmask, const uint32_t* __restrict__ bin_off,
+                                                               uint32_t dmask, const uint32_t* bin_off,
                                                                uint32_t* __restrict__ desc,
                                                                uint32_t* __restrict__ tile_counter,
                                                                uint32_t* __restrict__ status,

@@ -444,7 +444,7 @@ __device__ __forceinline__ void tw_warp_split(const K* codes, uint32_t x, uint32
 // (nullable) receives every split's record (split_rec.cuh).
 template <class K, bool SEG, class SH>
 __global__ void __launch_bounds__(TW_THREADS, SH::MINB) radix_tree_window_kernel(
-    const K* __restrict__ codes, const uint32_t* d_u, uint32_t u_host, const uint32_t* uoff, uint32_t S,
+    const K* codes, const uint32_t* d_u, uint32_t u_host, const uint32_t* uoff, uint32_t S,
     uint8_t* __restrict__ prefix_n, uint8_t* __restrict__ hll, uint8_t* __restrict__ hlr,
     int32_t* __restrict__ left, int32_t* __restrict__ parent, uint32_t* __restrict__ edge, uint32_t* d_m,
     uint32_t* __restrict__ rec) {
@@ -473,27 +473,27 @@ __global__ void __launch_bounds__(TW_THREADS, SH::MINB) radix_tree_window_kernel
     if (vec && x >= 0 && x + 4 <= (int)P) {
       K c[5];
       if (sizeof(K) == 8) {
-        const uint4 q0 = __ldg(reinterpret_cast<const uint4*>(codes + x));
-        const uint4 q1 = __ldg(reinterpret_cast<const uint4*>(codes + x + 2));
+        const uint4 q0 = *reinterpret_cast<const uint4*>(codes + x);
+        const uint4 q1 = *reinterpret_cast<const uint4*>(codes + x + 2);
         c[0] = (K)(q0.x | ((uint64_t)q0.y << 32));
         c[1] = (K)(q0.z | ((uint64_t)q0.w << 32));
         c[2] = (K)(q1.x | ((uint64_t)q1.y << 32));
         c[3] = (K)(q1.z | ((uint64_t)q1.w << 32));
       } else {
-        const uint4 q0 = __ldg(reinterpret_cast<const uint4*>(codes + x));
+        const uint4 q0 = *reinterpret_cast<const uint4*>(codes + x);
         c[0] = (K)q0.x;
         c[1] = (K)q0.y;
         c[2] = (K)q0.z;
         c[3] = (K)q0.w;
       }
-      c[4] = __ldg(codes + x + 4);
+      c[4] = codes[x + 4];
 #pragma unroll
       for (int e = 0; e < 4; ++e) v |= (uint32_t)delta_key(c[e], c[e + 1]) << (8 * e);
     } else {
 #pragma unroll
       for (int e = 0; e < 4; ++e)
         if (x + e >= 0 && x + e < (int)P)
-          v |= (uint32_t)delta_key(__ldg(codes + x + e), __ldg(codes + x + e + 1)) << (8 * e);
+          v |= (uint32_t)delta_key(codes[x + e], codes[x + e + 1]) << (8 * e);
     }
     reinterpret_cast<uint32_t*>(s.d)[g] = v;
   }
