@@ -215,7 +215,8 @@ __global__ void __launch_bounds__(BM_THREADS) bt_morton_kernel(const float4* pts
   for (uint32_t t = t0; t < min(t0 + group, tiles); ++t) {  // block-uniform
     if (t >= tile_start[cloud + 1]) {
       flush();
-      while (t >= tile_start[cloud + 1]) ++cloud;  // skips empty clouds
+      ++cloud;
+      if (t >= tile_start[cloud + 1]) cloud = warp_upper_bound_u32(tile_start, S + 1, t) - 1;  // empty clouds between
     }
     if (tid == 0) tile_cloud[t] = cloud;
     const TileRange r = tile_range(t, cloud, tile_start, off, tile);
@@ -406,30 +407,53 @@ __device__ __forceinline__ BtStarts bt_starts_from(const uint32_t* off, uint32_t
   const uint32_t c = r > 0 ? warp_upper_bound_u32(off, S + 1, r - 1) : 0u;
   return BtStarts{c, c <= S ? off[c] : ~0u};
 }
-// The cloud starts in [r, r + 32) as a mask; steps past them.
-__device__ __forceinline__ uint32_t bt_row_starts(const uint32_t* off, uint32_t S, uint32_t r, BtStarts& st) {
-  uint32_t smask = 0;
-  while (st.cloud < S && st.at < r + 32) {  // warp-uniform
-    smask |= 1u << (st.at - r);
-    ++st.cloud;
-    st.at = off[st.cloud];
+// The cloud starts in rows [r0, end) as masks, row j's in lane j; steps past
+// them, 32 clouds at a time, and past the rest of a long run of empty clouds by
+// search (whole warp).  RECORD: writes their U_c instead, with row j's kept
+// mask and first output position in lane j.  One loop over the rows that clouds
+// start in, outside the caller's unrolled ones, which it would fill with code.
+template <bool RECORD>
+__device__ __forceinline__ uint32_t bt_starts(const uint32_t* off, uint32_t S, uint32_t r0, uint32_t end, BtStarts& st,
+                                              uint32_t bals, uint32_t runs, uint32_t* uoff) {
+  const uint32_t lane = threadIdx.x & 31;
+  uint32_t masks = 0;
+#pragma unroll 1
+  while (st.cloud < S && st.at < end) {  // warp-uniform
+    const uint32_t j = (st.at - r0) / 32, r = r0 + 32 * j;
+    const uint32_t c = st.cloud + lane;
+    const uint32_t p = off[min(c, S)];
+    const bool in = c < S && p < r + 32;
+    const uint32_t k = __popc(__ballot_sync(0xffffffffu, in));  // a prefix of the lanes, of one at least
+    uint32_t bal = 0, run = 0;
+    if (RECORD) {
+      bal = __shfl_sync(0xffffffffu, bals, j);
+      run = __shfl_sync(0xffffffffu, runs, j);
+      if (in) uoff[c] = run + __popc(bal & ((1u << (p - r)) - 1u));
+    } else {
+      const uint32_t m = __reduce_or_sync(0xffffffffu, in ? 1u << (p - r) : 0u);
+      if (lane == j) masks |= m;
+    }
+    st.cloud += k;
+    if (k < 32) {
+      st.at = __shfl_sync(0xffffffffu, p, k);
+    } else {
+      const uint32_t last = __shfl_sync(0xffffffffu, p, 31);
+      st.at = off[st.cloud];
+      if (st.at == last) {
+        const uint32_t c0 = st.cloud;
+        st.cloud += warp_upper_bound_u32(off + c0, S - c0, last);
+        if (RECORD) {
+          for (uint32_t q = c0 + lane; q < st.cloud; q += 32) uoff[q] = run + __popc(bal & ((1u << (last - r)) - 1u));
+        }
+        st.at = off[st.cloud];
+      }
+    }
   }
-  return smask;
+  return masks;
 }
-// Records U_c of the clouds that start in [r, r + 32), and steps past them:
-// bal is the row's kept mask, run its first output position.
-__device__ __forceinline__ void bt_row_record(const uint32_t* off, uint32_t S, uint32_t r, BtStarts& st, uint32_t bal,
-                                              uint32_t run, uint32_t* uoff) {
-  while (st.cloud < S && st.at < r + 32) {
-    if ((threadIdx.x & 31) == 0) uoff[st.cloud] = run + __popc(bal & ((1u << (st.at - r)) - 1u));
-    ++st.cloud;
-    st.at = off[st.cloud];
-  }
-}
-// Past the last row: U_S and the empty clouds behind the last code (lane 0).
-__device__ __forceinline__ void bt_record_end(const uint32_t* off, uint32_t S, uint32_t run, uint32_t* uoff) {
-  uoff[S] = run;
-  for (uint32_t c = S; c > 0 && off[c - 1] == off[S]; --c) uoff[c - 1] = run;
+// Past the last row: the empty clouds behind it, from cloud c on, and U_S (whole warp).
+__device__ __forceinline__ void bt_record_end(uint32_t c, uint32_t S, uint32_t run, uint32_t* uoff) {
+  for (c += threadIdx.x & 31; c <= S; c += 32) uoff[c] = run;
 }
 
 template <int ROWS>
@@ -457,11 +481,12 @@ __global__ void __launch_bounds__(CS_THREADS) bt_row_unique_kernel(const uint32_
   uint32_t carry = (lane == 0 && r0 > 0 && r0 < n) ? kin[r0 - 1] : 0u;
   const BtStarts first = bt_starts_from(off, S, min(r0, n));
   BtStarts st = first;
+  const uint32_t masks = bt_starts<false>(off, S, r0, min(r0 + ROWS * 32, n), st, 0u, 0u, nullptr);
   uint32_t keep = 0, cnt = 0;
 #pragma unroll
   for (int j = 0; j < ROWS; ++j) {
-    const uint32_t r = r0 + j * 32, i = r + lane;
-    const uint32_t smask = r < n ? bt_row_starts(off, S, r, st) : 0u;
+    const uint32_t i = r0 + j * 32 + lane;
+    const uint32_t smask = __shfl_sync(0xffffffffu, masks, j);
     uint32_t prev = __shfl_up_sync(0xffffffffu, k[j], 1);
     if (lane == 0) prev = carry;
     const bool kp = i < n && (k[j] != prev || ((smask >> lane) & 1u));
@@ -471,10 +496,9 @@ __global__ void __launch_bounds__(CS_THREADS) bt_row_unique_kernel(const uint32_
   }
   if (lane == 0) s_seg[warp] = cnt;
   uint32_t run = cs_block_prefix(ws + 64, s_seg, s_red, status) + s_seg[warp];
-  st = first;
+  uint32_t bals = 0, runs = 0;
 #pragma unroll
   for (int j = 0; j < ROWS; ++j) {
-    const uint32_t r = r0 + j * 32;
     const bool kp = (keep >> j) & 1u;
     const uint32_t bal = __ballot_sync(0xffffffffu, kp);
     if (kp) {
@@ -482,15 +506,20 @@ __global__ void __launch_bounds__(CS_THREADS) bt_row_unique_kernel(const uint32_
       kout[o] = k[j];
       vout[o] = v[j];
     }
-    if (r < n) bt_row_record(off, S, r, st, bal, run, uoff);
+    if (lane == j) {
+      bals = bal;
+      runs = run;
+    }
     run += __popc(bal);
   }
-  if (blockIdx.x == gridDim.x - 1 && warp == CS_WARPS - 1 && lane == 0) bt_record_end(off, S, run, uoff);
+  st = first;
+  bt_starts<true>(off, S, r0, min(r0 + ROWS * 32, n), st, bals, runs, uoff);
+  if (blockIdx.x == gridDim.x - 1 && warp == CS_WARPS - 1) bt_record_end(st.cloud, S, run, uoff);
 }
 
 // Segments of any length, read twice (scan.cu's chunk_unique_kernel), eight
 // rows in flight per warp.
-__global__ void __launch_bounds__(CS_THREADS) bt_chunk_unique_kernel(const uint32_t* kin,
+__global__ void __launch_bounds__(CS_THREADS, 3) bt_chunk_unique_kernel(const uint32_t* kin,
                                                                      const uint32_t* vin,
                                                                      uint32_t* __restrict__ kout,
                                                                      uint32_t* __restrict__ vout, uint32_t n,
@@ -525,10 +554,11 @@ __global__ void __launch_bounds__(CS_THREADS) bt_chunk_unique_kernel(const uint3
         const uint32_t i = r0 + 32 * j + lane;
         k[j] = i < end ? ld_hint(kin + i, keep_pol) : 0u;
       }
+      const uint32_t masks = bt_starts<false>(off, S, r0, min(r0 + 32 * R, end), st, 0u, 0u, nullptr);
 #pragma unroll
       for (int j = 0; j < R; ++j) {
-        const uint32_t r = r0 + 32 * j, i = r + lane;
-        const uint32_t smask = r < end ? bt_row_starts(off, S, r, st) : 0u;
+        const uint32_t i = r0 + 32 * j + lane;
+        const uint32_t smask = __shfl_sync(0xffffffffu, masks, j);
         uint32_t prev = __shfl_up_sync(0xffffffffu, k[j], 1);
         if (lane == 0) prev = carry;
         cnt += __popc(__ballot_sync(0xffffffffu, i < end && (k[j] != prev || ((smask >> lane) & 1u))));
@@ -543,9 +573,9 @@ __global__ void __launch_bounds__(CS_THREADS) bt_chunk_unique_kernel(const uint3
   run += s_seg[warp];
 
   // 3. rescan and write, recording every cloud's U_c
+  BtStarts st = first;
   {
     uint32_t carry = first_prev;
-    BtStarts st = first;
     for (uint32_t r0 = beg; r0 < end; r0 += 32 * R) {
       uint32_t k[R], v[R];
 #pragma unroll
@@ -554,11 +584,13 @@ __global__ void __launch_bounds__(CS_THREADS) bt_chunk_unique_kernel(const uint3
         k[j] = i < end ? ld_hint(kin + i, drop_pol) : 0u;
         v[j] = i < end ? ld_hint(vin + i, drop_pol) : 0u;
       }
+      BtStarts here = st;
+      const uint32_t masks = bt_starts<false>(off, S, r0, min(r0 + 32 * R, end), here, 0u, 0u, nullptr);
+      uint32_t bals = 0, runs = 0;
 #pragma unroll
       for (int j = 0; j < R; ++j) {
-        const uint32_t r = r0 + 32 * j, i = r + lane;
-        BtStarts here = st;
-        const uint32_t smask = r < end ? bt_row_starts(off, S, r, st) : 0u;
+        const uint32_t i = r0 + 32 * j + lane;
+        const uint32_t smask = __shfl_sync(0xffffffffu, masks, j);
         uint32_t prev = __shfl_up_sync(0xffffffffu, k[j], 1);
         if (lane == 0) prev = carry;
         const bool kp = i < end && (k[j] != prev || ((smask >> lane) & 1u));
@@ -568,14 +600,18 @@ __global__ void __launch_bounds__(CS_THREADS) bt_chunk_unique_kernel(const uint3
           kout[o] = k[j];
           vout[o] = v[j];
         }
-        if (smask) bt_row_record(off, S, r, here, bal, run, uoff);
+        if (lane == j) {
+          bals = bal;
+          runs = run;
+        }
         run += __popc(bal);
         carry = __shfl_sync(0xffffffffu, k[j], 31);
       }
+      bt_starts<true>(off, S, r0, min(r0 + 32 * R, end), st, bals, runs, uoff);
     }
   }
   // The last warp of the last block ends at n: its running count is U.
-  if (blockIdx.x == gridDim.x - 1 && warp == CS_WARPS - 1 && lane == 0) bt_record_end(off, S, run, uoff);
+  if (blockIdx.x == gridDim.x - 1 && warp == CS_WARPS - 1) bt_record_end(st.cloud, S, run, uoff);
 }
 
 // Radix tree of every cloud, one thread per unique code.
