@@ -23,8 +23,9 @@
 //               edge in each cloud's last slot;
 //   6. one inclusive scan of all edge counts; cloud c's node offsets are the
 //               scan minus its value just before U_c (the bias);
-//   7. octree of each cloud (octree_warp_batch) into its node range starting
-//               at O_c = (non-empty clouds before c) + bias.
+//   7. octree of each cloud (octree_window.cuh; octree_warp_batch under the
+//               per-node method) into its node range starting at O_c =
+//               (non-empty clouds before c) + bias.
 
 #include <atomic>
 #include <utility>
@@ -59,7 +60,7 @@ constexpr int BPASSES = 4;  // 30-bit codes in 8-bit digits
 constexpr int BM_THREADS = 512;  // Morton kernel: one block per tile
 // Segmented onesweep tile shapes (threads x keys per thread), compiled as
 // variants: pinned with gtc_batched_set_variant, else the autotuner's pick
-// for the batch's size (gtc_autotune_batched), else variant 0.  Every tile
+// for the batch's size (gtc_autotune_batched), else by size (below).  Every tile
 // division of the batch (tile list, Morton blocks, sort tiles) uses the
 // chosen shape's tile.
 struct BtVariant {
@@ -301,7 +302,7 @@ __global__ void __launch_bounds__(THREADS, MINB) bt_onesweep_kernel(const uint32
   Sm& s = *reinterpret_cast<Sm*>(smem_raw);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t lt_mask = (1u << lane) - 1u;
-  const uint32_t tile = blockIdx.x;  // blocks start in increasing order (sort.cu)
+  const uint32_t tile = blockIdx.x;  // sort.cu has what that assumes
   if (tile >= tile_start[S]) return;
   const TileRange r = tile_range(tile, tile_cloud[tile], tile_start, off, Sm::TILE);
 
@@ -457,8 +458,7 @@ __device__ __forceinline__ void bt_record_end(uint32_t c, uint32_t S, uint32_t r
 }
 
 template <int ROWS>
-__global__ void __launch_bounds__(CS_THREADS) bt_row_unique_kernel(const uint32_t* kin,
-                                                                   const uint32_t* vin,
+__global__ void __launch_bounds__(CS_THREADS) bt_row_unique_kernel(const uint32_t* kin, const uint32_t* vin,
                                                                    uint32_t* __restrict__ kout,
                                                                    uint32_t* __restrict__ vout, uint32_t n,
                                                                    const uint32_t* off, uint32_t S, uint32_t* uoff,
@@ -518,14 +518,14 @@ __global__ void __launch_bounds__(CS_THREADS) bt_row_unique_kernel(const uint32_
 }
 
 // Segments of any length, read twice (scan.cu's chunk_unique_kernel), eight
-// rows in flight per warp.
-__global__ void __launch_bounds__(CS_THREADS, 3) bt_chunk_unique_kernel(const uint32_t* kin,
-                                                                     const uint32_t* vin,
-                                                                     uint32_t* __restrict__ kout,
-                                                                     uint32_t* __restrict__ vout, uint32_t n,
-                                                                     const uint32_t* off, uint32_t S, uint32_t* uoff,
-                                                                     uint32_t* ws, const uint32_t* bad,
-                                                                     uint32_t* status) {
+// rows in flight per warp, three blocks per SM (512 clouds, 74M points: 263 of
+// 3,515 us).
+__global__ void __launch_bounds__(CS_THREADS, 3) bt_chunk_unique_kernel(const uint32_t* kin, const uint32_t* vin,
+                                                                        uint32_t* __restrict__ kout,
+                                                                        uint32_t* __restrict__ vout, uint32_t n,
+                                                                        const uint32_t* off, uint32_t S,
+                                                                        uint32_t* uoff, uint32_t* ws,
+                                                                        const uint32_t* bad, uint32_t* status) {
   griddep_wait();
   __shared__ uint32_t s_seg[CS_WARPS];
   __shared__ uint32_t s_red[CS_WARPS];
@@ -666,7 +666,6 @@ __global__ void bt_cloud_offsets_kernel(uint32_t* uoff, const uint32_t* ne_start
   if (c == S - 1) node_off[S] = O + o;
 }
 
-// One octree body: code g of the cloud described by ci.
 // Octree of every cloud, and the cloud-local node offsets (what the
 // single-cloud node-offset scan gives each cloud).  Warp slices of 32 codes:
 // the slice's cloud comes from one binary search (then a step or two per

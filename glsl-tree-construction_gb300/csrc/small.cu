@@ -3,8 +3,8 @@
 //
 // The stage kernels (morton.comp .. octree.comp, main.rs:60-170) each cost a
 // launch and a chain of dependent global round trips however few points there
-// are: eleven kernels, about 5 us each, for 4,096 points.  Up to SB_MAX points
-// one block of 1,024 threads holds the cloud in shared memory and does every
+// are: eleven kernels, about 5 us each, for 4,096 points.  Up to
+// SMALL_BUILD_MAX points one block holds the cloud in shared memory and does every
 // stage there: Morton codes, stable LSD sort, unique, Karras tree, edge
 // counts, node offsets and octree nodes, with the same outputs as the stage
 // kernels.  One SM's issue rate bounds it (the sort's ranking above all), so

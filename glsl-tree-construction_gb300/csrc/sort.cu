@@ -6,9 +6,11 @@
 // carried alongside the keys and 8-bit digits over [begin_bit, end_bit).
 //
 // One pass over a tile of TILE = THREADS * KPT keys:
-//   1. block b takes tile b: blocks start in increasing order, so a tile only
-//      ever waits on tiles that are already running or done (and every wait is
-//      bounded).  A ticket from an atomic counter costs a tile 2,100 of its
+//   1. block b takes tile b.  That the tiles it waits on are running or done
+//      rests on blocks being started in increasing order, as the hardware
+//      does and CUDA does not promise; if it did not, the bounded waits would
+//      run out and the context report GTC_ERR_TIMEOUT.  A ticket from an
+//      atomic counter needs no such order but costs a tile 2,100 of its
 //      20,000 to 23,000 cycles before its first load; only variant 2 keeps it,
 //      the fastest on 64-bit inputs of tens of millions of keys, where tickets
 //      keep the tiles' order tighter (33.5M pairs: 1809 us, 1854 without);
@@ -1055,7 +1057,8 @@ constexpr Variant kVariants[] = {{256, 16, 0, 3, 0}, {384, 16, 0, 2, 0}, {512, 1
                                  {256, 16, 4, 3, 2}, {512, 12, 4, 2, 2}, {384, 16, 4, 2, 2}, {256, 4, 5, 1, 1},
                                  {512, 4, 5, 1, 1},  {1024, 4, 0, 1, 0}};
 constexpr int kNumVariants = sizeof(kVariants) / sizeof(kVariants[0]);
-static const int g_variant[2] = {0, 2};  // [u32, u64]: what gtc_sort_get_variant reports with nothing pinned
+static const int g_variant[2] = {0, 2};  // [u32, u64]: what gtc_sort_get_variant reports with nothing pinned (the
+                                          // sort then goes by size, sort_select_variant)
 static std::atomic<int> g_pinned[2] = {{-1}, {-1}};  // gtc_sort_set_variant: overrides the tuned choice
 
 // Largest inputs of the one-wave variants (kind 5).  The short tiles' limits

@@ -71,7 +71,9 @@ struct TwShape {
   static_assert(NWB <= 32, "one ballot covers the window's warp-blocks");
 };
 using TwLarge = TwShape<4096, 512, 4>;
-using TwSegLarge = TwShape<8192, 1024, 4>;     // batches, where each block also finds its clouds: a build of 83.5M points takes 4.68 ms, 4.73 with TwLarge
+// Batches, where each block also finds its clouds: 512 clouds of 74M points
+// take 3.535 ms, 3.563 with TwLarge.
+using TwSegLarge = TwShape<8192, 1024, 4>;
 
 // One wave: up to 1.87M splits the shape is one whose blocks all run at once,
 // spread evenly over 152 SMs - the shortest tile of that kind, since an SM
@@ -94,7 +96,7 @@ using TwSegLarge = TwShape<8192, 1024, 4>;     // batches, where each block also
 //   10M                                         4096/4 712     (4096/3 725)
 // (1024/4 is taken up to 700,000, where some SMs have a fifth block: 85.0
 // against 86.3 of 2560/2, and 104.3 against 105.0.)
-constexpr uint32_t TW_SMS = 152;
+constexpr uint32_t TW_SMS = 152;  // fewer would cost speed only: a second wave
 constexpr uint32_t TW_TWO_MAX = 2 * TW_SMS * 4096, TW_WAVE_MAX = 3 * TW_SMS * 4096;
 
 // Calls window(shape) with the one-wave shape for work <= TW_TWO_MAX splits.

@@ -84,8 +84,8 @@ GTC_API const char* gtc_version(void);
  * look-back spin is unbounded (new_radix_sort.comp:209-223).  The budget is
  * 2^20 polls with backoff (well under a second); gtc_set_spin_limit sets it
  * for this context (polls = 0 restores the default).  gtc_debug_skip_first_tile
- * makes the next gtc_sort_pairs_u32/u64 on this context hand out its last
- * pass's tile tickets from 1, so that pass's tile 0 is never sorted and never
+ * makes the last pass of the next gtc_sort_pairs_u32/u64 on this context
+ * start at tile 1, so that pass's tile 0 is never sorted and never
  * publishes its counts: the look-backs that reach it run out of polls (a test
  * of the timeout path; that sort's output is then undefined but every write
  * stays in bounds).  One-shot.  Neither has a counterpart in the reference. */
@@ -438,6 +438,9 @@ GTC_API gtc_status gtc_sort_variant_shape(int variant, int* threads, int* keys_p
 /* Pins one variant for every sort of that key width (overriding the tuned
  * choice); variant = -1 unpins. */
 GTC_API gtc_status gtc_sort_set_variant(int key_bits, int variant);
+/* The pinned variant.  With none pinned, the first choice for that key width
+ * (0 or 2), although a sort then takes the tuner's pick for its shape
+ * (gtc_autotune_lookup), else one by its number of keys. */
 GTC_API int gtc_sort_get_variant(int key_bits);
 /* Digit width of gtc_sort_pairs_u32/u64: 8 bits (4 / 8 passes over full
  * keys), or 7 or 6 where the bit range fits in 8 passes.  Pins one width
